@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "qgpu_internal.cuh"
+#include "qgpu_onevec.cuh"
 
 typedef std::complex<double> cd;
 
@@ -269,7 +270,7 @@ struct Gram {
 }  // namespace
 
 // *real = none of the n values of v has an imaginary part
-static qg_status any_imag(qg_context ctx, const double2 *v, int64_t n, bool *real) {
+qg_status qg_all_real(qg_context ctx, const double2 *v, int64_t n, bool *real) {
   unsigned int *d_im = nullptr, h_im = 1;
   cudaStream_t s = ctx->stream;
   cudaError_t e = cudaMalloc(&d_im, sizeof(unsigned int));
@@ -302,58 +303,6 @@ static qg_status any_imag(qg_context ctx, const double2 *v, int64_t n, bool *rea
 // Ground state of a 29,635-determinant impurity to a variance of 1e-12, 1305 steps in 9
 // restarts: 123 ms, against 578 ms with block products of one column (complex storage, 16 bytes per
 // entry strided by the Krylov dimension), host round trips and allocations in every step.
-template <bool REAL>
-struct OneT;
-template <>
-struct OneT<true> {
-  typedef double T;
-};
-template <>
-struct OneT<false> {
-  typedef double2 T;
-};
-
-__device__ __forceinline__ double one_zero(double) { return 0.0; }
-__device__ __forceinline__ double2 one_zero(double2) { return make_double2(0.0, 0.0); }
-// acc + conj(a) b
-__device__ __forceinline__ double one_dot(double acc, double a, double b) { return fma(a, b, acc); }
-__device__ __forceinline__ double2 one_dot(double2 acc, double2 a, double2 b) {
-  acc.x = fma(a.x, b.x, fma(a.y, b.y, acc.x));
-  acc.y = fma(a.x, b.y, fma(-a.y, b.x, acc.y));
-  return acc;
-}
-// acc - a b
-__device__ __forceinline__ double one_sub(double acc, double a, double b) { return fma(-a, b, acc); }
-__device__ __forceinline__ double2 one_sub(double2 acc, double2 a, double2 b) {
-  acc.x = fma(-a.x, b.x, fma(a.y, b.y, acc.x));
-  acc.y = fma(-a.x, b.y, fma(-a.y, b.x, acc.y));
-  return acc;
-}
-__device__ __forceinline__ double one_axpy(double w, double a, double v) { return fma(-a, v, w); }
-__device__ __forceinline__ double2 one_axpy(double2 w, double a, double2 v) { return qg_axpy2(w, a, v); }
-__device__ __forceinline__ double one_scaled(double v, double s) { return v * s; }
-__device__ __forceinline__ double2 one_scaled(double2 v, double s) { return make_double2(v.x * s, v.y * s); }
-__device__ __forceinline__ double one_sum(double a, double b) { return a + b; }
-__device__ __forceinline__ double2 one_sum(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ double one_norm2(double v) { return v * v; }
-__device__ __forceinline__ double one_norm2(double2 v) { return qg_norm2(v); }
-__device__ __forceinline__ double one_plus_real(double a, double r) { return a + r; }
-__device__ __forceinline__ double2 one_plus_real(double2 a, double r) { return make_double2(a.x + r, a.y); }
-__device__ __forceinline__ double one_shfl(double v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
-__device__ __forceinline__ double2 one_shfl(double2 v, int o) {
-  return make_double2(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o));
-}
-__device__ __forceinline__ double one_ldcg(const double *p) { return __ldcg(p); }
-__device__ __forceinline__ double2 one_ldcg(const double2 *p) { return __ldcg(p); }
-__device__ __forceinline__ double2 one_complex(double v) { return make_double2(v, 0.0); }
-__device__ __forceinline__ double2 one_complex(double2 v) { return v; }
-__device__ __forceinline__ double one_conj(double v) { return v; }
-__device__ __forceinline__ double2 one_conj(double2 v) { return make_double2(v.x, -v.y); }
-__device__ __forceinline__ bool one_is0(double v) { return v == 0.0; }
-__device__ __forceinline__ bool one_is0(double2 v) { return v.x == 0.0 && v.y == 0.0; }
-__device__ __forceinline__ void one_take(double2 v, double &o) { o = v.x; }
-__device__ __forceinline__ void one_take(double2 v, double2 &o) { o = v; }
-
 // scalars of the chain, in device memory
 struct OneScal {
   double alpha;  // a_j of the current step
@@ -380,90 +329,27 @@ __global__ void __launch_bounds__(512) k_one_alpha(const double2 *__restrict__ p
 }
 
 // wo = w - alpha v_j, then c_i = <v_i|wo> for i <= j and column j of the projected matrix
-// (ct[i] = c_i + a_j [i == j] + b_j [i == j - 1]).  A block walks chunks of 256 rows, their wo in
-// shared memory; its warps take the vectors of the block's share (blockIdx.y) four at a time, so
-// that the four lane sums fold into one another (6 additions instead of 20).  The last block
-// sums the blocks' partials in order.
+// (ct[i] = c_i + a_j [i == j] + b_j [i == j - 1])
 template <bool REAL>
 __global__ void __launch_bounds__(256)
     k_one_project(const typename OneT<REAL>::T *__restrict__ V, int64_t n, int j, const typename OneT<REAL>::T *__restrict__ w,
                   typename OneT<REAL>::T *__restrict__ wo, typename OneT<REAL>::T *__restrict__ part,
                   typename OneT<REAL>::T *__restrict__ c, typename OneT<REAL>::T *__restrict__ ct, OneScal *sc) {
   typedef typename OneT<REAL>::T T;
-  extern __shared__ char smem_raw[];
-  T *acc = reinterpret_cast<T *>(smem_raw);  // the block's share of j + 1 sums
-  __shared__ T sw[256];
-  __shared__ int s_last;
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, k = j + 1;
-  const int share = ((k + (int)gridDim.y - 1) / (int)gridDim.y + 3) & ~3;
-  const int b0 = min(k, (int)blockIdx.y * share), b1 = min(k, b0 + share);
-  const double alpha = sc->alpha;
+  const double alpha = sc->alpha, beta = sc->beta;
   const T *vj = V + (int64_t)j * n;
-  for (int i = tid; i < b1 - b0; i += 256) acc[i] = one_zero(T());
-  for (int64_t r0 = (int64_t)blockIdx.x * 256; r0 < n; r0 += (int64_t)gridDim.x * 256) {
-    const int64_t r = r0 + tid;
-    __syncthreads();  // the previous chunk is done with sw
-    T wv = one_zero(T());
-    if (r < n) {
-      wv = one_axpy(w[r], alpha, vj[r]);
-      if (blockIdx.y == 0) wo[r] = wv;
-    }
-    sw[tid] = wv;
-    __syncthreads();
-    const int rows = (int)(n - r0 < 256 ? n - r0 : 256);
-    for (int i0 = b0 + wid * 4; i0 < b1; i0 += 32) {
-      T a[4];
-#pragma unroll
-      for (int q = 0; q < 4; q++) a[q] = one_zero(T());
-#pragma unroll
-      for (int t = 0; t < 8; t++) {
-        const int rr = lane + 32 * t;
-        if (rr < rows) {
-          const T x = sw[rr];
-#pragma unroll
-          for (int q = 0; q < 4; q++)
-            if (i0 + q < b1) a[q] = one_dot(a[q], V[(int64_t)(i0 + q) * n + r0 + rr], x);
-        }
-      }
-      // fold: lanes of bit 4 keep sums 2, 3, the others 0, 1; then bit 3 the odd one
-      const bool h1 = lane & 16, h2 = lane & 8;
-      T k0 = h1 ? a[2] : a[0], k1 = h1 ? a[3] : a[1], g0 = h1 ? a[0] : a[2], g1 = h1 ? a[1] : a[3];
-      k0 = one_sum(k0, one_shfl(g0, 16));
-      k1 = one_sum(k1, one_shfl(g1, 16));
-      T f = h2 ? k1 : k0, g = h2 ? k0 : k1;
-      f = one_sum(f, one_shfl(g, 8));
-      for (int o = 4; o; o >>= 1) f = one_sum(f, one_shfl(f, o));
-      const int q = (h1 ? 2 : 0) + (h2 ? 1 : 0);
-      if ((lane & 7) == 0 && i0 + q < b1) acc[i0 - b0 + q] = one_sum(acc[i0 - b0 + q], f);
-    }
-  }
-  __syncthreads();
-  for (int i = tid; i < b1 - b0; i += 256) part[(int64_t)blockIdx.x * k + b0 + i] = acc[i];
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) s_last = atomicAdd(&sc->tickets[0], 1u) == gridDim.x * gridDim.y - 1;
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  // 32 sums at a time, a lane each, the warps sharing the blocks (sw: their eight parts)
-  const double beta = sc->beta;
-  for (int i0 = 0; i0 < k; i0 += 32) {
-    T s = one_zero(T());
-    if (i0 + lane < k) {
-#pragma unroll 8
-      for (int b = wid; b < (int)gridDim.x; b += 8) s = one_sum(s, one_ldcg(part + (int64_t)b * k + i0 + lane));
-    }
-    sw[tid] = s;
-    __syncthreads();
-    if (wid == 0 && i0 + lane < k) {
-      for (int g = 1; g < 8; g++) s = one_sum(s, sw[32 * g + lane]);
-      const int i = i0 + lane;
-      c[i] = s;
-      ct[i] = one_plus_real(s, i == j ? alpha : i == j - 1 ? beta : 0.0);
-    }
-    __syncthreads();
-  }
-  if (tid == 0) sc->tickets[0] = 0u;
+  one_multidot<T>(
+      V, n, j + 1,
+      [&](int64_t r) {
+        const T v = one_axpy(w[r], alpha, vj[r]);
+        if (blockIdx.y == 0) wo[r] = v;
+        return v;
+      },
+      part, &sc->tickets[0],
+      [&](int i, T t) {
+        c[i] = t;
+        ct[i] = one_plus_real(t, i == j ? alpha : i == j - 1 ? beta : 0.0);
+      });
 }
 
 // w -= sum_i c_i v_i over i < k (out = w), and the squared norm of the result: the last block
@@ -473,55 +359,26 @@ __global__ void __launch_bounds__(128)
     k_one_update(const typename OneT<REAL>::T *__restrict__ V, int64_t n, int k, const typename OneT<REAL>::T *__restrict__ c,
                  typename OneT<REAL>::T *__restrict__ w, double *__restrict__ part, int step, OneScal *sc) {
   typedef typename OneT<REAL>::T T;
-  extern __shared__ char smem_raw[];
+  extern __shared__ __align__(16) char smem_raw[];
   T *cs = reinterpret_cast<T *>(smem_raw);
   __shared__ double sh[4];
   __shared__ int s_last;
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int tid = threadIdx.x;
   for (int i = tid; i < k; i += 128) cs[i] = c[i];
   __syncthreads();
   double s = 0.0;
   for (int64_t r = (int64_t)blockIdx.x * 128 + tid; r < n; r += (int64_t)gridDim.x * 128) {
-    T x = w[r], y = one_zero(T());
-    int i = 0;
-    for (; i + 8 <= k; i += 8) {
-      T v[8];
-#pragma unroll
-      for (int q = 0; q < 8; q++) v[q] = V[(int64_t)(i + q) * n + r];
-#pragma unroll
-      for (int q = 0; q < 8; q += 2) {
-        x = one_sub(x, v[q], cs[i + q]);
-        y = one_sub(y, v[q + 1], cs[i + q + 1]);
-      }
-    }
-    for (; i < k; i++) x = one_sub(x, V[(int64_t)i * n + r], cs[i]);
-    x = one_sum(x, y);
+    const T x = one_minus_sum(w[r], V, n, k, cs, r);
     if (k) w[r] = x;
     s += one_norm2(x);
   }
-  for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) sh[wid] = s;
-  __syncthreads();
-  if (tid == 0) {
-    part[blockIdx.x] = (sh[0] + sh[1]) + (sh[2] + sh[3]);
-    __threadfence();
-    s_last = atomicAdd(&sc->tickets[1], 1u) == gridDim.x - 1;
-  }
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  s = 0.0;
-  for (int b = tid; b < (int)gridDim.x; b += 128) s += __ldcg(part + b);
-  for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) sh[wid] = s;
-  __syncthreads();
-  if (tid == 0) {
-    const double t = (sh[0] + sh[1]) + (sh[2] + sh[3]), b = sqrt(t);
+  const double t = one_total128(s, part, sh, &s_last, &sc->tickets[1]);
+  if (s_last && tid == 0) {
+    const double b = sqrt(t);
     sc->norm2 = t;
     sc->beta = b;
     sc->scale = b > 0.0 ? 1.0 / b : 0.0;
     if (!(b > 0.0) && step < sc->dead) sc->dead = step;
-    sc->tickets[1] = 0u;
   }
 }
 
@@ -531,18 +388,6 @@ __global__ void k_one_scale(int64_t n, const typename OneT<REAL>::T *__restrict_
   const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (r == 0 && tsub) *tsub = sc->beta;
   if (r < n) v[r] = one_scaled(w[r], sc->scale);
-}
-
-// the start vector of the caller (complex) / the state back to the caller
-template <bool REAL>
-__global__ void k_one_in(int64_t n, const double2 *__restrict__ x, typename OneT<REAL>::T *__restrict__ v) {
-  const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (r < n) one_take(x[r], v[r]);
-}
-template <bool REAL>
-__global__ void k_one_out(int64_t n, const typename OneT<REAL>::T *__restrict__ v, double2 *__restrict__ x) {
-  const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (r < n) x[r] = one_complex(v[r]);
 }
 
 // M (k x k row-major): the Hermitian part of the projected matrix, column j of it in ct[j * ldt +
@@ -572,7 +417,7 @@ __global__ void __launch_bounds__(128)
     k_one_combine(const typename OneT<REAL>::T *__restrict__ V, int64_t n, int k, const double2 *__restrict__ y,
                   typename OneT<REAL>::T *__restrict__ x) {
   typedef typename OneT<REAL>::T T;
-  extern __shared__ char smem_raw[];
+  extern __shared__ __align__(16) char smem_raw[];
   T *cs = reinterpret_cast<T *>(smem_raw);
   for (int i = threadIdx.x; i < k; i += 128) {
     T t;
@@ -582,20 +427,7 @@ __global__ void __launch_bounds__(128)
   __syncthreads();
   const int64_t r = blockIdx.x * (int64_t)128 + threadIdx.x;
   if (r >= n) return;
-  T a = one_zero(T()), b = one_zero(T());
-  int i = 0;
-  for (; i + 8 <= k; i += 8) {
-    T v[8];
-#pragma unroll
-    for (int q = 0; q < 8; q++) v[q] = V[(int64_t)(i + q) * n + r];
-#pragma unroll
-    for (int q = 0; q < 8; q += 2) {
-      a = one_sub(a, v[q], cs[i + q]);
-      b = one_sub(b, v[q + 1], cs[i + q + 1]);
-    }
-  }
-  for (; i < k; i++) a = one_sub(a, V[(int64_t)i * n + r], cs[i]);
-  x[r] = one_sum(a, b);
+  x[r] = one_minus_sum(one_zero(T()), V, n, k, cs, r);
 }
 
 #define ONE_MAX_K 2500  // the coefficients of a step fit one block's default shared memory
@@ -609,7 +441,7 @@ static qg_status groundstate_one(qg_context ctx, qg_operator op, qg_basis b, dou
   cudaStream_t s = ctx->stream;
   const int64_t n = b->n;
   const int Pa = qg_apply_grid(b);
-  const unsigned gp = (unsigned)std::min<int64_t>((n + 255) / 256, 4LL * ctx->num_sms);
+  const unsigned gp = one_multidot_grid(ctx, n, 1).x;
   const unsigned gu = (unsigned)std::min<int64_t>((n + 127) / 128, 8LL * ctx->num_sms);
   const unsigned g1 = (unsigned)((n + 255) / 256), gc = (unsigned)((n + 127) / 128);
   T *V = nullptr, *w = nullptr, *wo = nullptr, *x = nullptr, *part = nullptr, *c = nullptr, *ct = nullptr;
@@ -668,9 +500,7 @@ static qg_status groundstate_one(qg_context ctx, qg_operator op, qg_basis b, dou
       (*applies)++;
       if (st != QG_OK) break;
       k_one_alpha<<<1, 512, 0, s>>>(dpart, Pa, sc);
-      // few rows: the vectors are shared out over enough blocks for two on every SM
-      const int gy = std::max(1, std::min((j + 32) / 32, (int)((2 * ctx->num_sms + gp - 1) / gp)));
-      k_one_project<REAL><<<dim3(gp, (unsigned)gy), 256, (size_t)(j + 4) * sizeof(T), s>>>(
+      k_one_project<REAL><<<one_multidot_grid(ctx, n, j + 1), 256, one_multidot_smem<T>(j + 1), s>>>(
           V, n, j, w, wo, part, c, ct + (size_t)j * K, sc);
       ctx->launches += 2;
       if (j + 1 < Kcur) {
@@ -761,7 +591,7 @@ extern "C" qg_status qg_block_groundstate(qg_context ctx, qg_operator op, qg_bas
     bool real = qg_operator_values_real(op), conv = false;
     int applies = 0;
     double energy = 0.0;
-    if (real) QG_TRY(any_imag(ctx, (const double2 *)x_dev, n, &real));
+    if (real) QG_TRY(qg_all_real(ctx, (const double2 *)x_dev, n, &real));
     qg_status st = real ? groundstate_one<true>(ctx, op, b, (double2 *)x_dev, &energy, tol, K, max_restarts, &applies, &conv)
                         : groundstate_one<false>(ctx, op, b, (double2 *)x_dev, &energy, tol, K, max_restarts, &applies, &conv);
     energies_host[0] = energy;
@@ -808,7 +638,7 @@ extern "C" qg_status qg_block_groundstate(qg_context ctx, qg_operator op, qg_bas
   // a real operator with real start vectors keeps every vector, every projection and the Ritz
   // vectors real (the reference's real-vector solver): the block products then run in real
   // arithmetic, one FMA per term instead of four
-  if (st == QG_OK && qg_operator_values_real(op)) st = any_imag(ctx, X, n * p, &G.real);
+  if (st == QG_OK && qg_operator_values_real(op)) st = qg_all_real(ctx, X, n * p, &G.real);
   std::vector<double> theta(p, 0.0);
   int it = 0;
   bool converged = false;

@@ -369,6 +369,8 @@ qg_status qg_eigh_device(qg_context ctx, int k, double2 *A, double *w_dev, doubl
 qg_status qg_eigh_tridiag(qg_context ctx, int k, double2 *A, double *w_dev, double2 *V_dev, int nv);
 qg_status qg_eigh_host_io(qg_context ctx, int k, const double *a_host, double *w_host, double *v_host, int nv);
 int qg_partial_blocks(qg_context ctx, int64_t n);
+// *real = none of the n values of v (device) has an imaginary part (qgpu_eigen.cu)
+qg_status qg_all_real(qg_context ctx, const double2 *v, int64_t n, bool *real);
 
 // dense complex block products (qgpu_blocks.cu); row-major n x k blocks
 //   C (ka x kb row-major) = A^H B, with a work buffer of work_elems complex entries for the

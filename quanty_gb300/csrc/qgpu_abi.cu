@@ -1,6 +1,11 @@
 // Context, error handling and small shared services of the C ABI (include/qgpu.h).
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
+#include <list>
+#include <mutex>
+#include <unordered_map>
+#include <vector>
 
 #include "qgpu_internal.cuh"
 
@@ -40,6 +45,131 @@ qg_status qg_check_device_error(qg_context ctx, const char *what) {
     return QG_ERR_TABLE_FULL;
   }
   return QG_OK;
+}
+
+// ------------------------------------------------------------------ device memory
+
+#define QG_POOL_BYTES ((size_t)1 << 30)  // kept per context
+#define QG_POOL_BLOCK ((size_t)1 << 29)  // the largest block kept
+
+struct QgPool {
+  std::mutex m;
+  bool open = true;
+  size_t held = 0;
+  std::list<std::pair<void *, size_t>> idle;  // oldest first
+
+  // give idle blocks back until at most `most` bytes are held (m locked)
+  void shrink(size_t most) {
+    while (!idle.empty() && held > most) {
+      cudaFree(idle.front().first);
+      held -= idle.front().second;
+      idle.pop_front();
+    }
+  }
+};
+
+namespace {
+std::mutex g_live_m;
+// every block handed out: its pool and its size
+std::unordered_map<void *, std::pair<std::shared_ptr<QgPool>, size_t>> g_live;
+std::vector<std::weak_ptr<QgPool>> g_pools;
+
+std::vector<std::shared_ptr<QgPool>> all_pools() {
+  std::lock_guard<std::mutex> l(g_live_m);
+  std::vector<std::shared_ptr<QgPool>> out;
+  for (auto &w : g_pools)
+    if (auto p = w.lock()) out.push_back(p);
+  return out;
+}
+}  // namespace
+
+cudaError_t qg_malloc_bytes(qg_context ctx, void **p, size_t bytes) {
+  *p = nullptr;
+  if (!bytes) return cudaSuccess;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (!ctx || !ctx->pool || cudaStreamIsCapturing(ctx->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return cudaMalloc(p, bytes);
+  }
+  const size_t need = (bytes + 511) & ~(size_t)511;
+  size_t got = need;
+  {
+    std::lock_guard<std::mutex> l(ctx->pool->m);
+    auto best = ctx->pool->idle.end();
+    for (auto it = ctx->pool->idle.begin(); it != ctx->pool->idle.end(); ++it)
+      if (it->second >= need && it->second <= need + need / 8 + 4096 &&
+          (best == ctx->pool->idle.end() || it->second < best->second))
+        best = it;
+    if (best != ctx->pool->idle.end()) {
+      *p = best->first;
+      got = best->second;
+      ctx->pool->held -= got;
+      ctx->pool->idle.erase(best);
+    }
+  }
+  if (!*p) {
+    cudaError_t e = cudaMalloc(p, need);
+    if (e == cudaErrorMemoryAllocation) {  // what the pools hold may be what is missing
+      cudaGetLastError();
+      for (auto &q : all_pools()) {
+        std::lock_guard<std::mutex> l(q->m);
+        q->shrink(0);
+      }
+      e = cudaMalloc(p, need);
+    }
+    if (e != cudaSuccess) {
+      *p = nullptr;
+      return e;
+    }
+  }
+  std::lock_guard<std::mutex> l(g_live_m);
+  g_live[*p] = {ctx->pool, got};
+  return cudaSuccess;
+}
+
+cudaError_t qg_free(void *p) {
+  if (!p) return cudaSuccess;
+  std::shared_ptr<QgPool> pool;
+  size_t size = 0;
+  {
+    std::lock_guard<std::mutex> l(g_live_m);
+    auto it = g_live.find(p);
+    if (it != g_live.end()) {
+      pool = it->second.first;
+      size = it->second.second;
+      g_live.erase(it);
+    }
+  }
+  if (!pool || size > QG_POOL_BLOCK) return cudaFree(p);
+  std::lock_guard<std::mutex> l(pool->m);
+  if (!pool->open) return cudaFree(p);
+  pool->shrink(QG_POOL_BYTES - size);
+  pool->idle.emplace_back(p, size);
+  pool->held += size;
+  return cudaSuccess;
+}
+
+cudaError_t qg_free_now(void *p) {
+  if (p) {
+    std::lock_guard<std::mutex> l(g_live_m);
+    g_live.erase(p);
+  }
+  return cudaFree(p);
+}
+
+cudaError_t qg_mem_info(size_t *free_bytes, size_t *total_bytes) {
+  cudaError_t e = cudaMemGetInfo(free_bytes, total_bytes);
+  if (e != cudaSuccess) return e;
+  for (auto &q : all_pools()) {
+    std::lock_guard<std::mutex> l(q->m);
+    *free_bytes += q->held;
+  }
+  return cudaSuccess;
+}
+
+cudaError_t qg_upload(qg_context ctx, void *dst, const void *src, size_t bytes) {
+  cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream);
+  return e == cudaSuccess ? cudaStreamSynchronize(ctx->stream) : e;
 }
 
 qg_status qg_ensure_scratch(qg_context ctx, size_t bytes) {
@@ -87,6 +217,13 @@ extern "C" qg_status qg_init(int device, qg_context *out) {
     delete ctx;
     return QG_ERR_CUDA;
   }
+  ctx->pool = std::make_shared<QgPool>();
+  {
+    std::lock_guard<std::mutex> l(g_live_m);
+    g_pools.erase(std::remove_if(g_pools.begin(), g_pools.end(), [](const std::weak_ptr<QgPool> &w) { return w.expired(); }),
+                  g_pools.end());
+    g_pools.push_back(ctx->pool);
+  }
   *out = ctx;
   return QG_OK;
 }
@@ -94,10 +231,15 @@ extern "C" qg_status qg_init(int device, qg_context *out) {
 extern "C" qg_status qg_finalize(qg_context ctx) {
   if (!ctx) return QG_OK;
   cudaStreamSynchronize(ctx->stream);
+  {
+    std::lock_guard<std::mutex> l(ctx->pool->m);
+    ctx->pool->open = false;
+    ctx->pool->shrink(0);
+  }
   cudaFree(ctx->d_err);
   cudaFree(ctx->d_scratch);
   cudaFreeHost(ctx->h_pinned);
-  cudaFree(ctx->d_io);
+  qg_free_now(ctx->d_io);
   if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
   return QG_OK;

@@ -1231,16 +1231,16 @@ __global__ void k_block_verify(const Key<W> *keys, int64_t n, int lo, uint32_t l
 }
 
 void qg_cache_free(OpBasisCache &c) {
-  cudaFree(c.d_diag);
-  cudaFree(c.d_wreq);
-  cudaFree(c.d_bstart);
-  cudaFree(c.d_cfg);
-  cudaFree(c.d_eoff);
-  cudaFree(c.d_ent);
-  cudaFree(c.d_ent_target);
-  cudaFree(c.d_cptr);
-  cudaFree(c.d_conn);
-  cudaFree(c.d_coef);
+  qg_free(c.d_diag);
+  qg_free(c.d_wreq);
+  qg_free(c.d_bstart);
+  qg_free(c.d_cfg);
+  qg_free(c.d_eoff);
+  qg_free(c.d_ent);
+  qg_free(c.d_ent_target);
+  qg_free(c.d_cptr);
+  qg_free(c.d_conn);
+  qg_free(c.d_coef);
   c = OpBasisCache();
 }
 
@@ -1297,11 +1297,11 @@ static qg_status build_local(qg_basis bs, qg_operator op, OpBasisCache &c) {
   uint32_t *cfg = nullptr, *flag = nullptr, *pos = nullptr, *bst = nullptr, *bcf = nullptr;
   void *tmp = nullptr;
   size_t tb = 0;
-  cudaError_t e = cudaMalloc(&cfg, n * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&flag, n * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&pos, n * 4);
+  cudaError_t e = qg_malloc(ctx, &cfg, n * 4);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &flag, n * 4);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &pos, n * 4);
   if (e == cudaSuccess) e = cub::DeviceScan::InclusiveSum(nullptr, tb, flag, pos, (int)n, s);
-  if (e == cudaSuccess) e = cudaMalloc(&tmp, tb);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &tmp, tb);
   if (e == cudaSuccess) {
     if (W == 1)
       k_local_cfg<1><<<grid_for(n, 256), 256, 0, s>>>((const Key<1> *)bs->d_keys, n, lo, lmask, cfg, flag);
@@ -1314,8 +1314,8 @@ static qg_status build_local(qg_basis bs, qg_operator op, OpBasisCache &c) {
   uint32_t nb = 0;
   if (e == cudaSuccess) e = cudaMemcpyAsync(&nb, pos + n - 1, 4, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e == cudaSuccess) e = cudaMalloc(&bst, (size_t)(nb + 1) * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&bcf, (size_t)nb * 4 + 4);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &bst, (size_t)(nb + 1) * 4);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &bcf, (size_t)nb * 4 + 4);
   if (e == cudaSuccess) {
     k_block_scatter<<<grid_for(n, 256), 256, 0, s>>>(cfg, flag, pos, n, bst, bcf);
     ctx->launches++;
@@ -1332,9 +1332,9 @@ static qg_status build_local(qg_basis bs, qg_operator op, OpBasisCache &c) {
   {
     unsigned long long *fp = nullptr;
     uint32_t *rep = nullptr, *mis = nullptr;
-    if (e == cudaSuccess) e = cudaMalloc(&fp, (size_t)nb * 16 + 16);
-    if (e == cudaSuccess) e = cudaMalloc(&rep, (size_t)nb * 4 + 4);
-    if (e == cudaSuccess) e = cudaMalloc(&mis, (size_t)nb * 4 + 4);
+    if (e == cudaSuccess) e = qg_malloc(ctx, &fp, (size_t)nb * 16 + 16);
+    if (e == cudaSuccess) e = qg_malloc(ctx, &rep, (size_t)nb * 4 + 4);
+    if (e == cudaSuccess) e = qg_malloc(ctx, &mis, (size_t)nb * 4 + 4);
     if (e == cudaSuccess) e = cudaMemsetAsync(mis, 0, (size_t)nb * 4 + 4, s);
     if (e == cudaSuccess) {
       if (W == 1)
@@ -1370,17 +1370,17 @@ static qg_status build_local(qg_basis bs, qg_operator op, OpBasisCache &c) {
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e == cudaSuccess)
       for (uint32_t k = 0; k < nb; k++) cls[k] = hmis[k] ? k : hrep[k];
-    cudaFree(fp);
-    cudaFree(rep);
-    cudaFree(mis);
+    qg_free(fp);
+    qg_free(rep);
+    qg_free(mis);
   }
-  cudaFree(cfg);
-  cudaFree(flag);
-  cudaFree(pos);
-  cudaFree(tmp);
-  cudaFree(bcf);
+  qg_free(cfg);
+  qg_free(flag);
+  qg_free(pos);
+  qg_free(tmp);
+  qg_free(bcf);
   if (e != cudaSuccess) {
-    cudaFree(bst);
+    qg_free(bst);
     return qg_cuda_fail(ctx, e, "local blocks");
   }
   // configuration -> block
@@ -1438,16 +1438,16 @@ static qg_status build_local(qg_basis bs, qg_operator op, OpBasisCache &c) {
   c.h_etarget = etarget;
   c.h_ent = ent;
   c.d_bstart = bst;
-  e = cudaMalloc(&c.d_cfg, table.size() * 4);
-  if (e == cudaSuccess) e = cudaMemcpy(c.d_cfg, table.data(), table.size() * 4, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMalloc(&c.d_eoff, eoff.size() * 4);
-  if (e == cudaSuccess) e = cudaMemcpy(c.d_eoff, eoff.data(), eoff.size() * 4, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMalloc(&c.d_ent, std::max<size_t>(ent.size(), 1) * sizeof(LocalEntry));
+  e = qg_malloc(ctx, &c.d_cfg, table.size() * 4);
+  if (e == cudaSuccess) e = qg_upload(ctx, c.d_cfg, table.data(), table.size() * 4);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &c.d_eoff, eoff.size() * 4);
+  if (e == cudaSuccess) e = qg_upload(ctx, c.d_eoff, eoff.data(), eoff.size() * 4);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &c.d_ent, std::max<size_t>(ent.size(), 1) * sizeof(LocalEntry));
   if (e == cudaSuccess && !ent.empty())
-    e = cudaMemcpy(c.d_ent, ent.data(), ent.size() * sizeof(LocalEntry), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMalloc(&c.d_ent_target, std::max<size_t>(etarget.size(), 1) * 4);
+    e = qg_upload(ctx, c.d_ent, ent.data(), ent.size() * sizeof(LocalEntry));
+  if (e == cudaSuccess) e = qg_malloc(ctx, &c.d_ent_target, std::max<size_t>(etarget.size(), 1) * 4);
   if (e == cudaSuccess && !etarget.empty())
-    e = cudaMemcpy(c.d_ent_target, etarget.data(), etarget.size() * 4, cudaMemcpyHostToDevice);
+    e = qg_upload(ctx, c.d_ent_target, etarget.data(), etarget.size() * 4);
   if (e != cudaSuccess) return qg_cuda_fail(ctx, e, "local entries");
   if (!exact) c.wreq_exact = false;
   return QG_OK;
@@ -1553,7 +1553,7 @@ OpBasisCache *qg_basis_cache(qg_basis b, qg_operator op, qg_status *st) {
   OpBasisCache c;
   c.op_uid = op->uid;
   c.op_version = op->version;
-  cudaError_t e = cudaMalloc(&c.d_diag, std::max<int64_t>(b->n, 1) * 16);
+  cudaError_t e = qg_malloc(ctx, &c.d_diag, std::max<int64_t>(b->n, 1) * 16);
   if (e != cudaSuccess) {
     *st = qg_cuda_fail(ctx, e, "diagonal");
     return nullptr;
@@ -1569,8 +1569,8 @@ OpBasisCache *qg_basis_cache(qg_basis b, qg_operator op, qg_status *st) {
       c.wreq_exact = move_bits(b, on, offb, wr[t]);
     }
     if (c.wreq_exact) {
-      e = cudaMalloc(&c.d_wreq, wr.size() * 8);
-      if (e == cudaSuccess) e = cudaMemcpy(c.d_wreq, wr.data(), wr.size() * 8, cudaMemcpyHostToDevice);
+      e = qg_malloc(ctx, &c.d_wreq, wr.size() * 8);
+      if (e == cudaSuccess) e = qg_upload(ctx, c.d_wreq, wr.data(), wr.size() * 8);
       if (e != cudaSuccess) {
         qg_cache_free(c);
         *st = qg_cuda_fail(ctx, e, "window bits");
@@ -1586,7 +1586,7 @@ OpBasisCache *qg_basis_cache(qg_basis b, qg_operator op, qg_status *st) {
       return nullptr;
     }
     if (keep_exact && !c.wreq_exact) {  // a local move outside the encoding: full checks
-      cudaFree(c.d_wreq);
+      qg_free(c.d_wreq);
       c.d_wreq = nullptr;
     }
   }
@@ -1661,7 +1661,7 @@ static qg_status build_conn(qg_context ctx, qg_operator op, qg_basis b, OpBasisC
   same_basis_view(op, b, &c, &tab, &lv, &wreq);
   cudaStream_t s = ctx->stream;
   size_t fr = 0, tot = 0;
-  if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
+  if (qg_mem_info(&fr, &tot) != cudaSuccess) {
     cudaGetLastError();
     return QG_OK;
   }
@@ -1670,10 +1670,10 @@ static qg_status build_conn(qg_context ctx, qg_operator op, qg_basis b, OpBasisC
   int64_t *cnt = nullptr, *cptr = nullptr;
   void *tmp = nullptr;
   size_t tb = 0;
-  cudaError_t e = cudaMalloc(&cnt, ptr_bytes);
-  if (e == cudaSuccess) e = cudaMalloc(&cptr, ptr_bytes);
+  cudaError_t e = qg_malloc(ctx, &cnt, ptr_bytes);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &cptr, ptr_bytes);
   if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt, cptr, n + 1, s);
-  if (e == cudaSuccess) e = cudaMalloc(&tmp, std::max<size_t>(tb, 16));
+  if (e == cudaSuccess) e = qg_malloc(ctx, &tmp, std::max<size_t>(tb, 16));
   if (e == cudaSuccess) e = cudaMemsetAsync(cnt + n, 0, 8, s);
   if (e == cudaSuccess) {
     if (b->W == 1)
@@ -1686,27 +1686,27 @@ static qg_status build_conn(qg_context ctx, qg_operator op, qg_basis b, OpBasisC
   int64_t total = 0;
   if (e == cudaSuccess) e = cudaMemcpyAsync(&total, cptr + n, 8, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  cudaFree(cnt);
-  cudaFree(tmp);
+  qg_free(cnt);
+  qg_free(tmp);
   if (e != cudaSuccess) {
-    cudaFree(cptr);
+    qg_free(cptr);
     return qg_cuda_fail(ctx, e, "connection counts");
   }
   QG_TRY(qg_check_device_error(ctx, "connection counts"));
   size_t conn_bytes = (size_t)std::max<int64_t>(total, 1) * sizeof(uint2);
-  if (cudaMemGetInfo(&fr, &tot) != cudaSuccess || 4 * conn_bytes > fr) {
+  if (qg_mem_info(&fr, &tot) != cudaSuccess || 4 * conn_bytes > fr) {
     cudaGetLastError();
-    cudaFree(cptr);
+    qg_free(cptr);
     return QG_OK;
   }
   uint2 *conn = nullptr;
   double2 *coef = nullptr;
-  e = cudaMalloc(&conn, conn_bytes);
-  if (e == cudaSuccess) e = cudaMalloc(&coef, (size_t)std::max(tab->nterms, 1) * 16);
+  e = qg_malloc(ctx, &conn, conn_bytes);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &coef, (size_t)std::max(tab->nterms, 1) * 16);
   if (e != cudaSuccess) {
-    cudaFree(cptr);
-    cudaFree(conn);
-    cudaFree(coef);
+    qg_free(cptr);
+    qg_free(conn);
+    qg_free(coef);
     cudaGetLastError();
     return QG_OK;  // no room: the hash path stays
   }
@@ -1728,9 +1728,9 @@ static qg_status build_conn(qg_context ctx, qg_operator op, qg_basis b, OpBasisC
   }
   if (st == QG_OK) st = qg_check_device_error(ctx, "connection lists");
   if (st != QG_OK) {
-    cudaFree(cptr);
-    cudaFree(conn);
-    cudaFree(coef);
+    qg_free(cptr);
+    qg_free(conn);
+    qg_free(coef);
     return st;
   }
   c.d_cptr = cptr;
@@ -1897,10 +1897,10 @@ static void launch_small_csr(qg_context ctx, qg_basis b, const OpBasisCache *c, 
 }
 
 void qg_small_csr_free(SmallCsr &c) {
-  cudaFree(c.rowptr);
-  cudaFree(c.col);
-  cudaFree(c.val);
-  cudaFree(c.kind);
+  qg_free(c.rowptr);
+  qg_free(c.col);
+  qg_free(c.val);
+  qg_free(c.kind);
   c = SmallCsr();
 }
 
@@ -1919,8 +1919,8 @@ qg_status qg_small_csr(qg_context ctx, qg_operator op, qg_basis b, int64_t max_n
   SmallCsr s;
   s.n = n;
   int *cnt = nullptr;
-  cudaError_t e = cudaMalloc(&cnt, (size_t)n * sizeof(int));
-  if (e == cudaSuccess) e = cudaMalloc(&s.rowptr, (size_t)(n + 1) * sizeof(int));
+  cudaError_t e = qg_malloc(ctx, &cnt, (size_t)n * sizeof(int));
+  if (e == cudaSuccess) e = qg_malloc(ctx, &s.rowptr, (size_t)(n + 1) * sizeof(int));
   if (e == cudaSuccess) {
     if (b->W == 1)
       launch_small_csr<1, false>(ctx, b, c, lv, real, cnt, nullptr, nullptr, nullptr, nullptr);
@@ -1931,7 +1931,7 @@ qg_status qg_small_csr(qg_context ctx, qg_operator op, qg_basis b, int64_t max_n
   std::vector<int> hc(n), hp(n + 1, 0);
   if (e == cudaSuccess) e = cudaMemcpyAsync(hc.data(), cnt, (size_t)n * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-  cudaFree(cnt);
+  qg_free(cnt);
   if (e != cudaSuccess) {
     qg_small_csr_free(s);
     return qg_cuda_fail(ctx, e, "small-basis rows");
@@ -1944,15 +1944,15 @@ qg_status qg_small_csr(qg_context ctx, qg_operator op, qg_basis b, int64_t max_n
   hp[n] = (int)std::min<int64_t>(tot, INT32_MAX);
   s.nnz = tot;
   if (tot > max_nnz) {  // too many terms for one block per chain: the caller takes the general path
-    cudaFree(s.rowptr);
+    qg_free(s.rowptr);
     out->n = n;
     out->nnz = tot;
     return QG_OK;
   }
   e = cudaMemcpyAsync(s.rowptr, hp.data(), (size_t)(n + 1) * sizeof(int), cudaMemcpyHostToDevice, ctx->stream);
-  if (e == cudaSuccess) e = cudaMalloc(&s.col, (size_t)std::max<int64_t>(tot, 1) * sizeof(int));
-  if (e == cudaSuccess) e = cudaMalloc(&s.val, (size_t)std::max<int64_t>(tot, 1) * sizeof(double2));
-  if (e == cudaSuccess) e = cudaMalloc(&s.kind, (size_t)std::max<int64_t>(tot, 1));
+  if (e == cudaSuccess) e = qg_malloc(ctx, &s.col, (size_t)std::max<int64_t>(tot, 1) * sizeof(int));
+  if (e == cudaSuccess) e = qg_malloc(ctx, &s.val, (size_t)std::max<int64_t>(tot, 1) * sizeof(double2));
+  if (e == cudaSuccess) e = qg_malloc(ctx, &s.kind, (size_t)std::max<int64_t>(tot, 1));
   if (e == cudaSuccess) {
     if (b->W == 1)
       launch_small_csr<1, true>(ctx, b, c, lv, real, nullptr, s.rowptr, s.col, s.val, s.kind);
@@ -2177,10 +2177,10 @@ extern "C" qg_status qg_apply_host(qg_context ctx, qg_operator op, qg_basis dst,
   size_t need = xb + (ymap ? 0 : yb);
   if (ctx->io_bytes < need) {
     cudaStreamSynchronize(ctx->stream);
-    cudaFree(ctx->d_io);
+    qg_free(ctx->d_io);
     ctx->d_io = nullptr;
     ctx->io_bytes = 0;
-    QG_CUDA(ctx, cudaMalloc(&ctx->d_io, need));
+    QG_CUDA(ctx, qg_malloc(ctx, &ctx->d_io, need));
     ctx->io_bytes = need;
   }
   double *dx = ctx->d_io, *dy = ymap ? ymap : ctx->d_io + xb / 8;
@@ -2244,7 +2244,7 @@ static qg_status count_nnz(qg_context ctx, qg_operator op, qg_basis b, int offdi
   if (row0 >= b->n) return QG_OK;
   const int64_t cnt = (b->n - row0 + stride - 1) / stride;
   unsigned long long *d = nullptr;
-  QG_CUDA(ctx, cudaMalloc(&d, 8));
+  QG_CUDA(ctx, qg_malloc(ctx, &d, 8));
   cudaError_t e = cudaMemsetAsync(d, 0, 8, ctx->stream);
   if (e == cudaSuccess) {
     if (op->W == 1)
@@ -2261,7 +2261,7 @@ static qg_status count_nnz(qg_context ctx, qg_operator op, qg_basis b, int offdi
   unsigned long long h = 0;
   if (e == cudaSuccess) e = cudaMemcpyAsync(&h, d, 8, cudaMemcpyDeviceToHost, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-  cudaFree(d);
+  qg_free(d);
   if (e != cudaSuccess) return qg_cuda_fail(ctx, e, "qg_count_nnz");
   *nnz = (int64_t)h;
   return qg_check_device_error(ctx, "qg_count_nnz");
@@ -2334,7 +2334,7 @@ extern "C" qg_status qg_apply_fp64_ops(qg_context ctx, qg_operator op, qg_basis 
   const uint64_t *wreq;
   same_basis_view(op, b, c, &tab, &lv, &wreq);
   unsigned long long *d = nullptr;
-  QG_CUDA(ctx, cudaMalloc(&d, 8));
+  QG_CUDA(ctx, qg_malloc(ctx, &d, 8));
   cudaError_t e = cudaMemsetAsync(d, 0, 8, ctx->stream);
   if (e == cudaSuccess) {
     if (b->W == 1)
@@ -2351,7 +2351,7 @@ extern "C" qg_status qg_apply_fp64_ops(qg_context ctx, qg_operator op, qg_basis 
   unsigned long long h = 0;
   if (e == cudaSuccess) e = cudaMemcpyAsync(&h, d, 8, cudaMemcpyDeviceToHost, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-  cudaFree(d);
+  qg_free(d);
   if (e != cudaSuccess) return qg_cuda_fail(ctx, e, "qg_apply_fp64_ops");
   *ops = (int64_t)h;
   return QG_OK;

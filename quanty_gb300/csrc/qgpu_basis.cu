@@ -172,17 +172,17 @@ static qg_status build_hash_t(qg_basis b) {
   qg_context ctx = b->ctx;
   int64_t hcap = hcap_for(b->n);
   if (b->d_slots && b->hcap != hcap) {
-    cudaFree(b->d_slots);
-    cudaFree(b->d_slot_row);
+    qg_free(b->d_slots);
+    qg_free(b->d_slot_row);
     b->d_slots = nullptr;
     b->d_slot_row = nullptr;
   }
   cudaError_t e = cudaSuccess;
   if (!b->d_slots) {
-    e = cudaMalloc(&b->d_slots, hcap * sizeof(Slot));
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_slot_row, hcap * sizeof(uint32_t));
+    e = qg_malloc(ctx, &b->d_slots, hcap * sizeof(Slot));
+    if (e == cudaSuccess) e = qg_malloc(ctx, &b->d_slot_row, hcap * sizeof(uint32_t));
   }
-  if (e == cudaSuccess && !b->d_row_slot) e = cudaMalloc(&b->d_row_slot, std::max<int64_t>(b->n, 1) * sizeof(uint32_t));
+  if (e == cudaSuccess && !b->d_row_slot) e = qg_malloc(ctx, &b->d_row_slot, std::max<int64_t>(b->n, 1) * sizeof(uint32_t));
   if (e != cudaSuccess) return qg_cuda_fail(ctx, e, "hash table");
   b->hcap = hcap;
   k_slots_clear<<<grid_for(hcap), 256, 0, ctx->stream>>>(b->d_slots, b->d_slot_row, hcap);
@@ -221,7 +221,7 @@ static qg_status from_keys_t(qg_context ctx, int nf, void *d_keys_in, int64_t n,
   cudaError_t e = cudaSuccess;
   int64_t nn = std::max<int64_t>(n, 1);
 #define ALLOC(p, bytes) \
-  if (e == cudaSuccess) e = cudaMalloc((void **)&p, bytes)
+  if (e == cudaSuccess) e = qg_malloc(ctx, &p, bytes)
   ALLOC(idx, nn * 4);
   ALLOC(idx2, nn * 4);
   ALLOC(flag, nn * 4);
@@ -266,23 +266,23 @@ static qg_status from_keys_t(qg_context ctx, int nf, void *d_keys_in, int64_t n,
       if (e == cudaSuccess) e = cudaStreamSynchronize(s);
       nuniq = last;
     }
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_keys, std::max<int64_t>(nuniq, 1) * sizeof(Key<W>));
+    if (e == cudaSuccess) e = qg_malloc(ctx, &b->d_keys, std::max<int64_t>(nuniq, 1) * sizeof(Key<W>));
     if (e == cudaSuccess) {
       k_compact_unique<W><<<grid_for(n), 256, 0, s>>>(sorted, flag, pos, idx, n, (Key<W> *)b->d_keys, d_perm);
       ctx->launches++;
     }
   } else if (e == cudaSuccess) {
-    e = cudaMalloc(&b->d_keys, sizeof(Key<W>));
+    e = qg_malloc(ctx, &b->d_keys, sizeof(Key<W>));
   }
   cudaStreamSynchronize(s);
-  cudaFree(idx);
-  cudaFree(idx2);
-  cudaFree(flag);
-  cudaFree(pos);
-  cudaFree(w);
-  cudaFree(w2);
-  cudaFree(sorted);
-  cudaFree(tmp);
+  qg_free(idx);
+  qg_free(idx2);
+  qg_free(flag);
+  qg_free(pos);
+  qg_free(w);
+  qg_free(w2);
+  qg_free(sorted);
+  qg_free(tmp);
   if (e != cudaSuccess) {
     qg_basis_destroy(b);
     return qg_cuda_fail(ctx, e, "basis sort");
@@ -314,9 +314,9 @@ extern "C" qg_status qg_basis_create(qg_context ctx, int32_t nf, int64_t n, cons
   void *d_keys = nullptr;
   int64_t *d_perm = nullptr;
   int64_t nn = std::max<int64_t>(n, 1);
-  QG_CUDA(ctx, cudaMalloc(&d_bytes, nn * nword));
-  QG_CUDA(ctx, cudaMalloc(&d_keys, nn * 8 * W));
-  if (perm_host) QG_CUDA(ctx, cudaMalloc(&d_perm, nn * 8));
+  QG_CUDA(ctx, qg_malloc(ctx, &d_bytes, nn * nword));
+  QG_CUDA(ctx, qg_malloc(ctx, &d_keys, nn * 8 * W));
+  if (perm_host) QG_CUDA(ctx, qg_malloc(ctx, &d_perm, nn * 8));
   if (n) QG_CUDA(ctx, cudaMemcpyAsync(d_bytes, dets_host, n * nword, cudaMemcpyHostToDevice, s));
   if (n) {
     if (W == 1)
@@ -332,22 +332,22 @@ extern "C" qg_status qg_basis_create(qg_context ctx, int32_t nf, int64_t n, cons
     if (e != cudaSuccess) st = qg_cuda_fail(ctx, e, "perm copy");
   }
   cudaStreamSynchronize(s);
-  cudaFree(d_bytes);
-  cudaFree(d_keys);
-  cudaFree(d_perm);
+  qg_free(d_bytes);
+  qg_free(d_keys);
+  qg_free(d_perm);
   if (st == QG_OK) st = qg_check_device_error(ctx, "qg_basis_create");
   return st;
 }
 
 extern "C" qg_status qg_basis_destroy(qg_basis b) {
   if (!b) return QG_OK;
-  cudaFree(b->d_keys);
-  cudaFree(b->d_slots);
-  cudaFree(b->d_slot_row);
-  cudaFree(b->d_row_slot);
-  cudaFree(b->d_rmask);
-  cudaFree(b->d_rmin);
-  cudaFree(b->d_rmax);
+  qg_free_now(b->d_keys);  // waits for the device: another context may still be using the basis
+  qg_free(b->d_slots);
+  qg_free(b->d_slot_row);
+  qg_free(b->d_row_slot);
+  qg_free(b->d_rmask);
+  qg_free(b->d_rmin);
+  qg_free(b->d_rmax);
   for (auto &c : b->caches) qg_cache_free(c);
   delete b;
   return QG_OK;
@@ -356,19 +356,19 @@ extern "C" qg_status qg_basis_destroy(qg_basis b) {
 qg_status qg_basis_set_windows(qg_basis b, int nres, const uint64_t *mask_host, const int32_t *min_host,
                                const int32_t *max_host) {
   qg_context ctx = b->ctx;
-  cudaFree(b->d_rmask);
-  cudaFree(b->d_rmin);
-  cudaFree(b->d_rmax);
+  qg_free(b->d_rmask);
+  qg_free(b->d_rmin);
+  qg_free(b->d_rmax);
   b->d_rmask = nullptr;
   b->d_rmin = b->d_rmax = nullptr;
   b->nres = 0;
   if (nres <= 0) return QG_OK;
-  QG_CUDA(ctx, cudaMalloc(&b->d_rmask, (size_t)nres * b->W * 8));
-  QG_CUDA(ctx, cudaMalloc(&b->d_rmin, nres * 4));
-  QG_CUDA(ctx, cudaMalloc(&b->d_rmax, nres * 4));
-  QG_CUDA(ctx, cudaMemcpy(b->d_rmask, mask_host, (size_t)nres * b->W * 8, cudaMemcpyHostToDevice));
-  QG_CUDA(ctx, cudaMemcpy(b->d_rmin, min_host, nres * 4, cudaMemcpyHostToDevice));
-  QG_CUDA(ctx, cudaMemcpy(b->d_rmax, max_host, nres * 4, cudaMemcpyHostToDevice));
+  QG_CUDA(ctx, qg_malloc(ctx, &b->d_rmask, (size_t)nres * b->W * 8));
+  QG_CUDA(ctx, qg_malloc(ctx, &b->d_rmin, nres * 4));
+  QG_CUDA(ctx, qg_malloc(ctx, &b->d_rmax, nres * 4));
+  QG_CUDA(ctx, qg_upload(ctx, b->d_rmask, mask_host, (size_t)nres * b->W * 8));
+  QG_CUDA(ctx, qg_upload(ctx, b->d_rmin, min_host, nres * 4));
+  QG_CUDA(ctx, qg_upload(ctx, b->d_rmax, max_host, nres * 4));
   b->nres = nres;
   b->h_rmask.assign(mask_host, mask_host + (size_t)nres * b->W);
   b->h_rmin.assign(min_host, min_host + nres);
@@ -384,7 +384,7 @@ extern "C" qg_status qg_basis_get_dets(qg_basis b, uint8_t *dets_host) {
   int nword = (b->nf + 7) / 8;
   if (!b->n) return QG_OK;
   uint8_t *d = nullptr;
-  QG_CUDA(ctx, cudaMalloc(&d, b->n * nword));
+  QG_CUDA(ctx, qg_malloc(ctx, &d, b->n * nword));
   if (b->W == 1)
     k_keys_to_bytes<1><<<grid_for(b->n), 256, 0, ctx->stream>>>((const Key<1> *)b->d_keys, b->nf, nword, b->n, d);
   else
@@ -392,7 +392,7 @@ extern "C" qg_status qg_basis_get_dets(qg_basis b, uint8_t *dets_host) {
   ctx->launches++;
   cudaError_t e = cudaMemcpyAsync(dets_host, d, b->n * nword, cudaMemcpyDeviceToHost, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-  cudaFree(d);
+  qg_free(d);
   if (e != cudaSuccess) return qg_cuda_fail(ctx, e, "qg_basis_get_dets");
   return QG_OK;
 }
@@ -414,9 +414,9 @@ extern "C" qg_status qg_basis_find(qg_basis b, int64_t n, const uint8_t *dets_ho
   uint8_t *d_bytes = nullptr;
   void *d_keys = nullptr;
   int64_t *d_out = nullptr;
-  QG_CUDA(ctx, cudaMalloc(&d_bytes, n * nword));
-  QG_CUDA(ctx, cudaMalloc(&d_keys, n * 8 * b->W));
-  QG_CUDA(ctx, cudaMalloc(&d_out, n * 8));
+  QG_CUDA(ctx, qg_malloc(ctx, &d_bytes, n * nword));
+  QG_CUDA(ctx, qg_malloc(ctx, &d_keys, n * 8 * b->W));
+  QG_CUDA(ctx, qg_malloc(ctx, &d_out, n * 8));
   QG_CUDA(ctx, cudaMemcpyAsync(d_bytes, dets_host, n * nword, cudaMemcpyHostToDevice, s));
   if (b->W == 1) {
     k_bytes_to_keys<1><<<grid_for(n), 256, 0, s>>>(d_bytes, b->nf, nword, n, (Key<1> *)d_keys);
@@ -430,9 +430,9 @@ extern "C" qg_status qg_basis_find(qg_basis b, int64_t n, const uint8_t *dets_ho
   ctx->launches += 2;
   cudaError_t e = cudaMemcpyAsync(index_host, d_out, n * 8, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  cudaFree(d_bytes);
-  cudaFree(d_keys);
-  cudaFree(d_out);
+  qg_free(d_bytes);
+  qg_free(d_keys);
+  qg_free(d_out);
   if (e != cudaSuccess) return qg_cuda_fail(ctx, e, "qg_basis_find");
   return qg_check_device_error(ctx, "qg_basis_find");
 }
@@ -659,15 +659,15 @@ static qg_status grow_t(qg_context ctx, qg_operator op, const Key<W> *seed_keys,
     if (!exact) twreq.clear();
   }
   if (R.n) {
-    QG_CUDA(ctx, cudaMalloc(&d_rmask, R.mask.size() * 8));
-    QG_CUDA(ctx, cudaMalloc(&d_rmin, R.n * 4));
-    QG_CUDA(ctx, cudaMalloc(&d_rmax, R.n * 4));
-    QG_CUDA(ctx, cudaMemcpy(d_rmask, R.mask.data(), R.mask.size() * 8, cudaMemcpyHostToDevice));
-    QG_CUDA(ctx, cudaMemcpy(d_rmin, R.mn.data(), R.n * 4, cudaMemcpyHostToDevice));
-    QG_CUDA(ctx, cudaMemcpy(d_rmax, R.mx.data(), R.n * 4, cudaMemcpyHostToDevice));
+    QG_CUDA(ctx, qg_malloc(ctx, &d_rmask, R.mask.size() * 8));
+    QG_CUDA(ctx, qg_malloc(ctx, &d_rmin, R.n * 4));
+    QG_CUDA(ctx, qg_malloc(ctx, &d_rmax, R.n * 4));
+    QG_CUDA(ctx, qg_upload(ctx, d_rmask, R.mask.data(), R.mask.size() * 8));
+    QG_CUDA(ctx, qg_upload(ctx, d_rmin, R.mn.data(), R.n * 4));
+    QG_CUDA(ctx, qg_upload(ctx, d_rmax, R.mx.data(), R.n * 4));
     if (!twreq.empty()) {
-      QG_CUDA(ctx, cudaMalloc(&d_twreq, twreq.size() * 8));
-      QG_CUDA(ctx, cudaMemcpy(d_twreq, twreq.data(), twreq.size() * 8, cudaMemcpyHostToDevice));
+      QG_CUDA(ctx, qg_malloc(ctx, &d_twreq, twreq.size() * 8));
+      QG_CUDA(ctx, qg_upload(ctx, d_twreq, twreq.data(), twreq.size() * 8));
     }
   }
   // list capacity; the set has 2*cap slots.  An expansion stops inserting once the list is
@@ -679,17 +679,17 @@ static qg_status grow_t(qg_context ctx, qg_operator op, const Key<W> *seed_keys,
   Slot *slots = nullptr;
   unsigned long long *d_count = nullptr;
   qg_status st = QG_OK;
-  cudaError_t e = cudaMalloc(&d_count, 8);
+  cudaError_t e = qg_malloc(ctx, &d_count, 8);
   auto alloc_table = [&](int64_t c) -> cudaError_t {
-    cudaFree(slots);
+    qg_free(slots);
     slots = nullptr;
-    cudaError_t ee = cudaMalloc(&slots, 2 * c * sizeof(Slot));
+    cudaError_t ee = qg_malloc(ctx, &slots, 2 * c * sizeof(Slot));
     if (ee != cudaSuccess) return ee;
     k_slots_clear<<<grid_for(2 * c), 256, 0, s>>>(slots, nullptr, 2 * c);
     ctx->launches++;
     return cudaGetLastError();
   };
-  if (e == cudaSuccess) e = cudaMalloc(&list, cap * sizeof(Key<W>));
+  if (e == cudaSuccess) e = qg_malloc(ctx, &list, cap * sizeof(Key<W>));
   if (e == cudaSuccess) e = alloc_table(cap);
   unsigned long long count = 0;
   if (e == cudaSuccess && include_seed && n_seed) {
@@ -734,12 +734,12 @@ static qg_status grow_t(qg_context ctx, qg_operator op, const Key<W> *seed_keys,
       int64_t ncap = cap;
       while (ncap < 2 * (int64_t)count + 1024) ncap <<= 1;
       Key<W> *nlist = nullptr;
-      e = cudaMalloc(&nlist, ncap * sizeof(Key<W>));
+      e = qg_malloc(ctx, &nlist, ncap * sizeof(Key<W>));
       if (e != cudaSuccess) break;
       e = cudaMemcpyAsync(nlist, list, kept * sizeof(Key<W>), cudaMemcpyDeviceToDevice, s);
       if (e != cudaSuccess) break;
       cudaStreamSynchronize(s);
-      cudaFree(list);
+      qg_free(list);
       list = nlist;
       if (include_seed) front = list;
       cap = ncap;
@@ -768,13 +768,13 @@ static qg_status grow_t(qg_context ctx, qg_operator op, const Key<W> *seed_keys,
     if (include_seed && n_seed) {
       unsigned long long *d_bad = nullptr;
       unsigned long long bad = 0;
-      if (cudaMalloc(&d_bad, 8) == cudaSuccess) {
+      if (qg_malloc(ctx, &d_bad, 8) == cudaSuccess) {
         cudaMemsetAsync(d_bad, 0, 8, s);
         k_count_outside<W><<<grid_for(n_seed), 256, 0, s>>>(seed_keys, n_seed, R.n, d_rmask, d_rmin, d_rmax, d_bad);
         ctx->launches++;
         cudaMemcpyAsync(&bad, d_bad, 8, cudaMemcpyDeviceToHost, s);
         cudaStreamSynchronize(s);
-        cudaFree(d_bad);
+        qg_free(d_bad);
         seeds_ok = (bad == 0);
       } else {
         seeds_ok = false;
@@ -783,13 +783,13 @@ static qg_status grow_t(qg_context ctx, qg_operator op, const Key<W> *seed_keys,
     if (seeds_ok) st = qg_basis_set_windows(*out, R.n, R.mask.data(), R.mn.data(), R.mx.data());
   }
   cudaStreamSynchronize(s);
-  cudaFree(list);
-  cudaFree(slots);
-  cudaFree(d_count);
-  cudaFree(d_rmask);
-  cudaFree(d_rmin);
-  cudaFree(d_rmax);
-  cudaFree(d_twreq);
+  qg_free(list);
+  qg_free(slots);
+  qg_free(d_count);
+  qg_free(d_rmask);
+  qg_free(d_rmin);
+  qg_free(d_rmax);
+  qg_free(d_twreq);
   if (rounds_done) *rounds_done = rounds;
   return st;
 }
@@ -819,12 +819,12 @@ extern "C" qg_status qg_basis_union(qg_context ctx, qg_basis a, qg_basis b, qg_b
   int W = a->W;
   void *d = nullptr;
   int64_t n = a->n + b->n;
-  QG_CUDA(ctx, cudaMalloc(&d, std::max<int64_t>(n, 1) * 8 * W));
+  QG_CUDA(ctx, qg_malloc(ctx, &d, std::max<int64_t>(n, 1) * 8 * W));
   QG_CUDA(ctx, cudaMemcpyAsync(d, a->d_keys, a->n * 8 * W, cudaMemcpyDeviceToDevice, ctx->stream));
   QG_CUDA(ctx, cudaMemcpyAsync((char *)d + a->n * 8 * W, b->d_keys, b->n * 8 * W, cudaMemcpyDeviceToDevice, ctx->stream));
   qg_status st = qg_basis_from_device_keys(ctx, a->nf, W, d, n, out, nullptr);
   cudaStreamSynchronize(ctx->stream);
-  cudaFree(d);
+  qg_free(d);
   return st;
 }
 

@@ -158,12 +158,12 @@ extern "C" qg_status qg_block_lanczos(qg_context ctx, qg_operator op, qg_basis b
   double2 *Qp = nullptr, *Q = nullptr, *W = nullptr, *T = nullptr;
   const size_t vb = (size_t)n * m * 16;
   bc.work_elems = std::max<int64_t>(64 * (int64_t)mm, 1 << 16);
-  cudaError_t e = cudaMalloc(&Qp, vb);
-  if (e == cudaSuccess) e = cudaMalloc(&Q, vb);
-  if (e == cudaSuccess) e = cudaMalloc(&W, vb);
-  if (e == cudaSuccess) e = cudaMalloc(&T, vb);
-  if (e == cudaSuccess) e = cudaMalloc(&bc.work, (size_t)bc.work_elems * 16);
-  if (e == cudaSuccess) e = cudaMalloc(&bc.C, mm * 16);
+  cudaError_t e = qg_malloc(ctx, &Qp, vb);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &Q, vb);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &W, vb);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &T, vb);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &bc.work, (size_t)bc.work_elems * 16);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &bc.C, mm * 16);
   qg_status st = e == cudaSuccess ? QG_OK : QG_ERR_OOM;
   if (st != QG_OK) ctx->last_error = "qg_block_lanczos: out of device memory";
   if (st == QG_OK) {
@@ -231,12 +231,12 @@ extern "C" qg_status qg_block_lanczos(qg_context ctx, qg_operator op, qg_basis b
     e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) st = qg_cuda_fail(ctx, e, "qg_block_lanczos");
   }
-  cudaFree(Qp);
-  cudaFree(Q);
-  cudaFree(W);
-  cudaFree(T);
-  cudaFree(bc.work);
-  cudaFree(bc.C);
+  qg_free(Qp);
+  qg_free(Q);
+  qg_free(W);
+  qg_free(T);
+  qg_free(bc.work);
+  qg_free(bc.C);
   if (st != QG_OK) return st;
   std::copy(A.begin(), A.end(), (cd *)a_host);
   std::copy(B.begin(), B.end(), (cd *)b_host);
@@ -355,9 +355,9 @@ extern "C" qg_status qg_block_cf_spectra(qg_context ctx, int32_t m, int32_t ntri
   const size_t mm = (size_t)m * m;
   double2 *a = nullptr, *b = nullptr, *g = nullptr;
   const size_t ab = (size_t)(ntri + 1) * mm * 16, bb = (size_t)ntri * mm * 16, gb = mm * (ne + 1) * 16;
-  cudaError_t e = cudaMalloc(&a, ab);
-  if (e == cudaSuccess) e = cudaMalloc(&b, bb);
-  if (e == cudaSuccess) e = cudaMalloc(&g, gb);
+  cudaError_t e = qg_malloc(ctx, &a, ab);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &b, bb);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &g, gb);
   if (e == cudaSuccess) e = cudaMemcpyAsync(a, a_host, ab, cudaMemcpyHostToDevice, ctx->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(b, b_host, bb, cudaMemcpyHostToDevice, ctx->stream);
   qg_status st = e == cudaSuccess ? QG_OK : qg_cuda_fail(ctx, e, "qg_block_cf_spectra");
@@ -371,8 +371,8 @@ extern "C" qg_status qg_block_cf_spectra(qg_context ctx, int32_t m, int32_t ntri
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) st = qg_cuda_fail(ctx, e, "qg_block_cf_spectra");
   }
-  cudaFree(a);
-  cudaFree(b);
-  cudaFree(g);
+  qg_free(a);
+  qg_free(b);
+  qg_free(g);
   return st;
 }

@@ -224,7 +224,7 @@ extern "C" qg_status qg_krylov_combine(qg_context ctx, const double *K_dev, int6
   if (!ctx || n < 0 || nk < 0 || np <= 0 || (n > 0 && (!K_dev || !out_dev)) || (nk > 0 && !C_host)) return QG_ERR_ARG;
   if (n == 0) return QG_OK;
   double2 *Cd = nullptr;
-  QG_CUDA(ctx, cudaMalloc(&Cd, (size_t)std::max(nk, 1) * np * 16));
+  QG_CUDA(ctx, qg_malloc(ctx, &Cd, (size_t)std::max(nk, 1) * np * 16));
   cudaError_t e = cudaMemcpyAsync(Cd, C_host, (size_t)nk * np * 16, cudaMemcpyHostToDevice, ctx->stream);
   qg_status st = e == cudaSuccess ? qg_block_combine(ctx, (const double2 *)K_dev, n, nk, Cd, np, (double2 *)out_dev)
                                   : qg_cuda_fail(ctx, e, "qg_krylov_combine");
@@ -232,7 +232,7 @@ extern "C" qg_status qg_krylov_combine(qg_context ctx, const double *K_dev, int6
     e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) st = qg_cuda_fail(ctx, e, "qg_krylov_combine");
   }
-  cudaFree(Cd);
+  qg_free(Cd);
   return st;
 }
 
@@ -247,11 +247,11 @@ extern "C" qg_status qg_block_adjoint_product(qg_context ctx, const double *A_de
   // partial tiles of up to 64 row chunks, at most 256 MB of them
   const int64_t work = std::max<int64_t>(m, std::min<int64_t>(64 * m, (256LL << 20) / 16));
   double2 *w = nullptr;
-  QG_CUDA(ctx, cudaMalloc(&w, (size_t)work * 16));
+  QG_CUDA(ctx, qg_malloc(ctx, &w, (size_t)work * 16));
   qg_status st = qg_block_gram(ctx, (const double2 *)A_dev, lda, ka, (const double2 *)B_dev, ldb, kb, n,
                                (double2 *)C_dev, w, work);
   cudaStreamSynchronize(ctx->stream);
-  cudaFree(w);
+  qg_free(w);
   return st;
 }
 

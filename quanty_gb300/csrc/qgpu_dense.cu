@@ -47,11 +47,11 @@ extern "C" qg_status qg_operator_dense(qg_context ctx, qg_operator op, qg_basis 
     return QG_ERR_ARG;
   }
   double2 *I = nullptr, *M = nullptr;
-  cudaError_t e = cudaMalloc(&I, (size_t)n * n * 16);
-  if (e == cudaSuccess) e = cudaMalloc(&M, (size_t)n * n * 16);
+  cudaError_t e = qg_malloc(ctx, &I, (size_t)n * n * 16);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &M, (size_t)n * n * 16);
   if (e != cudaSuccess) {
-    cudaFree(I);
-    cudaFree(M);
+    qg_free(I);
+    qg_free(M);
     ctx->last_error = "qg_operator_dense: out of device memory";
     return QG_ERR_OOM;
   }
@@ -65,8 +65,8 @@ extern "C" qg_status qg_operator_dense(qg_context ctx, qg_operator op, qg_basis 
     if (e != cudaSuccess) st = qg_cuda_fail(ctx, e, "qg_operator_dense");
   }
   cudaStreamSynchronize(ctx->stream);
-  cudaFree(I);
-  cudaFree(M);
+  qg_free(I);
+  qg_free(M);
   if (st == QG_OK) st = qg_check_device_error(ctx, "qg_operator_dense");
   return st;
 }
@@ -81,10 +81,10 @@ extern "C" qg_status qg_poles_spectra(qg_context ctx, int32_t nspec, int32_t npo
   size_t pb = (size_t)nspec * std::max(npole, 1) * 8, gb = (size_t)nspec * (ne + 1) * 16;
   double *da = nullptr, *db = nullptr, *de0 = nullptr;
   double2 *dg = nullptr;
-  cudaError_t e = cudaMalloc(&da, pb);
-  if (e == cudaSuccess) e = cudaMalloc(&db, pb);
-  if (e == cudaSuccess) e = cudaMalloc(&de0, (size_t)nspec * 8);
-  if (e == cudaSuccess) e = cudaMalloc(&dg, gb);
+  cudaError_t e = qg_malloc(ctx, &da, pb);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &db, pb);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &de0, (size_t)nspec * 8);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &dg, gb);
   if (e == cudaSuccess && npole) e = cudaMemcpyAsync(da, a_host, (size_t)nspec * npole * 8, cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess && npole) e = cudaMemcpyAsync(db, b_host, (size_t)nspec * npole * 8, cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(de0, e0_host, (size_t)nspec * 8, cudaMemcpyHostToDevice, s);
@@ -99,9 +99,9 @@ extern "C" qg_status qg_poles_spectra(qg_context ctx, int32_t nspec, int32_t npo
   }
   if (e != cudaSuccess && st == QG_OK) st = qg_cuda_fail(ctx, e, "qg_poles_spectra");
   cudaStreamSynchronize(s);
-  cudaFree(da);
-  cudaFree(db);
-  cudaFree(de0);
-  cudaFree(dg);
+  qg_free(da);
+  qg_free(db);
+  qg_free(de0);
+  qg_free(dg);
   return st;
 }

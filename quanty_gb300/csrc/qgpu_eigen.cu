@@ -212,13 +212,13 @@ struct Gram {
     // one-column kernels), or the row-chunk tiles of a block product (qg_block_gram uses as many
     // chunks as fit, at most the few dozen that fill the SMs)
     part_elems = std::max<int64_t>(std::max<int64_t>(nchunk * (int64_t)kcol, (int64_t)nblk * 32 * QG_GRAM_LANE_COLS), 16 * (int64_t)maxm);
-    QG_CUDA(ctx, cudaMalloc(&part, (size_t)part_elems * 16));
-    QG_CUDA(ctx, cudaMalloc(&out, (size_t)maxm * 16));
+    QG_CUDA(ctx, qg_malloc(ctx, &part, (size_t)part_elems * 16));
+    QG_CUDA(ctx, qg_malloc(ctx, &out, (size_t)maxm * 16));
     return QG_OK;
   }
   void release() {
-    cudaFree(part);
-    cudaFree(out);
+    qg_free(part);
+    qg_free(out);
   }
   template <bool REAL>
   void col_gram(cudaStream_t s, const double2 *A, int lda, int a0, int ka, const double2 *B, int ldb, int b0) {
@@ -273,7 +273,7 @@ struct Gram {
 qg_status qg_all_real(qg_context ctx, const double2 *v, int64_t n, bool *real) {
   unsigned int *d_im = nullptr, h_im = 1;
   cudaStream_t s = ctx->stream;
-  cudaError_t e = cudaMalloc(&d_im, sizeof(unsigned int));
+  cudaError_t e = qg_malloc(ctx, &d_im, sizeof(unsigned int));
   if (e == cudaSuccess) e = cudaMemsetAsync(d_im, 0, sizeof(unsigned int), s);
   if (e == cudaSuccess) {
     k_any_imag<<<(unsigned)std::min<int64_t>((n + 255) / 256, 4LL * ctx->num_sms), 256, 0, s>>>(v, n, d_im);
@@ -281,7 +281,7 @@ qg_status qg_all_real(qg_context ctx, const double2 *v, int64_t n, bool *real) {
     e = cudaMemcpyAsync(&h_im, d_im, sizeof(unsigned int), cudaMemcpyDeviceToHost, s);
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  cudaFree(d_im);
+  qg_free(d_im);
   if (e != cudaSuccess) return qg_cuda_fail(ctx, e, "qg_block_groundstate");
   *real = h_im == 0;
   return QG_OK;
@@ -448,21 +448,21 @@ static qg_status groundstate_one(qg_context ctx, qg_operator op, qg_basis b, dou
   double *npart = nullptr, *sub = nullptr, *wd = nullptr, *zero = nullptr;
   double2 *dpart = nullptr, *Md = nullptr, *Y = nullptr;
   OneScal *sc = nullptr;
-  cudaError_t e = cudaMalloc(&V, (size_t)n * K * sizeof(T));
-  if (e == cudaSuccess) e = cudaMalloc(&w, (size_t)n * sizeof(T));
-  if (e == cudaSuccess) e = cudaMalloc(&wo, (size_t)n * sizeof(T));
-  if (e == cudaSuccess) e = cudaMalloc(&x, (size_t)n * sizeof(T));
-  if (e == cudaSuccess) e = cudaMalloc(&part, (size_t)gp * K * sizeof(T));
-  if (e == cudaSuccess) e = cudaMalloc(&c, (size_t)K * sizeof(T));
-  if (e == cudaSuccess) e = cudaMalloc(&ct, (size_t)K * K * sizeof(T));
-  if (e == cudaSuccess) e = cudaMalloc(&npart, (size_t)gu * sizeof(double));
-  if (e == cudaSuccess) e = cudaMalloc(&sub, (size_t)K * sizeof(double));
-  if (e == cudaSuccess) e = cudaMalloc(&wd, (size_t)K * sizeof(double));
-  if (e == cudaSuccess) e = cudaMalloc(&zero, sizeof(double));
-  if (e == cudaSuccess) e = cudaMalloc(&dpart, (size_t)Pa * 16);
-  if (e == cudaSuccess) e = cudaMalloc(&Md, (size_t)K * K * 16);
-  if (e == cudaSuccess) e = cudaMalloc(&Y, (size_t)K * 16);
-  if (e == cudaSuccess) e = cudaMalloc(&sc, sizeof(OneScal));
+  cudaError_t e = qg_malloc(ctx, &V, (size_t)n * K * sizeof(T));
+  if (e == cudaSuccess) e = qg_malloc(ctx, &w, (size_t)n * sizeof(T));
+  if (e == cudaSuccess) e = qg_malloc(ctx, &wo, (size_t)n * sizeof(T));
+  if (e == cudaSuccess) e = qg_malloc(ctx, &x, (size_t)n * sizeof(T));
+  if (e == cudaSuccess) e = qg_malloc(ctx, &part, (size_t)gp * K * sizeof(T));
+  if (e == cudaSuccess) e = qg_malloc(ctx, &c, (size_t)K * sizeof(T));
+  if (e == cudaSuccess) e = qg_malloc(ctx, &ct, (size_t)K * K * sizeof(T));
+  if (e == cudaSuccess) e = qg_malloc(ctx, &npart, (size_t)gu * sizeof(double));
+  if (e == cudaSuccess) e = qg_malloc(ctx, &sub, (size_t)K * sizeof(double));
+  if (e == cudaSuccess) e = qg_malloc(ctx, &wd, (size_t)K * sizeof(double));
+  if (e == cudaSuccess) e = qg_malloc(ctx, &zero, sizeof(double));
+  if (e == cudaSuccess) e = qg_malloc(ctx, &dpart, (size_t)Pa * 16);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &Md, (size_t)K * K * 16);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &Y, (size_t)K * 16);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &sc, sizeof(OneScal));
   if (e == cudaSuccess) e = cudaMemsetAsync(zero, 0, sizeof(double), s);
   qg_status st = QG_OK;
   if (e != cudaSuccess) {
@@ -552,21 +552,21 @@ static qg_status groundstate_one(qg_context ctx, qg_operator op, qg_basis b, dou
     st = qg_check_launch(ctx, "qg_block_groundstate");
   }
   cudaStreamSynchronize(s);
-  cudaFree(V);
-  cudaFree(w);
-  cudaFree(wo);
-  cudaFree(x);
-  cudaFree(part);
-  cudaFree(c);
-  cudaFree(ct);
-  cudaFree(npart);
-  cudaFree(sub);
-  cudaFree(wd);
-  cudaFree(zero);
-  cudaFree(dpart);
-  cudaFree(Md);
-  cudaFree(Y);
-  cudaFree(sc);
+  qg_free(V);
+  qg_free(w);
+  qg_free(wo);
+  qg_free(x);
+  qg_free(part);
+  qg_free(c);
+  qg_free(ct);
+  qg_free(npart);
+  qg_free(sub);
+  qg_free(wd);
+  qg_free(zero);
+  qg_free(dpart);
+  qg_free(Md);
+  qg_free(Y);
+  qg_free(sc);
   return st;
 }
 
@@ -606,21 +606,21 @@ extern "C" qg_status qg_block_groundstate(qg_context ctx, qg_operator op, qg_bas
   double2 *V = nullptr, *W = nullptr, *Cd = nullptr, *X = nullptr, *Md = nullptr, *Sd = nullptr;
   double *wd = nullptr;
   size_t vb = (size_t)n * K * 16, wb = (size_t)n * p * 16;
-  cudaError_t e = cudaMalloc(&V, vb);
-  if (e == cudaSuccess) e = cudaMalloc(&W, wb);
-  if (e == cudaSuccess) e = cudaMalloc(&X, wb);
-  if (e == cudaSuccess) e = cudaMalloc(&Cd, (size_t)K * std::max(K, p) * 16);
-  if (e == cudaSuccess) e = cudaMalloc(&Md, (size_t)K * K * 16);
-  if (e == cudaSuccess) e = cudaMalloc(&wd, (size_t)K * sizeof(double));
-  if (e == cudaSuccess) e = cudaMalloc(&Sd, (size_t)p * p * 16);
+  cudaError_t e = qg_malloc(ctx, &V, vb);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &W, wb);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &X, wb);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &Cd, (size_t)K * std::max(K, p) * 16);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &Md, (size_t)K * K * 16);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &wd, (size_t)K * sizeof(double));
+  if (e == cudaSuccess) e = qg_malloc(ctx, &Sd, (size_t)p * p * 16);
   if (e != cudaSuccess) {
-    cudaFree(V);
-    cudaFree(W);
-    cudaFree(X);
-    cudaFree(Cd);
-    cudaFree(Md);
-    cudaFree(wd);
-    cudaFree(Sd);
+    qg_free(V);
+    qg_free(W);
+    qg_free(X);
+    qg_free(Cd);
+    qg_free(Md);
+    qg_free(wd);
+    qg_free(Sd);
     ctx->last_error = "qg_block_groundstate: out of device memory";
     return QG_ERR_OOM;
   }
@@ -858,13 +858,13 @@ extern "C" qg_status qg_block_groundstate(qg_context ctx, qg_operator op, qg_bas
     ctx->launches++;
   }
   cudaStreamSynchronize(s);
-  cudaFree(V);
-  cudaFree(W);
-  cudaFree(X);
-  cudaFree(Cd);
-  cudaFree(Md);
-  cudaFree(wd);
-  cudaFree(Sd);
+  qg_free(V);
+  qg_free(W);
+  qg_free(X);
+  qg_free(Cd);
+  qg_free(Md);
+  qg_free(wd);
+  qg_free(Sd);
   for (int j = 0; j < nwant; j++) energies_host[j] = theta[j];
   if (iterations) *iterations = it;
   if (st == QG_OK) st = qg_check_device_error(ctx, "qg_block_groundstate");

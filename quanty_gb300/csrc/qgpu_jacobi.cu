@@ -206,7 +206,7 @@ qg_status qg_eigh_device(qg_context ctx, int k, double2 *A, double *w_dev, doubl
   if (nv < 0 || nv > k) return QG_ERR_ARG;
   cudaStream_t s = ctx->stream;
   int *d_status = nullptr;
-  QG_CUDA(ctx, cudaMalloc(&d_status, sizeof(int)));
+  QG_CUDA(ctx, qg_malloc(ctx, &d_status, sizeof(int)));
   qg_status st = QG_OK;
   int sweeps = 0;
   if (k <= QG_JAC_SMALL) {
@@ -229,7 +229,7 @@ qg_status qg_eigh_device(qg_context ctx, int k, double2 *A, double *w_dev, doubl
   } else {
     st = qg_eigh_tridiag(ctx, k, A, w_dev, V_dev, nv);
   }
-  cudaFree(d_status);
+  qg_free(d_status);
   if (st == QG_OK && sweeps > QG_JAC_SWEEPS) {
     ctx->last_error = "qg_eigh_device: Jacobi did not converge";
     return QG_ERR_TIMEOUT;
@@ -243,9 +243,9 @@ qg_status qg_eigh_host_io(qg_context ctx, int k, const double *a_host, double *w
   double2 *A = nullptr, *V = nullptr;
   double *w = nullptr;
   const size_t ab = (size_t)k * k * sizeof(double2), vb = (size_t)k * std::max(nv, 1) * sizeof(double2);
-  cudaError_t e = cudaMalloc(&A, ab);
-  if (e == cudaSuccess) e = cudaMalloc(&V, vb);
-  if (e == cudaSuccess) e = cudaMalloc(&w, (size_t)k * sizeof(double));
+  cudaError_t e = qg_malloc(ctx, &A, ab);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &V, vb);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &w, (size_t)k * sizeof(double));
   if (e == cudaSuccess) e = cudaMemcpyAsync(A, a_host, ab, cudaMemcpyHostToDevice, ctx->stream);
   qg_status st = e == cudaSuccess ? QG_OK : qg_cuda_fail(ctx, e, "qg_hermitian_eigh");
   if (st == QG_OK) st = qg_eigh_device(ctx, k, A, w, V, nv);
@@ -256,9 +256,9 @@ qg_status qg_eigh_host_io(qg_context ctx, int k, const double *a_host, double *w
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) st = qg_cuda_fail(ctx, e, "qg_hermitian_eigh");
   }
-  cudaFree(A);
-  cudaFree(V);
-  cudaFree(w);
+  qg_free(A);
+  qg_free(V);
+  qg_free(w);
   return st;
 }
 

@@ -202,12 +202,12 @@ qg_status qg_dot_dev(qg_context ctx, int64_t n, int nvec, const double *x, const
 
 static qg_status dot_to_host(qg_context ctx, int64_t n, int nvec, const double *x, const double *y, double *host) {
   double2 *d = nullptr;
-  QG_CUDA(ctx, cudaMalloc(&d, nvec * 16));
+  QG_CUDA(ctx, qg_malloc(ctx, &d, nvec * 16));
   qg_status st = qg_dot_dev(ctx, n, nvec, x, y, (double *)d);
   cudaError_t e = cudaSuccess;
   if (st == QG_OK) e = cudaMemcpyAsync(host, d, nvec * 16, cudaMemcpyDeviceToHost, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-  cudaFree(d);
+  qg_free(d);
   if (st != QG_OK) return st;
   if (e != cudaSuccess) return qg_cuda_fail(ctx, e, "dot copy");
   return QG_OK;
@@ -242,7 +242,7 @@ extern "C" qg_status qg_axpy(qg_context ctx, int64_t n, int32_t nvec, const doub
   if (!ctx || n < 0 || nvec <= 0 || !alpha_host || (n && (!x || !y))) return QG_ERR_ARG;
   if (!n) return QG_OK;
   double2 *d = nullptr;
-  QG_CUDA(ctx, cudaMalloc(&d, nvec * 16));
+  QG_CUDA(ctx, qg_malloc(ctx, &d, nvec * 16));
   // every path from here frees d
   cudaError_t e = cudaMemcpyAsync(d, alpha_host, nvec * 16, cudaMemcpyHostToDevice, ctx->stream);
   if (e == cudaSuccess) {
@@ -252,7 +252,7 @@ extern "C" qg_status qg_axpy(qg_context ctx, int64_t n, int32_t nvec, const doub
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-  cudaFree(d);
+  qg_free(d);
   if (e != cudaSuccess) return qg_cuda_fail(ctx, e, "qg_axpy");
   return qg_check_launch(ctx, "qg_axpy");
 }
@@ -265,10 +265,10 @@ extern "C" qg_status qg_expectation(qg_context ctx, qg_operator op, qg_basis b, 
     return QG_OK;
   }
   double *y = nullptr;
-  QG_CUDA(ctx, cudaMalloc(&y, b->n * nvec * 16));
+  QG_CUDA(ctx, qg_malloc(ctx, &y, b->n * nvec * 16));
   qg_status st = qg_apply_launch(ctx, op, b, b, x, y, nvec, nullptr);
   if (st == QG_OK) st = dot_to_host(ctx, b->n, nvec, x, y, val_host);
-  cudaFree(y);
+  qg_free(y);
   return st;
 }
 
@@ -721,8 +721,8 @@ static qg_status lanczos_small(qg_context ctx, qg_operator op, qg_basis b, const
     attr = true;
   }
   double *ah = nullptr, *bh = nullptr;
-  cudaError_t e = cudaMalloc(&ah, (size_t)nvec * (ntri + 1) * sizeof(double));
-  if (e == cudaSuccess) e = cudaMalloc(&bh, (size_t)nvec * ntri * sizeof(double));
+  cudaError_t e = qg_malloc(ctx, &ah, (size_t)nvec * (ntri + 1) * sizeof(double));
+  if (e == cudaSuccess) e = qg_malloc(ctx, &bh, (size_t)nvec * ntri * sizeof(double));
   if (e == cudaSuccess) e = cudaMemsetAsync(ah, 0, (size_t)nvec * (ntri + 1) * sizeof(double), s);
   qg_status st = e == cudaSuccess ? QG_OK : qg_cuda_fail(ctx, e, "qg_lanczos_tridiag");
   if (st == QG_OK) {
@@ -745,8 +745,8 @@ static qg_status lanczos_small(qg_context ctx, qg_operator op, qg_basis b, const
     if (e != cudaSuccess) st = qg_cuda_fail(ctx, e, "qg_lanczos_tridiag");
   }
   cudaStreamSynchronize(s);
-  cudaFree(ah);
-  cudaFree(bh);
+  qg_free(ah);
+  qg_free(bh);
   qg_small_csr_free(csr);
   if (st == QG_OK) {
     for (int q = 0; q < nvec; q++) a_host[q * (ntri + 1)] = 0.0;
@@ -781,7 +781,7 @@ static qg_status lanczos_general(qg_context ctx, qg_operator op, qg_basis b, con
   size_t vb = std::max<int64_t>(len, 1) * 16;
   cudaError_t e = cudaSuccess;
 #define ALLOC(p, bytes) \
-  if (e == cudaSuccess) e = cudaMalloc((void **)&p, bytes)
+  if (e == cudaSuccess) e = qg_malloc(ctx, &p, bytes)
   ALLOC(vp, vb);
   ALLOC(vc, vb);
   ALLOC(w, vb);
@@ -795,8 +795,8 @@ static qg_status lanczos_general(qg_context ctx, qg_operator op, qg_basis b, con
   ALLOC(scal, nscal * 8);
 #undef ALLOC
   if (e != cudaSuccess) {
-    cudaFree(vp); cudaFree(vc); cudaFree(w); cudaFree(w2); cudaFree(vraw); cudaFree(zero);
-    cudaFree(npart); cudaFree(dpart); cudaFree(scal);
+    qg_free(vp); qg_free(vc); qg_free(w); qg_free(w2); qg_free(vraw); qg_free(zero);
+    qg_free(npart); qg_free(dpart); qg_free(scal);
     ctx->last_error = "qg_lanczos_tridiag: out of device memory";
     return QG_ERR_OOM;
   }
@@ -813,8 +813,8 @@ static qg_status lanczos_general(qg_context ctx, qg_operator op, qg_basis b, con
     if (me != cudaSuccess) st0 = qg_cuda_fail(ctx, me, "lanczos zero vector");
   }
   if (st0 != QG_OK) {
-    cudaFree(vp); cudaFree(vc); cudaFree(w); cudaFree(w2); cudaFree(vraw); cudaFree(zero);
-    cudaFree(npart); cudaFree(dpart); cudaFree(scal);
+    qg_free(vp); qg_free(vc); qg_free(w); qg_free(w2); qg_free(vraw); qg_free(zero);
+    qg_free(npart); qg_free(dpart); qg_free(scal);
     return st0;
   }
   // the normalised, truncated Krylov vector vc from a raw vector: for one vector the same
@@ -947,8 +947,8 @@ static qg_status lanczos_general(qg_context ctx, qg_operator op, qg_basis b, con
   }
   if (e != cudaSuccess && st == QG_OK) st = qg_cuda_fail(ctx, e, "qg_lanczos_tridiag");
   cudaStreamSynchronize(s);
-  cudaFree(vp); cudaFree(vc); cudaFree(w); cudaFree(w2); cudaFree(vraw); cudaFree(zero);
-  cudaFree(npart); cudaFree(dpart); cudaFree(scal);
+  qg_free(vp); qg_free(vc); qg_free(w); qg_free(w2); qg_free(vraw); qg_free(zero);
+  qg_free(npart); qg_free(dpart); qg_free(scal);
   if (st == QG_OK) {
     for (int k = 0; k < nchain; k++) a_host[k * (ntri + 1)] = 0.0;
     st = qg_check_device_error(ctx, "qg_lanczos_tridiag");
@@ -1026,7 +1026,7 @@ extern "C" qg_status qg_lanczos_tridiag(qg_context ctx, qg_operator op, qg_basis
   if (ctx->split_chains && !krylov_dev && nvec <= 4096 && qg_operator_values_real(op) && qg_apply_uses_lists(op, b)) {
     unsigned int *d_flags = nullptr;
     std::vector<unsigned int> fl(2 * (size_t)nvec, 0u);
-    cudaError_t e = cudaMalloc(&d_flags, fl.size() * sizeof(unsigned int));
+    cudaError_t e = qg_malloc(ctx, &d_flags, fl.size() * sizeof(unsigned int));
     if (e == cudaSuccess) e = cudaMemsetAsync(d_flags, 0, fl.size() * sizeof(unsigned int), s);
     if (e == cudaSuccess) {
       const unsigned g = (unsigned)std::min<int64_t>((n * nvec + 255) / 256, 4LL * ctx->num_sms);
@@ -1036,7 +1036,7 @@ extern "C" qg_status qg_lanczos_tridiag(qg_context ctx, qg_operator op, qg_basis
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(fl.data(), d_flags, fl.size() * sizeof(unsigned int), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    cudaFree(d_flags);
+    qg_free(d_flags);
     if (e != cudaSuccess) return qg_cuda_fail(ctx, e, "qg_lanczos_tridiag");
     std::vector<int> rcol, rpart, ccol;  // real chains (column, part) and complex columns
     for (int k = 0; k < nvec; k++) {
@@ -1049,7 +1049,7 @@ extern "C" qg_status qg_lanczos_tridiag(qg_context ctx, qg_operator op, qg_basis
     }
     if (nvec == 1 && rcol.size() == 1) {
       double *xr = nullptr;
-      e = cudaMalloc(&xr, (size_t)n * sizeof(double));
+      e = qg_malloc(ctx, &xr, (size_t)n * sizeof(double));
       if (e == cudaSuccess) {
         k_take_part<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, (const double2 *)v0_dev, rpart[0], xr);
         ctx->launches++;
@@ -1058,7 +1058,7 @@ extern "C" qg_status qg_lanczos_tridiag(qg_context ctx, qg_operator op, qg_basis
       qg_status st = e == cudaSuccess ? lanczos_general(ctx, op, b, xr, 1, ntri, eps, gamma, a_host, b_host, nullptr, 0, 1)
                                       : qg_cuda_fail(ctx, e, "qg_lanczos_tridiag");
       cudaStreamSynchronize(s);
-      cudaFree(xr);
+      qg_free(xr);
       return st;
     }
     if (rcol.size() >= 2) {
@@ -1080,10 +1080,10 @@ extern "C" qg_status qg_lanczos_tridiag(qg_context ctx, qg_operator op, qg_basis
       idx.insert(idx.end(), sb.begin(), sb.end());
       idx.insert(idx.end(), pb.begin(), pb.end());
       idx.insert(idx.end(), ccol.begin(), ccol.end());
-      e = cudaMalloc(&d_idx, (size_t)ni * sizeof(int));
+      e = qg_malloc(ctx, &d_idx, (size_t)ni * sizeof(int));
       if (e == cudaSuccess) e = cudaMemcpyAsync(d_idx, idx.data(), (size_t)ni * sizeof(int), cudaMemcpyHostToDevice, s);
-      if (e == cudaSuccess) e = cudaMalloc(&zp, (size_t)n * np * sizeof(double2));
-      if (e == cudaSuccess && nc) e = cudaMalloc(&zc, (size_t)n * nc * sizeof(double2));
+      if (e == cudaSuccess) e = qg_malloc(ctx, &zp, (size_t)n * np * sizeof(double2));
+      if (e == cudaSuccess && nc) e = qg_malloc(ctx, &zc, (size_t)n * nc * sizeof(double2));
       if (e == cudaSuccess) {
         k_pack_columns<<<(unsigned)((n * np + 255) / 256), 256, 0, s>>>(n, nvec, (const double2 *)v0_dev, np, d_idx,
                                                                        d_idx + np, d_idx + 2 * np, d_idx + 3 * np, zp);
@@ -1115,9 +1115,9 @@ extern "C" qg_status qg_lanczos_tridiag(qg_context ctx, qg_operator op, qg_basis
           }
       }
       cudaStreamSynchronize(s);
-      cudaFree(d_idx);
-      cudaFree(zp);
-      cudaFree(zc);
+      qg_free(d_idx);
+      qg_free(zp);
+      qg_free(zc);
       return st;
     }
   }
@@ -1166,7 +1166,7 @@ extern "C" qg_status qg_cf_spectra(qg_context ctx, int32_t nspec, int32_t ntri, 
   cudaStream_t s = ctx->stream;
   double *d = nullptr;
   size_t na = (size_t)nspec * (ntri + 1), nb = (size_t)nspec * ntri, ng = (size_t)nspec * (ne + 1);
-  QG_CUDA(ctx, cudaMalloc(&d, (na + nb + nspec) * 8 + ng * 16));
+  QG_CUDA(ctx, qg_malloc(ctx, &d, (na + nb + nspec) * 8 + ng * 16));
   double *da = d, *db = d + na, *de0 = db + nb;
   double2 *dg = (double2 *)(de0 + nspec);
   cudaError_t e = cudaMemcpyAsync(da, a_host, na * 8, cudaMemcpyHostToDevice, s);
@@ -1178,7 +1178,7 @@ extern "C" qg_status qg_cf_spectra(qg_context ctx, int32_t nspec, int32_t ntri, 
     e = cudaMemcpyAsync(g_host, dg, ng * 16, cudaMemcpyDeviceToHost, s);
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  cudaFree(d);
+  qg_free(d);
   if (e != cudaSuccess) return qg_cuda_fail(ctx, e, "qg_cf_spectra");
   return qg_check_launch(ctx, "qg_cf_spectra");
 }

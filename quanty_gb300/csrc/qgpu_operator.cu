@@ -224,8 +224,8 @@ void build_table(qg_context ctx, const std::vector<Entry> &terms, HostTable &tab
   if (gb) std::memcpy(blob.data(), g.data(), gb);
   if (tb) std::memcpy(blob.data() + gb, tt.data(), tb);
   if (!tg.empty()) std::memcpy(blob.data() + gb + tb, tg.data(), tg.size() * 4);
-  cudaError_t e = cudaMalloc(&tab.d_blob, blob.size());
-  if (e == cudaSuccess) e = cudaMemcpy(tab.d_blob, blob.data(), blob.size(), cudaMemcpyHostToDevice);
+  cudaError_t e = qg_malloc(ctx, &tab.d_blob, blob.size());
+  if (e == cudaSuccess) e = qg_upload(ctx, tab.d_blob, blob.data(), blob.size());
   tab.h_blob = std::move(blob);
   tab.d_groups = tab.d_blob;
   tab.d_terms = (unsigned char *)tab.d_blob + gb;
@@ -430,11 +430,11 @@ extern "C" qg_status qg_operator_create(qg_context ctx, int32_t nf, int32_t nter
 
 extern "C" qg_status qg_operator_destroy(qg_operator op) {
   if (!op) return QG_OK;
-  cudaFree(op->pull.d_blob);
-  cudaFree(op->pull_off.d_blob);
-  cudaFree(op->diag.d_blob);
-  cudaFree(op->pull_nl.d_blob);
-  cudaFree(op->push.d_blob);
+  qg_free_now(op->pull.d_blob);  // waits for the device: another context may still be using the operator
+  qg_free(op->pull_off.d_blob);
+  qg_free(op->diag.d_blob);
+  qg_free(op->pull_nl.d_blob);
+  qg_free(op->push.d_blob);
   delete op;
   return QG_OK;
 }

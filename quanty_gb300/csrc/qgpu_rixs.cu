@@ -185,17 +185,17 @@ static qg_status lanczos_krylov_t(qg_context ctx, qg_operator op, qg_basis b, co
   double *ab = nullptr, *npart = nullptr, *zero = nullptr;
   double2 *dpart = nullptr;
   KryScal<T> *sc = nullptr;
-  cudaError_t e = cudaMalloc(&w, n * sizeof(T));
-  if (e == cudaSuccess) e = cudaMalloc(&wo, n * sizeof(T));
-  if (e == cudaSuccess) e = cudaMalloc(&part, (size_t)gp * std::min(ntri, KRY_PART) * sizeof(T));
-  if (e == cudaSuccess) e = cudaMalloc(&c, (size_t)std::min(ntri, KRY_PART) * sizeof(T));
-  if (e == cudaSuccess) e = cudaMalloc(&ab, (2 * (size_t)ntri + 1) * sizeof(double));
-  if (e == cudaSuccess) e = cudaMalloc(&npart, (size_t)gu * sizeof(double));
-  if (e == cudaSuccess) e = cudaMalloc(&sc, sizeof(KryScal<T>));
+  cudaError_t e = qg_malloc(ctx, &w, n * sizeof(T));
+  if (e == cudaSuccess) e = qg_malloc(ctx, &wo, n * sizeof(T));
+  if (e == cudaSuccess) e = qg_malloc(ctx, &part, (size_t)gp * std::min(ntri, KRY_PART) * sizeof(T));
+  if (e == cudaSuccess) e = qg_malloc(ctx, &c, (size_t)std::min(ntri, KRY_PART) * sizeof(T));
+  if (e == cudaSuccess) e = qg_malloc(ctx, &ab, (2 * (size_t)ntri + 1) * sizeof(double));
+  if (e == cudaSuccess) e = qg_malloc(ctx, &npart, (size_t)gu * sizeof(double));
+  if (e == cudaSuccess) e = qg_malloc(ctx, &sc, sizeof(KryScal<T>));
   if (REAL) {  // real vectors of their own, handed out as complex ones at the end
-    if (e == cudaSuccess) e = cudaMalloc(&K, (size_t)n * ntri * sizeof(T));
-    if (e == cudaSuccess) e = cudaMalloc(&dpart, (size_t)Pa * 16);
-    if (e == cudaSuccess) e = cudaMalloc(&zero, sizeof(double));
+    if (e == cudaSuccess) e = qg_malloc(ctx, &K, (size_t)n * ntri * sizeof(T));
+    if (e == cudaSuccess) e = qg_malloc(ctx, &dpart, (size_t)Pa * 16);
+    if (e == cudaSuccess) e = qg_malloc(ctx, &zero, sizeof(double));
     if (e == cudaSuccess) e = cudaMemsetAsync(zero, 0, sizeof(double), s);
   } else {
     K = reinterpret_cast<T *>(Kout);
@@ -274,16 +274,16 @@ static qg_status lanczos_krylov_t(qg_context ctx, qg_operator op, qg_basis b, co
     a_host[0] = 0.0;
   }
   cudaStreamSynchronize(s);
-  cudaFree(w);
-  cudaFree(wo);
-  cudaFree(part);
-  cudaFree(c);
-  cudaFree(ab);
-  cudaFree(npart);
-  cudaFree(sc);
-  if (REAL) cudaFree(K);
-  cudaFree(dpart);
-  cudaFree(zero);
+  qg_free(w);
+  qg_free(wo);
+  qg_free(part);
+  qg_free(c);
+  qg_free(ab);
+  qg_free(npart);
+  qg_free(sc);
+  if (REAL) qg_free(K);
+  qg_free(dpart);
+  qg_free(zero);
   return st;
 }
 
@@ -401,14 +401,14 @@ extern "C" qg_status qg_resonant_spectra(qg_context ctx, qg_operator H1, qg_oper
   cudaError_t e = cudaSuccess;
   do {
     if ((st = qg_operator_psi_basis(ctx, T1, psi_basis, o->res1, &bt)) != QG_OK) break;
-    if ((e = cudaMalloc(&tpsi, std::max<int64_t>(bt->n, 1) * 16)) != cudaSuccess) break;
+    if ((e = qg_malloc(ctx, &tpsi, std::max<int64_t>(bt->n, 1) * 16)) != cudaSuccess) break;
     if ((st = qg_apply(ctx, T1, bt, psi_basis, psi_dev, tpsi, 1)) != QG_OK) break;
     int rounds = 0;
     if ((st = qg_basis_closure(ctx, H1, bt, o->res1, -1, &b1, &rounds)) != QG_OK) break;
     int64_t n1 = b1->n;
-    if ((e = cudaMalloc(&x1, std::max<int64_t>(n1, 1) * 16)) != cudaSuccess) break;
+    if ((e = qg_malloc(ctx, &x1, std::max<int64_t>(n1, 1) * 16)) != cudaSuccess) break;
     if ((st = qg_basis_map(ctx, bt, tpsi, b1, x1, 1)) != QG_OK) break;
-    if ((e = cudaMalloc(&K, (size_t)o->ntri1 * std::max<int64_t>(n1, 1) * 16)) != cudaSuccess) break;
+    if ((e = qg_malloc(ctx, &K, (size_t)o->ntri1 * std::max<int64_t>(n1, 1) * 16)) != cudaSuccess) break;
     if ((st = lanczos_krylov(ctx, H1, b1, x1, o->ntri1, o->epsilon, a1.data(), b1v.data(), (double2 *)K)) != QG_OK)
       break;
     std::vector<double> ev;
@@ -443,9 +443,9 @@ extern "C" qg_status qg_resonant_spectra(qg_context ctx, qg_operator H1, qg_oper
         C[(size_t)i * np + p] = b1v[0] * acc;
       }
     }
-    if ((e = cudaMalloc(&Cd, C.size() * 16)) != cudaSuccess) break;
+    if ((e = qg_malloc(ctx, &Cd, C.size() * 16)) != cudaSuccess) break;
     if ((e = cudaMemcpyAsync(Cd, C.data(), C.size() * 16, cudaMemcpyHostToDevice, s)) != cudaSuccess) break;
-    if ((e = cudaMalloc(&gt, (size_t)std::max<int64_t>(n1, 1) * np * 16)) != cudaSuccess) break;
+    if ((e = qg_malloc(ctx, &gt, (size_t)std::max<int64_t>(n1, 1) * np * 16)) != cudaSuccess) break;
     if ((st = qg_block_combine(ctx, (const double2 *)K, n1, nt, Cd, np, (double2 *)gt)) != QG_OK) break;
     // T2 targets of all operators, their closure under H2: the common final-state basis
     for (int j = 0; j < nt2 && st == QG_OK; j++) {
@@ -465,7 +465,7 @@ extern "C" qg_status qg_resonant_spectra(qg_context ctx, qg_operator H1, qg_oper
     if (st != QG_OK) break;
     if ((st = qg_basis_closure(ctx, H2, bt2, o->res2, -1, &b2, &rounds)) != QG_OK) break;
     int64_t n2 = b2->n;
-    if ((e = cudaMalloc(&x2, (size_t)std::max<int64_t>(n2, 1) * ncol * 16)) != cudaSuccess) break;
+    if ((e = qg_malloc(ctx, &x2, (size_t)std::max<int64_t>(n2, 1) * ncol * 16)) != cudaSuccess) break;
     for (int j = 0; j < nt2 && st == QG_OK; j++)
       st = qg_apply_strided(ctx, T2[j], b2, b1, gt, np, x2 + 2 * (size_t)j * np, ncol, np, nullptr, false);
     if (st != QG_OK) break;
@@ -504,12 +504,12 @@ extern "C" qg_status qg_resonant_spectra(qg_context ctx, qg_operator H1, qg_oper
   } while (0);
   if (e != cudaSuccess && st == QG_OK) st = qg_cuda_fail(ctx, e, "qg_resonant_spectra");
   cudaStreamSynchronize(s);
-  cudaFree(tpsi);
-  cudaFree(x1);
-  cudaFree(K);
-  cudaFree(Cd);
-  cudaFree(gt);
-  cudaFree(x2);
+  qg_free(tpsi);
+  qg_free(x1);
+  qg_free(K);
+  qg_free(Cd);
+  qg_free(gt);
+  qg_free(x2);
   qg_basis_destroy(bt);
   qg_basis_destroy(b1);
   qg_basis_destroy(bt2);

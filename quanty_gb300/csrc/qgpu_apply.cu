@@ -1990,8 +1990,29 @@ static int tuned_chunk(const OpBasisCache *c, int nvec) {
 static qg_status apply_chunked(qg_context ctx, qg_operator op, qg_basis dst, qg_basis src, const double *x, int xs,
                                double *y, int ys, int nvec, const ApplyFuse *fz, bool x_packed, int chunk);
 
-// The autotuner: the first multi-vector apply of an operator on a basis (outside stream
-// capture) times one plain apply per candidate number of vectors per pass (8, 4, 3, 2, 1) and
+// Vectors per pass over connection lists.  All passes of one width are one launch, the passes
+// in the grid's second dimension, so narrow passes fill the chip on small bases and wide ones
+// save the index work on large ones, where the two FMAs per connection and vector bound every
+// width; what is left over after the full passes takes a launch per power of two.  Measured on
+// bases of 45 to 1.7 M determinants with 2 to 200 vectors (real and complex operators), a rule
+// on the rows and the vectors is within 8 % of the best width nearly everywhere (us per apply):
+//   n 780, 8 vectors: 1 per pass 12, 8 per pass 36;     n 780, 48 vectors: 15 and 37
+//   n 127,895, 8: 4 per pass 131, 1 per pass 139, 8 per pass 139;  n 290,280, 6: 2 per pass 185, 8 207
+//   n 290,280, 48: 8 per pass 1424, 1 per pass 1779;    n 1,717,440, 16: 2713 and 4505
+// A warp per row (32 or 64 vectors per pass, no lists) was 2 to 110 times slower there.  Timing the
+// widths instead cost seven applies for every new operator and basis (10 ms of the 54 ms of a
+// RIXS call, 12 ms of the 73 ms of a dense spectrum).
+static int list_chunk(int64_t n, int nvec) {
+  const int64_t work = n * nvec;
+  if (n < 16384 || nvec <= 3) return 1;                     // launches and latency, or nothing to share
+  if (work > ((int64_t)1 << 23)) return nvec >= 5 ? 8 : nvec == 4 ? 4 : 2;
+  if (work > ((int64_t)1 << 21) && nvec >= 8) return 8;
+  if (nvec % 4 == 0) return 4;
+  return nvec % 2 == 0 && work > ((int64_t)1 << 19) ? 2 : 1;
+}
+
+// The autotuner of the hash path (no connection lists): the first multi-vector apply of an operator
+// on a basis (outside stream capture) times one plain apply per candidate number of vectors per pass (8, 4, 3, 2, 1) and
 // keeps the fastest for that vector count.  The candidates compute bitwise the same result
 // (each vector's sum runs in the same order), so the choice changes only the speed.
 static qg_status autotune(qg_context ctx, qg_operator op, qg_basis b, OpBasisCache *c, const double *x, int xs,
@@ -2043,6 +2064,11 @@ qg_status qg_apply_strided(qg_context ctx, qg_operator op, qg_basis dst, qg_basi
     OpBasisCache *c = qg_basis_cache(dst, op, &st);
     if (st != QG_OK) return st;
     chunk = tuned_chunk(c, nvec);
+    if (!chunk && ctx->autotune) {
+      QG_TRY(ensure_conn(ctx, op, dst, c));
+      if (c->conn_state == 1) c->chunk.push_back({nvec, list_chunk(dst->n, nvec)});
+      chunk = tuned_chunk(c, nvec);
+    }
     if (!chunk && ctx->autotune) {
       QG_TRY(autotune(ctx, op, dst, c, x, xs, y, ys, nvec));
       chunk = tuned_chunk(c, nvec);

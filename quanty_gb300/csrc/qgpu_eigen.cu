@@ -310,33 +310,41 @@ struct OneScal {
   double scale;  // 1 / beta, 0 for a vanished vector
   double norm2;  // the squared norm of the last update
   int dead;      // first step whose next vector vanished (the space is invariant), else a large number
-  unsigned int tickets[2];
+  unsigned int tickets[1 + ONE_SHARES];
 };
 
-// alpha = sum of the apply's partials (one block, fixed order)
-__global__ void __launch_bounds__(512) k_one_alpha(const double2 *__restrict__ part, int np, OneScal *sc) {
-  __shared__ double sh[16];
+#define ONE_ALPHA 1024  // up to so many partials of the apply every block sums for itself
+
+// alpha = sum of the apply's partials (one block of 256, fixed order)
+__device__ __forceinline__ double one_alpha(const double2 *__restrict__ part, int np) {
+  __shared__ double sh[8];
+  const int lane = threadIdx.x & 31;
   double s = 0.0;
-  for (int i = threadIdx.x; i < np; i += 512) s += part[i].x;
+  for (int i = threadIdx.x; i < np; i += 256) s += part[i].x;
   for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+  if (lane == 0) sh[threadIdx.x >> 5] = s;
   __syncthreads();
-  if (threadIdx.x < 32) {
-    s = threadIdx.x < 16 ? sh[threadIdx.x] : 0.0;
-    for (int o = 8; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (threadIdx.x == 0) sc->alpha = s;
-  }
+  s = sh[lane & 7];
+  for (int o = 4; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+
+__global__ void __launch_bounds__(256) k_one_alpha(const double2 *__restrict__ part, int np, OneScal *sc) {
+  const double s = one_alpha(part, np);
+  if (threadIdx.x == 0) sc->alpha = s;
 }
 
 // wo = w - alpha v_j, then c_i = <v_i|wo> for i <= j and column j of the projected matrix
-// (ct[i] = c_i + a_j [i == j] + b_j [i == j - 1])
+// (ct[i] = c_i + a_j [i == j] + b_j [i == j - 1]).  np: alpha from the apply's np partials here (a
+// launch less; every block sums them alike), 0: from k_one_alpha
 template <bool REAL>
 __global__ void __launch_bounds__(256)
     k_one_project(const typename OneT<REAL>::T *__restrict__ V, int64_t n, int j, const typename OneT<REAL>::T *__restrict__ w,
                   typename OneT<REAL>::T *__restrict__ wo, typename OneT<REAL>::T *__restrict__ part,
-                  typename OneT<REAL>::T *__restrict__ c, typename OneT<REAL>::T *__restrict__ ct, OneScal *sc) {
+                  typename OneT<REAL>::T *__restrict__ c, typename OneT<REAL>::T *__restrict__ ct, OneScal *sc,
+                  const double2 *__restrict__ dpart, int np) {
   typedef typename OneT<REAL>::T T;
-  const double alpha = sc->alpha, beta = sc->beta;
+  const double alpha = np ? one_alpha(dpart, np) : sc->alpha, beta = sc->beta;
   const T *vj = V + (int64_t)j * n;
   one_multidot<T>(
       V, n, j + 1,
@@ -345,7 +353,7 @@ __global__ void __launch_bounds__(256)
         if (blockIdx.y == 0) wo[r] = v;
         return v;
       },
-      part, &sc->tickets[0],
+      part, &sc->tickets[1],
       [&](int i, T t) {
         c[i] = t;
         ct[i] = one_plus_real(t, i == j ? alpha : i == j - 1 ? beta : 0.0);
@@ -372,7 +380,7 @@ __global__ void __launch_bounds__(128)
     if (k) w[r] = x;
     s += one_norm2(x);
   }
-  const double t = one_total128(s, part, sh, &s_last, &sc->tickets[1]);
+  const double t = one_total128(s, part, sh, &s_last, &sc->tickets[0]);
   if (s_last && tid == 0) {
     const double b = sqrt(t);
     sc->norm2 = t;
@@ -499,10 +507,13 @@ static qg_status groundstate_one(qg_context ctx, qg_operator op, qg_basis b, dou
       st = qg_apply_strided(ctx, op, b, b, (const double *)vj, 1, (double *)w, 1, 1, &fz);
       (*applies)++;
       if (st != QG_OK) break;
-      k_one_alpha<<<1, 512, 0, s>>>(dpart, Pa, sc);
+      if (Pa > ONE_ALPHA) {
+        k_one_alpha<<<1, 256, 0, s>>>(dpart, Pa, sc);
+        ctx->launches++;
+      }
       k_one_project<REAL><<<one_multidot_grid(ctx, n, j + 1), 256, one_multidot_smem<T>(j + 1), s>>>(
-          V, n, j, w, wo, part, c, ct + (size_t)j * K, sc);
-      ctx->launches += 2;
+          V, n, j, w, wo, part, c, ct + (size_t)j * K, sc, dpart, Pa > ONE_ALPHA ? 0 : Pa);
+      ctx->launches++;
       if (j + 1 < Kcur) {
         k_one_update<REAL><<<gu, 128, (size_t)(j + 1) * sizeof(T), s>>>(V, n, j + 1, c, wo, npart, j, sc);
         k_one_scale<REAL><<<g1, 256, 0, s>>>(n, wo, sc, V + (size_t)(j + 1) * n, sub + j);

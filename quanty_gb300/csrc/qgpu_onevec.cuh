@@ -74,12 +74,14 @@ static __global__ void k_one_out(int64_t n, const typename OneT<REAL>::T *__rest
   if (r < n) x[r] = one_complex(v[r]);
 }
 
+#define ONE_SHARES 8  // at most so many blocks share out the vectors of one row chunk
+
 // sink(i, <v_i|x>) for i < k with x_r = load(r), r < n (every r is loaded once per blockIdx.y).
 // A block of 256 threads walks chunks of 256 rows, their x in shared memory; its warps take the
 // vectors of the block's share (blockIdx.y) four at a time, so that the four lane sums fold into
-// one another (6 additions instead of 20).  The last block to arrive sums the blocks' partials
-// in order, 32 sums at a time, and calls sink from one thread per sum; true on its threads (the
-// caller synchronises before it reads what other threads' sinks wrote).  part: k * gridDim.x.
+// one another (6 additions instead of 20).  The last block of a share to arrive sums the
+// blocks' partials in order, 32 sums at a time, and calls sink from one thread per sum; true on its
+// threads (of each share's last block).  part: k * gridDim.x; ticket: one per share (ONE_SHARES).
 template <typename T, typename Load, typename Sink>
 __device__ __forceinline__ bool one_multidot(const T *__restrict__ V, int64_t n, int k, Load load, T *__restrict__ part,
                                              unsigned int *ticket, Sink sink) {
@@ -127,25 +129,25 @@ __device__ __forceinline__ bool one_multidot(const T *__restrict__ V, int64_t n,
   for (int i = tid; i < b1 - b0; i += 256) part[(int64_t)blockIdx.x * k + b0 + i] = acc[i];
   __threadfence();
   __syncthreads();
-  if (tid == 0) s_last = atomicAdd(ticket, 1u) == gridDim.x * gridDim.y - 1;
+  if (tid == 0) s_last = atomicAdd(ticket + blockIdx.y, 1u) == gridDim.x - 1;
   __syncthreads();
   if (!s_last) return false;
   __threadfence();
-  for (int i0 = 0; i0 < k; i0 += 32) {  // a lane per sum, the warps sharing the blocks (sw: their eight parts)
+  for (int i0 = b0; i0 < b1; i0 += 32) {  // a lane per sum, the warps sharing the blocks (sw: their eight parts)
     T s = one_zero(T());
-    if (i0 + lane < k) {
+    if (i0 + lane < b1) {
 #pragma unroll 8
       for (int b = wid; b < (int)gridDim.x; b += 8) s = one_sum(s, one_ldcg(part + (int64_t)b * k + i0 + lane));
     }
     sw[tid] = s;
     __syncthreads();
-    if (wid == 0 && i0 + lane < k) {
+    if (wid == 0 && i0 + lane < b1) {
       for (int g = 1; g < 8; g++) s = one_sum(s, sw[32 * g + lane]);
       sink(i0 + lane, s);
     }
     __syncthreads();
   }
-  if (tid == 0) *ticket = 0u;
+  if (tid == 0) ticket[blockIdx.y] = 0u;
   return true;
 }
 
@@ -194,11 +196,11 @@ __device__ __forceinline__ double one_total128(double s, double *__restrict__ pa
   return (sh[0] + sh[1]) + (sh[2] + sh[3]);
 }
 
-// the launch of one_multidot: where the rows are few the vectors are shared out over enough blocks for two on
+// the launch of one_multidot: where the rows are few the vectors are shared out over enough blocks for four on
 // every SM (a basis of 29,635 rows, 1305 steps over 75 vectors on average: 38.9 -> 27.6 ms)
 static inline dim3 one_multidot_grid(qg_context ctx, int64_t n, int k) {
   const int gx = (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 4LL * ctx->num_sms));
-  const int gy = std::max(1, std::min((k + 31) / 32, (2 * ctx->num_sms + gx - 1) / gx));
+  const int gy = std::max(1, std::min(std::min((k + 31) / 32, ONE_SHARES), (4 * ctx->num_sms + gx - 1) / gx));
   return dim3((unsigned)gx, (unsigned)gy);
 }
 template <typename T>

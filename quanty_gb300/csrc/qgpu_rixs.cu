@@ -39,7 +39,8 @@ struct KryScal {
   double keep;    // 0 when the orthogonality test failed
   double err;     // accumulated error of the truncation schedule
   double thr2;    // (eps / err)^2
-  unsigned int tickets[4];
+  unsigned int shares;  // of the test that are done
+  unsigned int tickets[2 + 2 * ONE_SHARES];  // single sums, then project and test by share
 };
 
 // wo = w - d v_d (d of the pass before; none for the first), then <v|wo> into d, and its real
@@ -83,7 +84,7 @@ __global__ void __launch_bounds__(256)
         if (blockIdx.y == 0) wo[r] = x;
         return x;
       },
-      part, &sc->tickets[1], [&](int i, T t) { c[i] = t; });
+      part, &sc->tickets[2], [&](int i, T t) { c[i] = t; });
 }
 
 // w -= sum_i c_i v_i (i < k); done: its norm into b and the scale
@@ -107,7 +108,7 @@ __global__ void __launch_bounds__(128)
     s += one_norm2(x);
   }
   if (!done) return;
-  s = one_total128(s, part, sh, &s_last, &sc->tickets[2]);
+  s = one_total128(s, part, sh, &s_last, &sc->tickets[1]);
   if (s_last && tid == 0) {
     const double b = sqrt(s);
     *b_out = b;
@@ -122,11 +123,11 @@ template <bool REAL>
 __global__ void __launch_bounds__(256)
     k_kry_test(const typename OneT<REAL>::T *__restrict__ V, int64_t n, int k, const typename OneT<REAL>::T *__restrict__ w,
                typename OneT<REAL>::T *__restrict__ v, typename OneT<REAL>::T *__restrict__ part,
-               KryScal<typename OneT<REAL>::T> *sc, double eps, const double *a_i, const double *b_i, int first,
+               typename OneT<REAL>::T *__restrict__ c, KryScal<typename OneT<REAL>::T> *sc, double eps, const double *a_i, const double *b_i, int first,
                int done) {
   typedef typename OneT<REAL>::T T;
   const double scale = sc->scale;
-  double t2 = 0.0;  // lanes of the first warp: their sums, in order
+  __shared__ int s_all;
   const bool last = one_multidot<T>(
       V, n, k,
       [&](int64_t r) {
@@ -135,8 +136,19 @@ __global__ void __launch_bounds__(256)
         if (blockIdx.y == 0) v[r] = x;
         return x;
       },
-      part, &sc->tickets[3], [&](int, T t) { t2 += one_abs2(t); });
-  if (!last || threadIdx.x >= 32) return;
+      part, &sc->tickets[2 + ONE_SHARES], [&](int i, T t) { c[i] = t; });
+  if (!last) return;
+  __syncthreads();
+  if (threadIdx.x == 0) {  // the last share's block adds the squares of all sums
+    __threadfence();
+    s_all = atomicAdd(&sc->shares, 1u) == gridDim.y - 1;
+    if (s_all) sc->shares = 0u;
+  }
+  __syncthreads();
+  if (!s_all || threadIdx.x >= 32) return;
+  __threadfence();
+  double t2 = 0.0;
+  for (int i = threadIdx.x; i < k; i += 32) t2 += one_abs2(one_ldcg(c + i));
   for (int o = 16; o; o >>= 1) t2 += __shfl_xor_sync(0xffffffffu, t2, o);
   if (threadIdx.x == 0) {
     if (!first) t2 += sc->overlap;
@@ -247,7 +259,7 @@ static qg_status lanczos_krylov_t(qg_context ctx, qg_operator op, qg_basis b, co
     for (int p = 0; p < nt; p++) {
       const int k0 = p * KRY_PART, kp = std::min(KRY_PART, i - k0);
       k_kry_test<REAL><<<one_multidot_grid(ctx, n, kp), 256, one_multidot_smem<T>(kp), s>>>(
-          K + (int64_t)k0 * n, n, kp, wo, Ki, part, sc, eps, ah + i, bh + i, p == 0, p == nt - 1);
+          K + (int64_t)k0 * n, n, kp, wo, Ki, part, c, sc, eps, ah + i, bh + i, p == 0, p == nt - 1);
     }
     k_kry_trunc<REAL><<<g1, 256, 0, s>>>(n, Ki, nullptr, sc);
     ctx->launches += 2 + 2 * np + nt;

@@ -1241,6 +1241,10 @@ void qg_cache_free(OpBasisCache &c) {
   qg_free(c.d_cptr);
   qg_free(c.d_conn);
   qg_free(c.d_coef);
+  qg_free(c.s_len);
+  qg_free(c.s_ptr);
+  qg_free(c.s_col);
+  qg_free(c.s_val);
   c = OpBasisCache();
 }
 
@@ -1821,7 +1825,8 @@ static bool op_values_real(qg_operator op);
 // move (certain offset or listed source) and every listed connection, in that kernel's order,
 // each with its source row and the value and form (kind) it multiplies with.  Count pass
 // (FILL false: cnt[r]) and fill pass (FILL true, rowptr given).
-template <int W, bool FILL, bool REAL>
+// SELL (with FILL and REAL): the explicit rows in slices, rowptr the slices, values double.
+template <int W, bool FILL, bool REAL, bool SELL = false>
 __global__ void k_small_csr(const Key<W> *__restrict__ rows, int64_t n, const int64_t *__restrict__ cptr,
                             const uint2 *__restrict__ conn, const double2 *__restrict__ coef,
                             const double2 *__restrict__ diag, LocalView lv, int *__restrict__ cnt,
@@ -1830,13 +1835,16 @@ __global__ void k_small_csr(const Key<W> *__restrict__ rows, int64_t n, const in
   const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (r >= n) return;
   int c = 0;
-  int64_t o = FILL ? rowptr[r] : 0;
+  int64_t o = !FILL ? 0 : SELL ? (int64_t)rowptr[r >> 5] * 32 + (r & 31) : rowptr[r];
   auto emit = [&](int64_t j, double2 v, unsigned char kd) {
     if (FILL) {
       col[o] = (int)j;
-      val[o] = v;
-      kind[o] = kd;
-      o++;
+      if (SELL)
+        reinterpret_cast<double *>(val)[o] = v.x;
+      else
+        val[o] = v;
+      if (!SELL) kind[o] = kd;
+      o += SELL ? 32 : 1;
     }
     c++;
   };
@@ -1966,6 +1974,208 @@ qg_status qg_small_csr(qg_context ctx, qg_operator op, qg_basis b, int64_t max_n
   }
   *out = s;
   return QG_OK;
+}
+
+static bool op_values_real(qg_operator op);
+
+// ------------------------------------------------------------------ one vector: explicit rows in slices
+//
+// On small bases one vector's apply is bound by latency, not by FP64 or memory: a thread walks
+// its row's entries through a chain of dependent loads (list or local entry, then the
+// amplitude) with a branch per entry.  Here the row is explicit -- source and value of every
+// entry in the list kernel's order -- in slices of 32 rows stored entry by entry, so a warp's
+// loads are contiguous, none depends on another, and eight entries are in flight.  The
+// arithmetic and its order are the list kernel's (and its dot partials'), so the result is
+// bitwise the same.  For operators whose values are real and fixed; us per apply, lists and rows:
+//   n 780: 12.3 and 10.0;  2,760: 15.5, 10.3;  29,635: 18.6, 10.7;  69,295: 20.6, 17.5;
+//   n 94,995: 22.7, 30.2;  290,280: 42.3, 56.6 (12 bytes per entry against 8 for a fifth of them)
+// and per Lanczos step of one real chain 28.7 and 20.5 at 29,635, 34.8 and 28.7 at 94,995, equal at
+// 165,000.  With complex values (20 bytes) lists were the faster at 780 and at 164,965 rows.
+template <bool FUSE, bool SPLIT, bool RV>
+__global__ void __launch_bounds__(256)
+    k_apply_sell(int64_t n_rows, const int *__restrict__ len_r, const int *__restrict__ ptr,
+                 const uint32_t *__restrict__ col, const double *__restrict__ val, const double2 *__restrict__ x, int xs,
+                 double2 *__restrict__ y, int ys, ApplyFuse fz) {
+  constexpr int U = 8;
+  const int64_t r = blockIdx.x * (int64_t)256 + threadIdx.x;
+  const bool live = r < n_rows;
+  const int len = live ? __ldg(len_r + r) : 0;
+  const int64_t base = live ? (int64_t)__ldg(ptr + (r >> 5)) * 32 + (r & 31) : 0;
+  const double *xr = reinterpret_cast<const double *>(x);
+  double2 acc = make_double2(0.0, 0.0);
+  for (int k0 = 0; k0 < len; k0 += U) {
+    uint32_t j[U];
+    double v[U];
+    double2 xv[U];
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (k0 + u < len) {
+        const int64_t o = base + (int64_t)(k0 + u) * 32;
+        j[u] = __ldg(col + o);
+        v[u] = __ldg(val + o);
+      }
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (k0 + u < len) {
+        if (RV)
+          xv[u].x = __ldg(xr + j[u]);
+        else
+          xv[u] = __ldg(x + (int64_t)j[u] * xs);
+      }
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (k0 + u < len) {
+        if (u == 0 && k0 == 0) {  // the diagonal product starts the sum
+          acc.x = v[u] * xv[u].x;
+          if (!RV) acc.y = v[u] * xv[u].y;
+        } else {
+          acc.x = fma(v[u], xv[u].x, acc.x);
+          if (!RV) acc.y = fma(v[u], xv[u].y, acc.y);
+        }
+      }
+  }
+  if (!FUSE) {
+    if (live) y[r * ys] = acc;
+    return;
+  }
+  // the list kernel's epilogue: y = H x - beta prev, the partials of <x|H x>
+  __shared__ double s_dot[2 * 256], s_red[2 * 8];
+  double dvs[2] = {0.0, 0.0};
+  if (live) {
+    if (RV) {
+      dvs[0] = __dmul_rn(xr[r], acc.x);
+      reinterpret_cast<double *>(y)[r] = fma(-fz.beta[0], reinterpret_cast<const double *>(fz.prev)[r], acc.x);
+    } else if (SPLIT) {
+      const double2 xv = x[r * xs], pv = fz.prev[r * ys];
+      dvs[0] = __dmul_rn(xv.x, acc.x);
+      dvs[1] = __dmul_rn(xv.y, acc.y);
+      y[r * ys] = make_double2(fma(-fz.beta[0], pv.x, acc.x), fma(-fz.beta[1], pv.y, acc.y));
+    } else {
+      dvs[0] = qg_redot(x[r * xs], acc);
+      y[r * ys] = qg_axpy2(acc, fz.beta[0], fz.prev[r * ys]);
+    }
+  }
+  fused_dot_partials<SPLIT ? 2 : 1, SPLIT>(dvs, threadIdx.x, s_dot, s_red, fz.dot_part, ys, 0);
+}
+
+static void launch_sell(qg_context ctx, const OpBasisCache *c, qg_basis b, const double2 *x, int xs, double2 *y, int ys,
+                        const ApplyFuse *fz) {
+  const unsigned g = (unsigned)qg_apply_grid(b);
+  const ApplyFuse f = fz ? *fz : ApplyFuse();
+  cudaStream_t s = ctx->stream;
+  if (!fz)
+    k_apply_sell<false, false, false><<<g, 256, 0, s>>>(b->n, c->s_len, c->s_ptr, c->s_col, c->s_val, x, xs, y, ys, f);
+  else if (f.real_vector)
+    k_apply_sell<true, false, true><<<g, 256, 0, s>>>(b->n, c->s_len, c->s_ptr, c->s_col, c->s_val, x, xs, y, ys, f);
+  else if (f.split)
+    k_apply_sell<true, true, false><<<g, 256, 0, s>>>(b->n, c->s_len, c->s_ptr, c->s_col, c->s_val, x, xs, y, ys, f);
+  else
+    k_apply_sell<true, false, false><<<g, 256, 0, s>>>(b->n, c->s_len, c->s_ptr, c->s_col, c->s_val, x, xs, y, ys, f);
+  ctx->launches++;
+}
+
+// entries of the longest row of every slice of 32 rows
+__global__ void k_slice_width(const int *__restrict__ len, int64_t n, int *__restrict__ width) {
+  const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  int w = r < n ? len[r] : 0;
+  for (int o = 16; o; o >>= 1) w = max(w, __shfl_xor_sync(0xffffffffu, w, o));
+  if ((threadIdx.x & 31) == 0 && r < n) width[r >> 5] = w;
+}
+
+#define QG_SELL_ROWS 80000   // most rows of a basis with explicit rows (see above)
+#define QG_SELL_APPLIES 4    // the apply that builds them when nothing was said before
+
+// Build the explicit rows of (op, b); sell_state -1 where the lists stay in use: large bases, complex
+// values, and sum operators, whose values change.
+static qg_status build_sell(qg_context ctx, qg_operator op, qg_basis b, OpBasisCache *c) {
+  c->sell_state = -1;
+  const int64_t n = b->n;
+  if (c->conn_state != 1 || n > QG_SELL_ROWS || op->ncomp || !op_values_real(op) || !c->d_diag) return QG_OK;
+  cudaStream_t s = ctx->stream;
+  const HostTable *tab;
+  LocalView lv;
+  const uint64_t *wreq;
+  same_basis_view(op, b, c, &tab, &lv, &wreq);
+  const int ns = (int)((n + 31) / 32);
+  int *width = nullptr;
+  void *tmp = nullptr;
+  size_t tb = 0;
+  cudaError_t e = qg_malloc(ctx, &c->s_len, (size_t)n * sizeof(int));
+  if (e == cudaSuccess) e = qg_malloc(ctx, &c->s_ptr, (size_t)(ns + 1) * sizeof(int));
+  if (e == cudaSuccess) e = qg_malloc(ctx, &width, (size_t)(ns + 1) * sizeof(int));
+  if (e == cudaSuccess) e = cudaMemsetAsync(width + ns, 0, sizeof(int), s);
+  if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(nullptr, tb, width, c->s_ptr, ns + 1, s);
+  if (e == cudaSuccess) e = qg_malloc_bytes(ctx, &tmp, std::max<size_t>(tb, 16));
+  int total = 0;
+  if (e == cudaSuccess) {
+    if (b->W == 1)
+      launch_small_csr<1, false>(ctx, b, c, lv, true, c->s_len, nullptr, nullptr, nullptr, nullptr);
+    else
+      launch_small_csr<2, false>(ctx, b, c, lv, true, c->s_len, nullptr, nullptr, nullptr, nullptr);
+    k_slice_width<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(c->s_len, n, width);
+    e = cub::DeviceScan::ExclusiveSum(tmp, tb, width, c->s_ptr, ns + 1, s);
+    ctx->launches += 3;
+  }
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&total, c->s_ptr + ns, sizeof(int), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  qg_free(width);
+  qg_free(tmp);
+  const size_t cells = std::max<size_t>((size_t)total * 32, 1);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &c->s_col, cells * sizeof(uint32_t));
+  if (e == cudaSuccess) e = qg_malloc(ctx, &c->s_val, cells * sizeof(double));
+  if (e == cudaSuccess) {
+    const unsigned g = (unsigned)((n + 255) / 256);
+    const double2 *diag = (const double2 *)c->d_diag;
+    if (b->W == 1)
+      k_small_csr<1, true, true, true><<<g, 256, 0, s>>>((const Key<1> *)b->d_keys, n, c->d_cptr, c->d_conn, c->d_coef,
+                                                         diag, lv, nullptr, c->s_ptr, (int *)c->s_col,
+                                                         (double2 *)c->s_val, nullptr);
+    else
+      k_small_csr<2, true, true, true><<<g, 256, 0, s>>>((const Key<2> *)b->d_keys, n, c->d_cptr, c->d_conn, c->d_coef,
+                                                         diag, lv, nullptr, c->s_ptr, (int *)c->s_col,
+                                                         (double2 *)c->s_val, nullptr);
+    ctx->launches++;
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) {
+    c->sell_state = 1;
+    return QG_OK;
+  }
+  qg_free(c->s_len);
+  qg_free(c->s_ptr);
+  qg_free(c->s_col);
+  qg_free(c->s_val);
+  c->s_len = c->s_ptr = nullptr;
+  c->s_col = nullptr;
+  c->s_val = nullptr;
+  if (e == cudaErrorMemoryAllocation) {  // no room: the lists stay in use
+    cudaGetLastError();
+    return QG_OK;
+  }
+  return qg_cuda_fail(ctx, e, "explicit rows");
+}
+
+// Whether the single-vector apply uses explicit rows; builds them once `applies` of them are due.
+static qg_status use_sell(qg_context ctx, qg_operator op, qg_basis b, OpBasisCache *c, int applies, bool *use) {
+  *use = c->sell_state == 1;
+  if (c->sell_state != 0 || (c->applies += applies) < QG_SELL_APPLIES) return QG_OK;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(ctx->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return QG_OK;  // tried again on a later apply
+  }
+  QG_TRY(build_sell(ctx, op, b, c));
+  *use = c->sell_state == 1;
+  return QG_OK;
+}
+
+qg_status qg_apply_prepare(qg_context ctx, qg_operator op, qg_basis b, int applies) {
+  if (!qg_apply_uses_lists(op, b)) return QG_OK;
+  qg_status st = QG_OK;
+  OpBasisCache *c = qg_basis_cache(b, op, &st);
+  if (st != QG_OK) return st;
+  bool use = false;
+  return use_sell(ctx, op, b, c, applies, &use);
 }
 
 // ------------------------------------------------------------------ entry points
@@ -2109,6 +2319,14 @@ static qg_status apply_chunked(qg_context ctx, qg_operator op, qg_basis dst, qg_
     if (c->wreq_exact && c->d_wreq && tab == &op->pull_nl) wreq = c->d_wreq;
     if (chunk > 0) {  // thread per row: gather through the connection lists when built
       QG_TRY(ensure_conn(ctx, op, dst, c));
+      if (c->conn_state == 1 && nvec == 1 && !ctx->y_host) {
+        bool use = false;
+        QG_TRY(use_sell(ctx, op, dst, c, 1, &use));
+        if (use) {
+          launch_sell(ctx, c, dst, x2, xs, y2, ys, fz);
+          return qg_check_launch(ctx, "qg_apply");
+        }
+      }
       if (c->conn_state == 1) {
         const ApplyFuse &f = fz ? *fz : none;
         const bool real = op_values_real(op);

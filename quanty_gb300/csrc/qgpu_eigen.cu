@@ -482,6 +482,7 @@ static qg_status groundstate_one(qg_context ctx, qg_operator op, qg_basis b, dou
     k_one_in<REAL><<<g1, 256, 0, s>>>(n, x_dev, x);
     ctx->launches++;
   }
+  if (st == QG_OK) st = qg_apply_prepare(ctx, op, b, K);
   int Kcur = std::min(K, std::max(2, 101));
   OneScal h;
   for (int restart = 0; restart <= max_restarts && st == QG_OK && !*converged; restart++) {

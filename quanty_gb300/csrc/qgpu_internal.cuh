@@ -196,6 +196,14 @@ struct OpBasisCache {
   int64_t *d_cptr = nullptr;      // [n + 1] list offsets
   uint2 *d_conn = nullptr;        // [nconn]
   double2 *d_coef = nullptr;      // [terms of the scanned table] (vre, vim)
+  // explicit rows for one vector (small bases, real values, qgpu_apply.cu): slices of 32 rows,
+  // entry k of row r at (s_ptr[r / 32] + k) * 32 + r % 32
+  int sell_state = 0;             // 0 not tried, 1 built, -1 not built
+  int applies = 0;                // single-vector applies so far, up to the one that builds them
+  int *s_len = nullptr;           // [n] entries per row
+  int *s_ptr = nullptr;           // [slices + 1]
+  uint32_t *s_col = nullptr;
+  double *s_val = nullptr;
   // autotuned vectors per pass of the apply kernel, per number of vectors (pairs nvec, chunk)
   std::vector<std::pair<int, int>> chunk;
 };
@@ -386,6 +394,9 @@ int qg_apply_grid(qg_basis dst);
 bool qg_apply_uses_lists(qg_operator op, qg_basis b);
 // every current value of the operator is real
 bool qg_operator_values_real(qg_operator op);
+// Says that `applies` single-vector applies of op on b follow: builds what pays for itself over
+// them (the explicit rows).  Nothing while the stream is captured.
+qg_status qg_apply_prepare(qg_context ctx, qg_operator op, qg_basis b, int applies);
 
 // Hermitian eigenproblems on the device (qgpu_jacobi.cu): A (k x k row-major, device,
 // overwritten) -> eigenvalues ascending (w_dev, k) and the lowest nv eigenvectors as the columns

@@ -849,6 +849,7 @@ static qg_status lanczos_general(qg_context ctx, qg_operator op, qg_basis b, con
                                            gamma, 1, split);
   ctx->launches += 2;
   st = qg_check_launch(ctx, "lanczos start norm");
+  if (st == QG_OK && nvec == 1) st = qg_apply_prepare(ctx, op, b, ntri);
   ApplyFuse fz;
   fz.prev = zero;
   fz.beta = zb;

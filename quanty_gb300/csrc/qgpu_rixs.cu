@@ -219,6 +219,7 @@ static qg_status lanczos_krylov_t(qg_context ctx, qg_operator op, qg_basis b, co
   if (e == cudaSuccess) e = cudaMemcpyAsync(sc, &init, sizeof(init), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(ab, 0, (2 * (size_t)ntri + 1) * sizeof(double), s);
   qg_status st = e == cudaSuccess ? QG_OK : qg_cuda_fail(ctx, e, "lanczos_krylov");
+  if (st == QG_OK) st = qg_apply_prepare(ctx, op, b, ntri);
   double *ah = ab, *bh = ab + ntri + 1;
   const unsigned g1 = gridn(n);
   auto apply = [&](const T *x, T *y) -> qg_status {

@@ -2190,43 +2190,41 @@ static bool op_values_real(qg_operator op) {
 
 bool qg_operator_values_real(qg_operator op) { return op_values_real(op); }
 
-static int tuned_chunk(const OpBasisCache *c, int nvec) {
-  if (c)
-    for (auto &p : c->chunk)
-      if (p.first == nvec) return p.second;
-  return 0;
+static OpBasisCache::Chunk *chunk_of(OpBasisCache *c, int nvec) {
+  for (auto &p : c->chunk)
+    if (p.nvec == nvec) return &p;
+  return nullptr;
 }
 
 static qg_status apply_chunked(qg_context ctx, qg_operator op, qg_basis dst, qg_basis src, const double *x, int xs,
                                double *y, int ys, int nvec, const ApplyFuse *fz, bool x_packed, int chunk);
 
-// Vectors per pass over connection lists.  All passes of one width are one launch, the passes
-// in the grid's second dimension, so narrow passes fill the chip on small bases and wide ones
-// save the index work on large ones, where the two FMAs per connection and vector bound every
-// width; what is left over after the full passes takes a launch per power of two.  Measured on
-// bases of 45 to 1.7 M determinants with 2 to 200 vectors (real and complex operators), a rule
-// on the rows and the vectors is within 8 % of the best width nearly everywhere (us per apply):
-//   n 780, 8 vectors: 1 per pass 12, 8 per pass 36;     n 780, 48 vectors: 15 and 37
-//   n 127,895, 8: 4 per pass 131, 1 per pass 139, 8 per pass 139;  n 290,280, 6: 2 per pass 185, 8 207
-//   n 290,280, 48: 8 per pass 1424, 1 per pass 1779;    n 1,717,440, 16: 2713 and 4505
-// A warp per row (32 or 64 vectors per pass, no lists) was 2 to 110 times slower there.  Timing the
-// widths instead cost seven applies for every new operator and basis (10 ms of the 54 ms of a
-// RIXS call, 12 ms of the 73 ms of a dense spectrum).
+// Vectors per pass over connection lists, for the first call on a basis.  All passes of one width
+// are one launch, the passes in the grid's second dimension, so narrow passes fill the chip on
+// small bases and wide ones save the index work on large ones, where the two FMAs per connection
+// and vector bound every width; what is left over after the full passes takes a launch per power
+// of two.  Over 336 timings (10,445 to 1.1 M determinants, 2 to 24 vectors, real and complex
+// operators) the rule is 1.4 % above the best width on average (us per apply; whole passes of 8
+// are taken earlier, since the fused Lanczos step reduces its products once per pass: 24 real
+// pairs on 127,895 rows take 730 us with 8 per pass and 920 with 2):
+//   n 780, 8 vectors: 1 per pass 12, 8 per pass 36;        n 29,635, 8: 1 and 2 per pass 1.0, 8 1.38 times
+//   n 290,280, 6: 2 per pass 185, 8 207, 1 181;            n 187,440, 12: 2 per pass 1.0, 8 1.39 times
+//   n 290,280, 48: 8 per pass 1424, 1 per pass 1779;       n 1,717,440, 16: 2713 and 4505
+// A warp per row (32 or 64 vectors per pass, no lists) was 2 to 110 times slower there.
 static int list_chunk(int64_t n, int nvec) {
   const int64_t work = n * nvec;
-  if (n < 16384 || nvec <= 3) return 1;                     // launches and latency, or nothing to share
-  if (work > ((int64_t)1 << 23)) return nvec >= 5 ? 8 : nvec == 4 ? 4 : 2;
-  if (work > ((int64_t)1 << 21) && nvec >= 8) return 8;
-  if (nvec % 4 == 0) return 4;
-  return nvec % 2 == 0 && work > ((int64_t)1 << 19) ? 2 : 1;
+  if (work < ((int64_t)1 << 19)) return 1;  // launches and latency
+  if (work > (nvec < 8 ? (int64_t)5931641 : nvec % 8 ? (int64_t)1 << 22 : (int64_t)1 << 21)) return 8;
+  return nvec % 2 ? 1 : 2;
 }
 
-// The autotuner of the hash path (no connection lists): the first multi-vector apply of an operator
-// on a basis (outside stream capture) times one plain apply per candidate number of vectors per pass (8, 4, 3, 2, 1) and
-// keeps the fastest for that vector count.  The candidates compute bitwise the same result
-// (each vector's sum runs in the same order), so the choice changes only the speed.
+// Times one plain apply per candidate number of vectors per pass and keeps the fastest for that
+// vector count: over lists 8, 4, 3, 2 or 1, on the second call (a basis that is used once never
+// pays for it: ten of the 54 ms of a RIXS call were timing); on the hash path also a warp per row with
+// 32 or 64, on the first.  Not while the stream is captured.  The candidates compute bitwise
+// the same result (each vector's sum runs in the same order), so the choice changes only the speed.
 static qg_status autotune(qg_context ctx, qg_operator op, qg_basis b, OpBasisCache *c, const double *x, int xs,
-                          double *y, int ys, int nvec) {
+                          double *y, int ys, int nvec, bool lists) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(ctx->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
     cudaGetLastError();
@@ -2236,17 +2234,16 @@ static qg_status autotune(qg_context ctx, qg_operator op, qg_basis b, OpBasisCac
   if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) {
     if (e0) cudaEventDestroy(e0);
     cudaGetLastError();
-    return QG_OK;  // untuned: the default chunk stays
+    return QG_OK;  // untimed: the choice in force stays
   }
   int best = 8;
   float best_ms = 0;
-  // thread per row with 8, 4, 3, 2 or 1 vectors per pass; warp per row with 32 or 64
   const int cand[7] = {8, 4, 3, 2, 1, -32, -64};
   qg_status st = QG_OK;
   for (int i = 0; i < 7 && st == QG_OK; i++) {
     int ch = cand[i];
     if (ch > nvec && ch != 8) continue;
-    if (ch < 0 && (nvec < 16 || (ch == -64 && nvec <= 32))) continue;
+    if (ch < 0 && (lists || nvec < 16 || (ch == -64 && nvec <= 32))) continue;
     if (i == 0) st = apply_chunked(ctx, op, b, b, x, xs, y, ys, nvec, nullptr, false, ch);  // warm
     cudaEventRecord(e0, ctx->stream);
     if (st == QG_OK) st = apply_chunked(ctx, op, b, b, x, xs, y, ys, nvec, nullptr, false, ch);
@@ -2262,8 +2259,14 @@ static qg_status autotune(qg_context ctx, qg_operator op, qg_basis b, OpBasisCac
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   cudaGetLastError();
-  if (st == QG_OK) c->chunk.push_back({nvec, best});
-  return st;
+  if (st != QG_OK) return st;
+  if (OpBasisCache::Chunk *p = chunk_of(c, nvec)) {
+    p->chunk = best;
+    p->settled = 1;
+  } else {
+    c->chunk.push_back({nvec, best, 1});
+  }
+  return QG_OK;
 }
 
 qg_status qg_apply_strided(qg_context ctx, qg_operator op, qg_basis dst, qg_basis src, const double *x, int xs,
@@ -2273,19 +2276,28 @@ qg_status qg_apply_strided(qg_context ctx, qg_operator op, qg_basis dst, qg_basi
     qg_status st = QG_OK;
     OpBasisCache *c = qg_basis_cache(dst, op, &st);
     if (st != QG_OK) return st;
-    chunk = tuned_chunk(c, nvec);
-    if (!chunk && ctx->autotune) {
-      QG_TRY(ensure_conn(ctx, op, dst, c));
-      if (c->conn_state == 1) c->chunk.push_back({nvec, list_chunk(dst->n, nvec)});
-      chunk = tuned_chunk(c, nvec);
+    OpBasisCache::Chunk *p = chunk_of(c, nvec);
+    if (ctx->autotune && !(p && p->settled)) {
+      if (!p) QG_TRY(ensure_conn(ctx, op, dst, c));
+      const bool lists = c->conn_state == 1;
+      if (!p && lists)
+        c->chunk.push_back({nvec, list_chunk(dst->n, nvec), 0});
+      else if (!lists || !fz)  // a step of a recursion is no second call (qg_apply_settle)
+        QG_TRY(autotune(ctx, op, dst, c, x, xs, y, ys, nvec, lists));
+      p = chunk_of(c, nvec);
     }
-    if (!chunk && ctx->autotune) {
-      QG_TRY(autotune(ctx, op, dst, c, x, xs, y, ys, nvec));
-      chunk = tuned_chunk(c, nvec);
-    }
-    if (!chunk) chunk = 8;
+    chunk = p ? p->chunk : 8;
   }
   return apply_chunked(ctx, op, dst, src, x, xs, y, ys, nvec, fz, x_packed, chunk);
+}
+
+qg_status qg_apply_settle(qg_context ctx, qg_operator op, qg_basis b, const double *x, double *y, int nvec) {
+  if (nvec < 2 || !ctx->autotune || !qg_apply_uses_lists(op, b)) return QG_OK;
+  qg_status st = QG_OK;
+  OpBasisCache *c = qg_basis_cache(b, op, &st);
+  if (st != QG_OK) return st;
+  const OpBasisCache::Chunk *p = chunk_of(c, nvec);
+  return p && !p->settled ? autotune(ctx, op, b, c, x, nvec, y, nvec, nvec, true) : QG_OK;
 }
 
 static qg_status apply_chunked(qg_context ctx, qg_operator op, qg_basis dst, qg_basis src, const double *x, int xs,
@@ -2535,12 +2547,12 @@ extern "C" qg_status qg_apply_set_chunk(qg_context ctx, qg_operator op, qg_basis
   qg_status st = QG_OK;
   OpBasisCache *c = qg_basis_cache(b, op, &st);
   if (st != QG_OK) return st;
-  for (auto &p : c->chunk)
-    if (p.first == nvec) {
-      p.second = chunk;
-      return QG_OK;
-    }
-  c->chunk.push_back({nvec, chunk});
+  if (OpBasisCache::Chunk *p = chunk_of(c, nvec)) {
+    p->chunk = chunk;
+    p->settled = 1;
+  } else {
+    c->chunk.push_back({nvec, chunk, 1});
+  }
   return QG_OK;
 }
 
@@ -2605,7 +2617,8 @@ extern "C" qg_status qg_apply_chunk(qg_context ctx, qg_operator op, qg_basis b, 
   if (!ctx || !op || !b || !chunk || nvec <= 0) return QG_ERR_ARG;
   *chunk = 0;
   for (auto &c : b->caches)
-    if (c.op_uid == op->uid) *chunk = tuned_chunk(&c, nvec);
+    if (c.op_uid == op->uid)
+      if (const OpBasisCache::Chunk *p = chunk_of(&c, nvec)) *chunk = p->chunk;
   return QG_OK;
 }
 

@@ -204,8 +204,12 @@ struct OpBasisCache {
   int *s_ptr = nullptr;           // [slices + 1]
   uint32_t *s_col = nullptr;
   double *s_val = nullptr;
-  // autotuned vectors per pass of the apply kernel, per number of vectors (pairs nvec, chunk)
-  std::vector<std::pair<int, int>> chunk;
+  // vectors per pass of the apply kernel, per number of vectors (nvec, chunk, settled: pinned or
+  // timed; otherwise from the rule, until the second call)
+  struct Chunk {
+    int nvec, chunk, settled;
+  };
+  std::vector<Chunk> chunk;
 };
 
 struct qg_basis_s {
@@ -397,6 +401,9 @@ bool qg_operator_values_real(qg_operator op);
 // Says that `applies` single-vector applies of op on b follow: builds what pays for itself over
 // them (the explicit rows).  Nothing while the stream is captured.
 qg_status qg_apply_prepare(qg_context ctx, qg_operator op, qg_basis b, int applies);
+// At the start of a recursion with nvec vectors: on a basis whose vectors per pass an earlier call took
+// from the rule, times the choices on x (y is overwritten).
+qg_status qg_apply_settle(qg_context ctx, qg_operator op, qg_basis b, const double *x, double *y, int nvec);
 
 // Hermitian eigenproblems on the device (qgpu_jacobi.cu): A (k x k row-major, device,
 // overwritten) -> eigenvalues ascending (w_dev, k) and the lowest nv eigenvectors as the columns

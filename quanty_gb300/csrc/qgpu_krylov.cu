@@ -857,6 +857,7 @@ static qg_status lanczos_general(qg_context ctx, qg_operator op, qg_basis b, con
   fz.split = split;
   fz.real_vector = rv;
   if (st == QG_OK) st = normalise((const double2 *)v0_dev);
+  if (st == QG_OK && nvec > 1) st = qg_apply_settle(ctx, op, b, (const double *)vc, (double *)w, nvec);
   if (st == QG_OK)
     st = qg_apply_strided(ctx, op, b, b, (const double *)vc, nvec, (double *)w, nvec, nvec, &fz, pack1);
   if (st == QG_OK && krylov_dev)

@@ -1230,10 +1230,111 @@ __global__ void k_block_verify(const Key<W> *keys, int64_t n, int lo, uint32_t l
   if (!qg_eq<W>(a, b)) mismatch[blk] = 1u;
 }
 
+// class of each block: its proposed representative unless the comparison failed
+__global__ void k_block_class(int nb, const uint32_t *__restrict__ rep, const uint32_t *__restrict__ mismatch,
+                              uint32_t *__restrict__ cls) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < nb) cls[k] = mismatch[k] ? k : rep[k];
+}
+
+__global__ void k_cfg_table(int nb, const uint32_t *__restrict__ bcfg, int32_t *__restrict__ table) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < nb) table[bcfg[k]] = k;
+}
+
+// Local terms of one flip: a configuration they apply to moves to cfg ^ fl.
+struct LocalFlip {
+  uint32_t fl;
+  int begin, end;  // its terms, in the operator's order
+};
+struct LocalTerm {
+  uint32_t n1, n0, sg, pad;
+  double re, im;
+};
+
+// The local moves of block k (one CUDA block each): per flip the sum of its applicable terms, in
+// their order, kept when the target configuration has a block (and the sum is not zero, unless
+// keep_zero); entries ascending in the target.  Count pass (FILL false: cnt[k]) and fill pass
+// (at eoff[k]); flags[0] is set when a move changes a window by more than the bit encoding holds.
+// Two passes of a few microseconds, where a map per block on the host took most of the 1.5 ms
+// that the first apply on a new basis cost.
+template <int W, bool FILL>
+__global__ void __launch_bounds__(128)
+    k_local_entries(const uint32_t *__restrict__ bcfg, const LocalFlip *__restrict__ flips, int nflip,
+                    const LocalTerm *__restrict__ terms, const int32_t *__restrict__ table,
+                    const uint32_t *__restrict__ bstart, const uint32_t *__restrict__ cls, int keep_zero, int lo, int nres,
+                    const uint64_t *__restrict__ rmask, uint32_t *__restrict__ cnt, const uint32_t *__restrict__ eoff,
+                    LocalEntry *__restrict__ ent, uint32_t *__restrict__ etarget, unsigned int *flags) {
+  extern __shared__ uint32_t s_kept[];  // a bit per flip
+  const uint32_t k = blockIdx.x, cc = bcfg[k];
+  const int words = (nflip + 31) / 32, tid = threadIdx.x;
+  for (int i = tid; i < words; i += 128) s_kept[i] = 0u;
+  __syncthreads();
+  auto sum = [&](int f, double &re, double &im) -> bool {
+    bool any = false;
+    re = im = 0.0;
+    for (int t = flips[f].begin; t < flips[f].end; t++) {
+      const LocalTerm T = terms[t];
+      if ((cc & T.n1) != T.n1 || (cc & T.n0)) continue;
+      const int par = __popc(cc & T.sg);
+      re += qg_flip_sign(T.re, par);
+      im += qg_flip_sign(T.im, par);
+      any = true;
+    }
+    return any;
+  };
+  for (int f = tid; f < nflip; f += 128) {
+    double re, im;
+    const bool any = sum(f, re, im);
+    if (any && table[cc ^ flips[f].fl] >= 0 && (keep_zero || re != 0.0 || im != 0.0))
+      atomicOr(&s_kept[f >> 5], 1u << (f & 31));
+  }
+  __syncthreads();
+  if (!FILL) {
+    __shared__ int s_n;
+    if (tid == 0) s_n = 0;
+    __syncthreads();
+    int n = 0;
+    for (int i = tid; i < words; i += 128) n += __popc(s_kept[i]);
+    if (n) atomicAdd(&s_n, n);
+    __syncthreads();
+    if (tid == 0) cnt[k] = (uint32_t)s_n;
+    return;
+  }
+  for (int f = tid; f < nflip; f += 128) {
+    if (!((s_kept[f >> 5] >> (f & 31)) & 1u)) continue;
+    const uint32_t tg = cc ^ flips[f].fl;
+    uint32_t rank = eoff[k];
+    for (int i = 0; i < words; i++)
+      for (uint32_t m = s_kept[i]; m; m &= m - 1) rank += (cc ^ flips[32 * i + __ffs((int)m) - 1].fl) < tg;
+    const int32_t tb = table[tg];
+    LocalEntry le;
+    le.tstart = bstart[tb];
+    le.tend = bstart[tb + 1] | (cls[k] == cls[tb] ? 0x80000000u : 0u);
+    sum(f, le.vre, le.vim);
+    le.wreq = 0;
+    if (nres && nres <= 12) {
+      for (int q = 0; q < nres; q++) {
+        const uint32_t m = (uint32_t)(lo >= 64 ? rmask[q * W + W - 1] >> (lo - 64)
+                                      : (rmask[q * W] >> lo) | (W == 2 && lo ? rmask[q * W + W - 1] << (64 - lo) : 0ull));
+        const int D = __popc(tg & ~cc & m) - __popc(cc & ~tg & m);
+        if (D < -2 || D > 2)
+          atomicOr(flags, 1u);
+        else if (D)
+          le.wreq |= 1ull << (5 * q + D + 2);
+      }
+    }
+    ent[rank] = le;
+    etarget[rank] = tg;
+  }
+}
+
 void qg_cache_free(OpBasisCache &c) {
   qg_free(c.d_diag);
   qg_free(c.d_wreq);
   qg_free(c.d_bstart);
+  qg_free(c.d_bcfg);
+  qg_free(c.d_class);
   qg_free(c.d_cfg);
   qg_free(c.d_eoff);
   qg_free(c.d_ent);
@@ -1278,19 +1379,71 @@ uint32_t to_local(const uint64_t *m, int lo, int W) {
   return (uint32_t)((m[0] >> lo) | (lo ? (m[1] << (64 - lo)) : 0ull));
 }
 
-void from_local(uint32_t c, int lo, int W, uint64_t *out) {
-  out[0] = out[1] = 0;
-  if (W == 1) {
-    out[0] = (uint64_t)c << lo;
-  } else if (lo >= 64) {
-    out[1] = (uint64_t)c << (lo - 64);
-  } else {
-    out[0] = (uint64_t)c << lo;
-    if (lo) out[1] = (uint64_t)c >> (64 - lo);
+}  // namespace
+
+// the operator's local terms on the device, grouped by flip, with its current values
+static qg_status local_terms(qg_context ctx, qg_operator op) {
+  if (op->n_lflip >= 0 && op->lterm_version == op->version) return QG_OK;
+  const int lo = op->nf - op->H, W = op->W;
+  std::map<uint32_t, std::vector<LocalTerm>> by;
+  for (auto &t : op->local_off)
+    by[to_local(t.fl, lo, W)].push_back(
+        {to_local(t.n1, lo, W), to_local(t.n0, lo, W), to_local(t.sg, lo, W), 0u, t.re, t.im});
+  std::vector<LocalFlip> flips;
+  std::vector<LocalTerm> terms;
+  for (auto &kv : by) {
+    LocalFlip f{kv.first, (int)terms.size(), 0};
+    terms.insert(terms.end(), kv.second.begin(), kv.second.end());
+    f.end = (int)terms.size();
+    flips.push_back(f);
   }
+  cudaError_t e = cudaSuccess;
+  if (op->n_lflip < 0) {
+    e = qg_malloc_bytes(op->ctx, &op->d_lflip, std::max<size_t>(flips.size(), 1) * sizeof(LocalFlip));
+    if (e == cudaSuccess) e = qg_malloc_bytes(op->ctx, &op->d_lterm, std::max<size_t>(terms.size(), 1) * sizeof(LocalTerm));
+  }
+  if (e == cudaSuccess && !flips.empty()) {
+    e = cudaMemcpyAsync(op->d_lflip, flips.data(), flips.size() * sizeof(LocalFlip), cudaMemcpyHostToDevice, ctx->stream);
+    if (e == cudaSuccess) e = qg_upload(ctx, op->d_lterm, terms.data(), terms.size() * sizeof(LocalTerm));
+  }
+  if (e != cudaSuccess) {
+    if (op->n_lflip < 0) {
+      qg_free(op->d_lflip);
+      qg_free(op->d_lterm);
+      op->d_lflip = op->d_lterm = nullptr;
+    }
+    return qg_cuda_fail(ctx, e, "local terms");
+  }
+  op->n_lflip = (int)flips.size();
+  op->lterm_version = op->version;
+  return QG_OK;
 }
 
-}  // namespace
+template <int W>
+static void launch_local_entries_w(qg_context ctx, qg_operator op, qg_basis b, const OpBasisCache &c, bool fill,
+                                   uint32_t *cnt, unsigned int *flags) {
+  const size_t smem = (size_t)std::max(1, (op->n_lflip + 31) / 32) * 4;
+  const LocalFlip *f = (const LocalFlip *)op->d_lflip;
+  const LocalTerm *t = (const LocalTerm *)op->d_lterm;
+  const int lo = b->nf - op->H, kz = op->keep_zero ? 1 : 0;
+  if (fill)
+    k_local_entries<W, true><<<c.nblocks, 128, smem, ctx->stream>>>(c.d_bcfg, f, op->n_lflip, t, c.d_cfg, c.d_bstart,
+                                                                    c.d_class, kz, lo, b->nres, b->d_rmask, cnt,
+                                                                    c.d_eoff, c.d_ent, c.d_ent_target, flags);
+  else
+    k_local_entries<W, false><<<c.nblocks, 128, smem, ctx->stream>>>(c.d_bcfg, f, op->n_lflip, t, c.d_cfg, c.d_bstart,
+                                                                     c.d_class, kz, lo, b->nres, b->d_rmask, cnt,
+                                                                     nullptr, nullptr, nullptr, flags);
+  ctx->launches++;
+}
+
+static void launch_local_entries(qg_context ctx, qg_operator op, qg_basis b, const OpBasisCache &c, bool fill,
+                                 uint32_t *cnt, unsigned int *flags) {
+  if (b->W == 1)
+    launch_local_entries_w<1>(ctx, op, b, c, fill, cnt, flags);
+  else
+    launch_local_entries_w<2>(ctx, op, b, c, fill, cnt, flags);
+}
 
 static qg_status build_local(qg_basis bs, qg_operator op, OpBasisCache &c) {
   qg_context ctx = bs->ctx;
@@ -1324,171 +1477,108 @@ static qg_status build_local(qg_basis bs, qg_operator op, OpBasisCache &c) {
     k_block_scatter<<<grid_for(n, 256), 256, 0, s>>>(cfg, flag, pos, n, bst, bcf);
     ctx->launches++;
   }
-  std::vector<uint32_t> hstart(nb + 1), hcfg(nb);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(hstart.data(), bst, (size_t)nb * 4, cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(hcfg.data(), bcf, (size_t)nb * 4, cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  hstart[nb] = (uint32_t)n;
-  if (e == cudaSuccess) e = cudaMemcpyAsync(bst + nb, &hstart[nb], 4, cudaMemcpyHostToDevice, s);
+  const uint32_t nrow = (uint32_t)n;
+  if (e == cudaSuccess) e = cudaMemcpyAsync(bst + nb, &nrow, 4, cudaMemcpyHostToDevice, s);
   // block classes (rows of blocks in one class align)
-  std::vector<uint32_t> cls(nb);
-  for (uint32_t k = 0; k < nb; k++) cls[k] = k;
-  {
-    unsigned long long *fp = nullptr;
-    uint32_t *rep = nullptr, *mis = nullptr;
-    if (e == cudaSuccess) e = qg_malloc(ctx, &fp, (size_t)nb * 16 + 16);
-    if (e == cudaSuccess) e = qg_malloc(ctx, &rep, (size_t)nb * 4 + 4);
-    if (e == cudaSuccess) e = qg_malloc(ctx, &mis, (size_t)nb * 4 + 4);
-    if (e == cudaSuccess) e = cudaMemsetAsync(mis, 0, (size_t)nb * 4 + 4, s);
-    if (e == cudaSuccess) {
-      if (W == 1)
-        k_block_fp<1><<<nb, 256, 0, s>>>((const Key<1> *)bs->d_keys, bst, lo, lmask, fp);
-      else
-        k_block_fp<2><<<nb, 256, 0, s>>>((const Key<2> *)bs->d_keys, bst, lo, lmask, fp);
-      ctx->launches++;
-    }
-    std::vector<unsigned long long> hfp((size_t)2 * nb);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(hfp.data(), fp, (size_t)nb * 16, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    std::vector<uint32_t> hrep(nb);
-    if (e == cudaSuccess) {
-      std::map<std::tuple<uint32_t, unsigned long long, unsigned long long>, uint32_t> first;
-      for (uint32_t k = 0; k < nb; k++) {
-        auto key = std::make_tuple(hstart[k + 1] - hstart[k], hfp[2 * k], hfp[2 * k + 1]);
-        auto it = first.find(key);
-        hrep[k] = it == first.end() ? (first[key] = k) : it->second;
-      }
-      e = cudaMemcpyAsync(rep, hrep.data(), (size_t)nb * 4, cudaMemcpyHostToDevice, s);
-    }
-    if (e == cudaSuccess) {
-      if (W == 1)
-        k_block_verify<1><<<grid_for(n, 256), 256, 0, s>>>((const Key<1> *)bs->d_keys, n, lo, lmask, pos, bst, rep,
-                                                           mis);
-      else
-        k_block_verify<2><<<grid_for(n, 256), 256, 0, s>>>((const Key<2> *)bs->d_keys, n, lo, lmask, pos, bst, rep,
-                                                           mis);
-      ctx->launches++;
-    }
-    std::vector<uint32_t> hmis(nb);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(hmis.data(), mis, (size_t)nb * 4, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e == cudaSuccess)
-      for (uint32_t k = 0; k < nb; k++) cls[k] = hmis[k] ? k : hrep[k];
-    qg_free(fp);
-    qg_free(rep);
-    qg_free(mis);
+  uint32_t *dcls = nullptr, *rep = nullptr, *mis = nullptr;
+  unsigned long long *fp = nullptr;
+  if (e == cudaSuccess) e = qg_malloc(ctx, &fp, (size_t)nb * 16 + 16);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &rep, (size_t)nb * 4 + 4);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &mis, (size_t)nb * 4 + 4);
+  if (e == cudaSuccess) e = qg_malloc(ctx, &dcls, (size_t)nb * 4 + 4);
+  if (e == cudaSuccess) e = cudaMemsetAsync(mis, 0, (size_t)nb * 4 + 4, s);
+  if (e == cudaSuccess) {
+    if (W == 1)
+      k_block_fp<1><<<nb, 256, 0, s>>>((const Key<1> *)bs->d_keys, bst, lo, lmask, fp);
+    else
+      k_block_fp<2><<<nb, 256, 0, s>>>((const Key<2> *)bs->d_keys, bst, lo, lmask, fp);
+    ctx->launches++;
   }
+  std::vector<unsigned long long> hfp((size_t)2 * nb);
+  std::vector<uint32_t> hstart(nb + 1), hrep(nb);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(hfp.data(), fp, (size_t)nb * 16, cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(hstart.data(), bst, (size_t)(nb + 1) * 4, cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e == cudaSuccess) {
+    std::map<std::tuple<uint32_t, unsigned long long, unsigned long long>, uint32_t> first;
+    for (uint32_t k = 0; k < nb; k++) {
+      auto key = std::make_tuple(hstart[k + 1] - hstart[k], hfp[2 * k], hfp[2 * k + 1]);
+      hrep[k] = first.emplace(key, k).first->second;
+    }
+    e = cudaMemcpyAsync(rep, hrep.data(), (size_t)nb * 4, cudaMemcpyHostToDevice, s);
+  }
+  if (e == cudaSuccess) {
+    if (W == 1)
+      k_block_verify<1><<<grid_for(n, 256), 256, 0, s>>>((const Key<1> *)bs->d_keys, n, lo, lmask, pos, bst, rep, mis);
+    else
+      k_block_verify<2><<<grid_for(n, 256), 256, 0, s>>>((const Key<2> *)bs->d_keys, n, lo, lmask, pos, bst, rep, mis);
+    k_block_class<<<grid_for(nb, 256), 256, 0, s>>>((int)nb, rep, mis, dcls);
+    ctx->launches += 2;
+  }
+  qg_free(fp);
+  qg_free(rep);
+  qg_free(mis);
   qg_free(cfg);
   qg_free(flag);
   qg_free(pos);
   qg_free(tmp);
-  qg_free(bcf);
-  if (e != cudaSuccess) {
-    qg_free(bst);
-    return qg_cuda_fail(ctx, e, "local blocks");
-  }
-  // configuration -> block
-  std::vector<int32_t> table((size_t)1 << H, -1);
-  for (uint32_t k = 0; k < nb; k++) table[hcfg[k]] = (int32_t)k;
-  // local terms in H-bit form
-  struct LT {
-    uint32_t n1, n0, fl, sg;
-    double re, im;
-  };
-  std::vector<LT> lt;
-  for (auto &t : op->local_off)
-    lt.push_back({to_local(t.n1, lo, W), to_local(t.n0, lo, W), to_local(t.fl, lo, W), to_local(t.sg, lo, W), t.re,
-                  t.im});
-  std::vector<uint32_t> eoff(nb + 1, 0);
-  std::vector<LocalEntry> ent;
-  std::vector<uint32_t> etarget;
-  bool exact = true;
-  for (uint32_t k = 0; k < nb; k++) {
-    uint32_t cc = hcfg[k];
-    std::map<uint32_t, std::pair<double, double>> acc;
-    for (auto &t : lt) {
-      if ((cc & t.n1) != t.n1 || (cc & t.n0)) continue;
-      uint32_t tg = cc ^ t.fl;
-      double sg = (__builtin_popcount(cc & t.sg) & 1) ? -1.0 : 1.0;
-      auto &v = acc[tg];
-      v.first += sg * t.re;
-      v.second += sg * t.im;
-    }
-    eoff[k] = (uint32_t)ent.size();
-    for (auto &kv : acc) {
-      int32_t tbk = table[kv.first];
-      if (tbk < 0 || (!op->keep_zero && kv.second.first == 0.0 && kv.second.second == 0.0)) continue;
-      LocalEntry le;
-      le.tstart = hstart[tbk];
-      le.tend = hstart[tbk + 1] | (cls[k] == cls[tbk] ? 0x80000000u : 0u);
-      etarget.push_back(kv.first);
-      le.vre = kv.second.first;
-      le.vim = kv.second.second;
-      le.wreq = 0;
-      if (bs->nres) {
-        uint64_t on[2], offb[2];
-        from_local(kv.first & ~cc, lo, W, on);
-        from_local(cc & ~kv.first, lo, W, offb);
-        exact &= move_bits(bs, on, offb, le.wreq);
-      }
-      ent.push_back(le);
-    }
-  }
-  eoff[nb] = (uint32_t)ent.size();
   c.nblocks = (int)nb;
-  c.nent = (int64_t)ent.size();
-  c.h_bcfg = hcfg;
-  c.h_eoff = eoff;
-  c.h_etarget = etarget;
-  c.h_ent = ent;
   c.d_bstart = bst;
-  e = qg_malloc(ctx, &c.d_cfg, table.size() * 4);
-  if (e == cudaSuccess) e = qg_upload(ctx, c.d_cfg, table.data(), table.size() * 4);
-  if (e == cudaSuccess) e = qg_malloc(ctx, &c.d_eoff, eoff.size() * 4);
-  if (e == cudaSuccess) e = qg_upload(ctx, c.d_eoff, eoff.data(), eoff.size() * 4);
-  if (e == cudaSuccess) e = qg_malloc(ctx, &c.d_ent, std::max<size_t>(ent.size(), 1) * sizeof(LocalEntry));
-  if (e == cudaSuccess && !ent.empty())
-    e = qg_upload(ctx, c.d_ent, ent.data(), ent.size() * sizeof(LocalEntry));
-  if (e == cudaSuccess) e = qg_malloc(ctx, &c.d_ent_target, std::max<size_t>(etarget.size(), 1) * 4);
-  if (e == cudaSuccess && !etarget.empty())
-    e = qg_upload(ctx, c.d_ent_target, etarget.data(), etarget.size() * 4);
+  c.d_bcfg = bcf;
+  c.d_class = dcls;
+  // configuration -> block
+  if (e == cudaSuccess) e = qg_malloc(ctx, &c.d_cfg, ((size_t)1 << H) * 4);
+  if (e == cudaSuccess) e = cudaMemsetAsync(c.d_cfg, 0xff, ((size_t)1 << H) * 4, s);
+  if (e == cudaSuccess) {
+    k_cfg_table<<<grid_for(nb, 256), 256, 0, s>>>((int)nb, bcf, c.d_cfg);
+    ctx->launches++;
+    e = cudaGetLastError();
+  }
+  if (e != cudaSuccess) return qg_cuda_fail(ctx, e, "local blocks");
+  // the moves: counted, then written
+  QG_TRY(local_terms(ctx, op));
+  uint32_t *cnt = nullptr;
+  void *scan = nullptr;
+  size_t sb = 0;
+  uint32_t head[2] = {0, 0};  // entries, flags
+  e = qg_malloc(ctx, &cnt, (size_t)(nb + 2) * 4);  // [nb] closes the scan, [nb + 1] the flags
+  if (e == cudaSuccess) e = qg_malloc(ctx, &c.d_eoff, (size_t)(nb + 1) * 4);
+  if (e == cudaSuccess) e = cudaMemsetAsync(cnt + nb, 0, 8, s);
+  if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(nullptr, sb, cnt, c.d_eoff, (int)nb + 1, s);
+  if (e == cudaSuccess) e = qg_malloc_bytes(ctx, &scan, std::max<size_t>(sb, 16));
+  if (e == cudaSuccess) {
+    launch_local_entries(ctx, op, bs, c, false, cnt, cnt + nb + 1);
+    e = cub::DeviceScan::ExclusiveSum(scan, sb, cnt, c.d_eoff, (int)nb + 1, s);
+    ctx->launches += 2;
+  }
+  if (e == cudaSuccess) e = cudaMemcpyAsync(head, c.d_eoff + nb, 4, cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  c.nent = head[0];
+  if (e == cudaSuccess) e = qg_malloc(ctx, &c.d_ent, std::max<size_t>(c.nent, 1) * sizeof(LocalEntry));
+  if (e == cudaSuccess) e = qg_malloc(ctx, &c.d_ent_target, std::max<size_t>(c.nent, 1) * 4);
+  if (e == cudaSuccess) {
+    launch_local_entries(ctx, op, bs, c, true, cnt, cnt + nb + 1);
+    if (c.wreq_exact) {
+      e = cudaMemcpyAsync(head + 1, cnt + nb + 1, 4, cudaMemcpyDeviceToHost, s);
+      if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    }
+  }
+  qg_free(cnt);
+  qg_free(scan);
   if (e != cudaSuccess) return qg_cuda_fail(ctx, e, "local entries");
-  if (!exact) c.wreq_exact = false;
-  return QG_OK;
+  if (head[1]) c.wreq_exact = false;
+  return qg_check_launch(ctx, "local entries");
 }
 
-// New values of a sum operator's local entries on the blocks of a cache (same entries, same
-// order: the entry set of a sum operator does not depend on its values).
+// new values of a sum operator: the entries again, in place (their structure does not change)
 static qg_status refresh_local(qg_basis bs, qg_operator op, OpBasisCache &c) {
   if (c.nent == 0) return QG_OK;
-  int H = op->H, lo = bs->nf - H, W = bs->W;
-  struct LT {
-    uint32_t n1, n0, fl, sg;
-    double re, im;
-  };
-  std::vector<LT> lt;
-  for (auto &t : op->local_off)
-    lt.push_back({to_local(t.n1, lo, W), to_local(t.n0, lo, W), to_local(t.fl, lo, W), to_local(t.sg, lo, W), t.re,
-                  t.im});
-  for (size_t k = 0; k + 1 < c.h_eoff.size(); k++) {
-    uint32_t cc = c.h_bcfg[k];
-    std::map<uint32_t, std::pair<double, double>> acc;
-    for (auto &t : lt) {
-      if ((cc & t.n1) != t.n1 || (cc & t.n0)) continue;
-      double sg = (__builtin_popcount(cc & t.sg) & 1) ? -1.0 : 1.0;
-      auto &v = acc[cc ^ t.fl];
-      v.first += sg * t.re;
-      v.second += sg * t.im;
-    }
-    for (uint32_t e = c.h_eoff[k]; e < c.h_eoff[k + 1]; e++) {
-      auto &v = acc[c.h_etarget[e]];
-      c.h_ent[e].vre = v.first;
-      c.h_ent[e].vim = v.second;
-    }
-  }
-  QG_CUDA(bs->ctx, cudaMemcpyAsync(c.d_ent, c.h_ent.data(), c.h_ent.size() * sizeof(LocalEntry),
-                                   cudaMemcpyHostToDevice, bs->ctx->stream));
-  return QG_OK;
+  QG_TRY(local_terms(bs->ctx, op));
+  unsigned int *flags = nullptr;
+  QG_CUDA(bs->ctx, qg_malloc(bs->ctx, &flags, sizeof(unsigned int)));
+  launch_local_entries(bs->ctx, op, bs, c, true, nullptr, flags);
+  qg_free(flags);
+  return qg_check_launch(bs->ctx, "local entries");
 }
 
 static void launch_diag(qg_context ctx, qg_operator op, qg_basis b, double *d_diag);

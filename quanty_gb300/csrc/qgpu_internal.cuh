@@ -145,6 +145,11 @@ struct qg_operator_s {
   // configuration of a basis; the rest (pull_nl, host copy nl_host in table order) is scanned
   int H = 0;
   std::vector<HostTerm> local_off;
+  // local_off on the device (qgpu_apply.cu), grouped by flip: LocalFlip[n_lflip], LocalTerm[], and
+  // the value version they hold
+  void *d_lflip = nullptr, *d_lterm = nullptr;
+  int n_lflip = -1;
+  uint64_t lterm_version = 0;
   HostTable pull_nl;
   std::vector<HostTerm> nl_host;
   // forward terms in creation order (masks and values)
@@ -171,15 +176,14 @@ struct LocalEntry {
 struct OpBasisCache {
   uint64_t op_uid = 0;
   uint64_t op_version = 0;        // the operator's value version the cached values belong to
-  // host copies for a value refresh (sum operators): configuration of each block, entries
-  std::vector<uint32_t> h_bcfg, h_eoff, h_etarget;
-  std::vector<LocalEntry> h_ent;
   double *d_diag = nullptr;       // complex per row: all diagonal terms
   uint64_t *d_wreq = nullptr;     // per term of op->pull_nl: window bits its source needs
   bool wreq_exact = false;        // every term's window change fits the bit encoding
   // local blocks (op->H > 0): rows sharing a local configuration are contiguous
   int nblocks = 0;
   uint32_t *d_bstart = nullptr;   // [nblocks + 1]
+  uint32_t *d_bcfg = nullptr;     // [nblocks] local configuration of each block
+  uint32_t *d_class = nullptr;    // [nblocks] class of each block (see build_local)
   int32_t *d_cfg = nullptr;       // [2^H] local configuration -> block, -1 if absent
   uint32_t *d_eoff = nullptr;     // [nblocks + 1]
   LocalEntry *d_ent = nullptr;

@@ -478,6 +478,8 @@ __device__ __forceinline__ bool expand_flush(const Key<W> *q, int n, int lane, S
 // closure (skip_diag) the sources are members of the set already, so the terms that leave a
 // determinant unchanged -- the densities and Coulomb direct terms, most of a Hamiltonian's
 // applicable terms -- are skipped, a whole group at a time where the group holds only those.
+// blockIdx.y shares out the groups (every gridDim.y-th), so that a round with few sources is not one
+// warp's walk through the whole table (a closure's first rounds: 53 us each on 26 orbitals).
 // A round stops early once an insert has found the list full (the host grows the set and
 // repeats the round): a thread checks the error word when it starts and stops at its first
 // new key past the limit, so the set exceeds the list capacity by at most one key per
@@ -517,7 +519,7 @@ __global__ void __launch_bounds__(256) k_expand(const Key<W> *src, int64_t r0, i
   }
   int qn = 0;
   bool halt = false;
-  for (int g = 0; g < ngroups && !halt; g++) {
+  for (int g = blockIdx.y; g < ngroups && !halt; g += gridDim.y) {
     const GroupDev<W> &G = groups[g];
     if (skip_diag && G.diag) continue;
     bool ok = live;
@@ -535,7 +537,7 @@ __global__ void __launch_bounds__(256) k_expand(const Key<W> *src, int64_t r0, i
       }
       // a term whose value is zero (a sum operator's component scaled to 0) reaches nothing,
       // as in the reference, whose operators hold no zero terms
-      has &= !(T.vre == 0.0 && T.vim == 0.0) && !(skip_diag && !moved);
+      has &= (qg_is_nonzero(T.vre) || qg_is_nonzero(T.vim)) && !(skip_diag && !moved);
       Key<W> tg;
 #pragma unroll
       for (int i = 0; i < W; i++) tg.w[i] = d.w[i] ^ T.flip[i];
@@ -713,7 +715,10 @@ static qg_status grow_t(qg_context ctx, qg_operator op, const Key<W> *seed_keys,
     unsigned int zero = 0;
     e = cudaMemcpyAsync(ctx->d_err, &zero, 4, cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) break;
-    k_expand<W><<<grid_for(f1 - f0), 256, 0, s>>>(
+    // at least eight warps for every quarter of an SM, by sharing out the groups
+    const int64_t warps = (f1 - f0 + 31) / 32;
+    const int shares = (int)std::max<int64_t>(1, std::min<int64_t>({32LL * ctx->num_sms / warps, op->push.ngroups, 64}));
+    k_expand<W><<<dim3(grid_for(f1 - f0), (unsigned)shares), 256, 0, s>>>(
         front, f0, f1, (const GroupDev<W> *)op->push.d_groups, op->push.ngroups, (const TermDev<W> *)op->push.d_terms,
         R.n, d_rmask, d_rmin, d_rmax, d_twreq, slots, (uint64_t)(2 * cap - 1), list, d_count,
         (unsigned long long)cap, ctx->d_err, include_seed ? 1 : 0);

@@ -276,6 +276,7 @@ __global__ void __launch_bounds__(256, NV == 1 ? QG_APPLY_MIN_BLOCKS : 1) k_appl
       }
     }
     // one term of the table: source = row ^ flip, looked up, accumulated with its sign
+    int64_t own = -2;  // slot of the row itself in the source basis, -1 absent, -2 not looked up
     auto term = [&](int t, bool known_applicable) {
       const TermDev<W> &T = terms[t];
       if (!known_applicable) {
@@ -296,15 +297,20 @@ __global__ void __launch_bounds__(256, NV == 1 ? QG_APPLY_MIN_BLOCKS : 1) k_appl
       if (dg && same_basis) {
         j = r;
       } else {
-        if (src.nres) {
-          if (wreq) {
-            uint64_t req = __ldg(wreq + t);
-            if ((okm & req) != req) return;
-          } else if (!in_windows<W>(s, src)) {
-            return;
+        if (dg) {  // the row itself, looked up once for all its diagonal terms
+          if (own == -2) own = qg_find_slot<W>(src.slots, src.hmask, d, err);
+          h = own;
+        } else {
+          if (src.nres) {
+            if (wreq) {
+              uint64_t req = __ldg(wreq + t);
+              if ((okm & req) != req) return;
+            } else if (!in_windows<W>(s, src)) {
+              return;
+            }
           }
+          h = qg_find_slot<W>(src.slots, src.hmask, s, err);
         }
-        h = qg_find_slot<W>(src.slots, src.hmask, s, err);
         if (h < 0) return;
         if (!(NV == 1 && packed)) j = (int64_t)__ldg(src.slot_row + h);
       }
@@ -1150,9 +1156,11 @@ __global__ void k_diag(const Key<W> *__restrict__ rows, int64_t n, const GroupDe
         par += __popcll(d.w[i] & terms[t].sgn[i]);
       }
       if (!app) continue;
-      double s = (par & 1) ? -1.0 : 1.0;
-      acc.x += s * terms[t].vre;
-      acc.y += s * terms[t].vim;
+      // the sign flipped as a bit, a zero part left out: one FP64 addition per term, not four
+      // operations (the FP64 pipe bounds this kernel)
+      acc.x += qg_flip_sign(terms[t].vre, par);
+      const double vi = terms[t].vim;
+      if (qg_is_nonzero(vi)) acc.y += qg_flip_sign(vi, par);
     }
   }
   diag[r] = acc;

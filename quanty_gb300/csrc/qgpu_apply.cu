@@ -170,12 +170,12 @@ __device__ __forceinline__ uint64_t window_bits(const Key<W> &d, const SrcView &
 // contributes fma(-0, x, acc) == acc exactly, so both forms give the same bits.
 
 // The fused Lanczos epilogue's per-block partial of a = Re <x|H x> for each of NV vectors (the
-// Lanczos diagonal is real).  The apply kernels are bound by the FP64 pipe, so the reduction
-// spends as few FP64 adds as it can: the rows' terms go to shared memory in row order (dvs of
-// the row at block position me), eight threads per vector add 32 terms each and one thread adds
-// their eight sums -- about one add per row, where a warp-shuffle tree costs five per row and
-// vector.  Every apply kernel reduces in this order, so their Lanczos chains agree bitwise.
-// Blocks of 256 threads; s_dot holds NV x 256 doubles (stride 256), s_red NV x 8.
+// Lanczos diagonal is real).  The rows' terms go to shared memory in row order (dvs of the row at
+// block position me); a warp per sum adds eight rows per lane (rows lane, lane + 32, ...) and
+// folds the lanes by a shuffle tree: 13 FP64 instructions, which hold a quarter of the SM for 64
+// cycles each, where eight threads adding 32 rows and one their sums took 40 in one warp.
+// Every apply kernel reduces in this order, so their Lanczos chains agree bitwise.
+// Blocks of 256 threads; s_dot holds NS x 256 doubles (stride 256), s_red NS.
 // NS sums per row (NV, or 2 NV with PAIR: the two parts of each vector, written as .x and .y).
 template <int NS, bool PAIR>
 __device__ __forceinline__ void fused_dot_partials(const double *dvs, int me, double *s_dot, double *s_red,
@@ -183,27 +183,27 @@ __device__ __forceinline__ void fused_dot_partials(const double *dvs, int me, do
 #pragma unroll
   for (int k = 0; k < NS; k++) s_dot[k * 256 + me] = dvs[k];
   __syncthreads();
-  if (threadIdx.x < NS * 8) {
-    const int k = threadIdx.x >> 3, seg = threadIdx.x & 7;
-    double t = 0.0;
-#pragma unroll 8
-    for (int i = 0; i < 32; i++) t += s_dot[k * 256 + seg * 32 + i];
-    s_red[k * 8 + seg] = t;
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int k0 = 0; k0 < NS; k0 += 8) {
+    const int k = k0 + (threadIdx.x >> 5);
+    if (k < NS) {
+      double t = s_dot[k * 256 + lane];
+#pragma unroll
+      for (int i = 1; i < 8; i++) t += s_dot[k * 256 + lane + 32 * i];
+      for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (lane == 0) {
+        if (PAIR)
+          s_red[k] = t;
+        else
+          part[blockIdx.x * ys + vec0 + k] = make_double2(t, 0.0);
+      }
+    }
   }
-  __syncthreads();
-  if (!PAIR && threadIdx.x < NS) {
-    double t = 0.0;
-#pragma unroll
-    for (int g = 0; g < 8; g++) t += s_red[threadIdx.x * 8 + g];
-    part[blockIdx.x * ys + vec0 + threadIdx.x] = make_double2(t, 0.0);
-  }
-  if (PAIR && threadIdx.x < NS / 2) {
-    double ta = 0.0, tb = 0.0;
-#pragma unroll
-    for (int g = 0; g < 8; g++) ta += s_red[2 * threadIdx.x * 8 + g];
-#pragma unroll
-    for (int g = 0; g < 8; g++) tb += s_red[(2 * threadIdx.x + 1) * 8 + g];
-    part[blockIdx.x * ys + vec0 + threadIdx.x] = make_double2(ta, tb);
+  if (PAIR) {
+    __syncthreads();
+    if (threadIdx.x < NS / 2)
+      part[blockIdx.x * ys + vec0 + threadIdx.x] = make_double2(s_red[2 * threadIdx.x], s_red[2 * threadIdx.x + 1]);
   }
 }
 
@@ -1106,7 +1106,7 @@ __global__ void k_pack(const Key<W> *__restrict__ keys, const uint32_t *__restri
     double sc = *scale, t2 = *thr2;
     v.x *= sc;
     v.y *= sc;
-    if (!(qg_norm2(v) > t2)) v = make_double2(0.0, 0.0);  // the reference keeps |a|^2 > eps^2
+    if (!qg_above(qg_norm2(v), t2)) v = make_double2(0.0, 0.0);  // the reference keeps |a|^2 > eps^2
   }
   if (own_out) own_out[r * xs] = v;
   Key<W> k = keys[r];

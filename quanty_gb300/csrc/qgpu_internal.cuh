@@ -470,17 +470,29 @@ __device__ __forceinline__ double2 qg_diag_mul(double2 dg, double2 xv, bool cplx
   if (cplx) return make_double2(fma(dg.x, xv.x, -(dg.y * xv.y)), fma(dg.x, xv.y, dg.y * xv.x));
   return make_double2(dg.x * xv.x, dg.x * xv.y);
 }
+// a > t for a square a (>= 0 or NaN) and a squared threshold t (>= 0 or NaN), on the integer pipe
+__device__ __forceinline__ bool qg_above(double a, double t) {
+  const long long ia = __double_as_longlong(a);
+  long long it = __double_as_longlong(t);
+  if ((it & 0x7fffffffffffffffll) > 0x7ff0000000000000ll) it = 0x7fffffffffffffffll;  // nothing is above NaN
+  return ia > it && ia <= 0x7ff0000000000000ll;
+}
 // after a Lanczos norm t = |v|^2: b = sqrt(t), scale = 1/b (0 for an empty vector), truncation
-// threshold (eps/err)^2 with the err before this step, err *= b^2/(b^2 + 4 gamma^2)
+// threshold (eps/err)^2 with the err before this step, err *= b^2/(b^2 + 4 gamma^2).  Called by a
+// whole warp with the same arguments: its first three lanes take one division each, at once.
 __device__ __forceinline__ void qg_lanczos_norm_scalars(double t, bool first, double eps, double gamma, double &b,
                                                         double &scale, double &thr2, double &err) {
+  const int lane = threadIdx.x & 31;
   b = sqrt(t);
-  scale = (b > 0.0) ? 1.0 / b : 0.0;
   const double e = first ? 1.0 : err;
-  const double th = eps / e;
-  thr2 = __dmul_rn(th, th);
   const double b2 = __dmul_rn(b, b), g4 = __dmul_rn(__dmul_rn(4.0, gamma), gamma);
-  err = first ? 1.0 : e * (b2 / (b2 + g4));
+  const double num = lane == 0 ? 1.0 : lane == 1 ? eps : b2, den = lane == 0 ? b : lane == 1 ? e : b2 + g4;
+  const double q = num / den;
+  const double inv = __shfl_sync(0xffffffffu, q, 0), th = __shfl_sync(0xffffffffu, q, 1),
+               f = __shfl_sync(0xffffffffu, q, 2);
+  scale = (b > 0.0) ? inv : 0.0;
+  thr2 = __dmul_rn(th, th);
+  err = first ? 1.0 : e * f;
 }
 
 // The same-basis apply of op on b as explicit rows (CSR) for the persistent Lanczos kernel of

@@ -404,10 +404,10 @@ __device__ double fin_sum(const double2 *__restrict__ part, int nblk, int nvec, 
   for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if (lane == 0) sh[wid] = s;
   __syncthreads();
-  double t = 0;
-  if (threadIdx.x == 0)
-    for (int w = 0; w < nw; w++) t += sh[w];
-  return t;
+  if (wid) return 0.0;
+  s = lane < nw ? sh[lane] : 0.0;
+  for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;  // every lane of the first warp
 }
 
 #define QG_FIN_THREADS 512
@@ -439,9 +439,10 @@ __global__ void __launch_bounds__(QG_FIN_THREADS) k_fin_b(const double2 *part, i
   const int k = blockIdx.x;
   const int col = *step;
   double t = split ? fin_sum(part, nblk, nvec, k >> 1, sh, k & 1) : fin_sum(part, nblk, nvec, k, sh);
+  if (threadIdx.x >= 32) return;
+  double b, sc, th2, e = first ? 1.0 : err[k];
+  qg_lanczos_norm_scalars(t, first != 0, eps, gamma, b, sc, th2, e);
   if (threadIdx.x == 0) {
-    double b, sc, th2, e = first ? 1.0 : err[k];
-    qg_lanczos_norm_scalars(t, first != 0, eps, gamma, b, sc, th2, e);
     b_now[k] = b;
     b_hist[k * stride + col] = b;
     scale[k] = sc;
@@ -450,17 +451,22 @@ __global__ void __launch_bounds__(QG_FIN_THREADS) k_fin_b(const double2 *part, i
   }
 }
 
+// i % nvec, in 32 bits where i fits (a 64-bit remainder is some fifty instructions)
+__device__ __forceinline__ int column_of(int64_t i, int nvec) {
+  return nvec == 1 ? 0 : i >> 32 ? (int)(i % nvec) : (int)((uint32_t)i % (uint32_t)nvec);
+}
+
 // v_out = truncate(v_in * scale) per vector (the reference keeps |a|^2 > (eps/err)^2)
 __global__ void k_scale_trunc(int64_t n, int nvec, const double2 *__restrict__ vin, const double *__restrict__ scale,
                               const double *__restrict__ thr2, double2 *__restrict__ vout) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= n * nvec) return;
-  int k = (int)(i % nvec);
+  const int k = column_of(i, nvec);
   double2 v = vin[i];
   double sc = scale[k];
   v.x *= sc;
   v.y *= sc;
-  if (!(qg_norm2(v) > thr2[k])) v = make_double2(0.0, 0.0);
+  if (!qg_above(qg_norm2(v), thr2[k])) v = make_double2(0.0, 0.0);
   vout[i] = v;
 }
 
@@ -470,12 +476,12 @@ __global__ void k_scale_trunc_split(int64_t n, int nvec, const double2 *__restri
                                     double2 *__restrict__ vout) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= n * nvec) return;
-  int k = (int)(i % nvec);
+  const int k = column_of(i, nvec);
   double2 v = vin[i];
   v.x *= scale[2 * k];
   v.y *= scale[2 * k + 1];
-  if (!(__dmul_rn(v.x, v.x) > thr2[2 * k])) v.x = 0.0;
-  if (!(__dmul_rn(v.y, v.y) > thr2[2 * k + 1])) v.y = 0.0;
+  if (!qg_above(__dmul_rn(v.x, v.x), thr2[2 * k])) v.x = 0.0;
+  if (!qg_above(__dmul_rn(v.y, v.y), thr2[2 * k + 1])) v.y = 0.0;
   vout[i] = v;
 }
 
@@ -526,7 +532,7 @@ __global__ void k_scale_trunc_real(int64_t n, const double *__restrict__ vin, co
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
   double v = vin[i] * scale[0];
-  if (!(__dmul_rn(v, v) > thr2[0])) v = 0.0;
+  if (!qg_above(__dmul_rn(v, v), thr2[0])) v = 0.0;
   vout[i] = v;
 }
 
@@ -561,108 +567,137 @@ __global__ void k_copy_col(const double2 *src, double2 *dst, int64_t n) {
 // with truncation, and the sum of the partials (k_fin_a / k_fin_b: for at most 32 partials, the
 // shuffle tree of warp 0) -- so a chain's coefficients are bitwise those of qg_lanczos_tridiag's
 // general path with one vector.  v0: n x nvec row-major; chain k = blockIdx.x.
-template <bool KRY>
-__global__ void __launch_bounds__(256)
-    k_lanczos_small(int n, int nvec, const int *__restrict__ rowptr, const int *__restrict__ col,
-                    const double2 *__restrict__ val, const unsigned char *__restrict__ kind,
-                    const double2 *__restrict__ v0, int ntri, double eps, double gamma, double *__restrict__ a_hist,
-                    double *__restrict__ b_hist, double2 *__restrict__ krylov) {
-  extern __shared__ double2 sm_vec[];
-  __shared__ double s_part[32], s_warp[8], s_dot[256], s_seg[8], s_scal[4];
+// A chain's steps are one after another in one block, so what counts is the FP64 instructions
+// of the longest warp (64 cycles each): sums over rows that are not there are left out (they add
+// zeros), the three divisions of a step are one instruction sequence, and with a real operator a
+// chain whose start vector has one part only (real or imaginary) keeps to that part, T = double
+// (one multiply-add per term; the other part stays zero).  Nine chains of 200 steps on 120
+// determinants: 1.71 ms as complex vectors with every sum in full, 0.81 ms here.
+template <typename T>
+struct SmallOps;
+template <>
+struct SmallOps<double2> {
+  static __device__ double norm2(double2 v) { return qg_norm2(v); }
+  static __device__ double redot(double2 x, double2 y) { return qg_redot(x, y); }
+  static __device__ double2 axpy(double2 w, double a, double2 p) { return qg_axpy2(w, a, p); }
+  static __device__ double2 scaled(double2 v, double s) { return make_double2(v.x * s, v.y * s); }
+  static __device__ double2 zero() { return make_double2(0.0, 0.0); }
+  static __device__ void term(double2 &acc, double2 v, unsigned char kd, double2 xv) {
+    if (kd < 2)
+      acc = qg_diag_mul(v, xv, kd == 1);
+    else if (kd == 3)
+      qg_cmac(acc, v.x, v.y, true, xv);
+    else
+      qg_cmac(acc, v.x, 0.0, false, xv);
+  }
+  static __device__ double2 from(double2 v, int) { return v; }
+  static __device__ double2 to(double2 v, int) { return v; }
+};
+template <>
+struct SmallOps<double> {
+  static __device__ double norm2(double v) { return __dmul_rn(v, v); }
+  static __device__ double redot(double x, double y) { return __dmul_rn(x, y); }
+  static __device__ double axpy(double w, double a, double p) { return fma(-a, p, w); }
+  static __device__ double scaled(double v, double s) { return v * s; }
+  static __device__ double zero() { return 0.0; }
+  static __device__ void term(double &acc, double2 v, unsigned char kd, double xv) {
+    acc = kd < 2 ? v.x * xv : fma(v.x, xv, acc);
+  }
+  static __device__ double from(double2 v, int part) { return part ? v.y : v.x; }
+  static __device__ double2 to(double v, int part) { return part ? make_double2(0.0, v) : make_double2(v, 0.0); }
+};
+
+template <typename T, bool KRY>
+__device__ void lanczos_small_chain(int n, int nvec, const int *__restrict__ rowptr, const int *__restrict__ col,
+                                    const double2 *__restrict__ val, const unsigned char *__restrict__ kind,
+                                    const double2 *__restrict__ v0, int part, int ntri, double eps, double gamma,
+                                    double *__restrict__ a_hist, double *__restrict__ b_hist,
+                                    double2 *__restrict__ krylov, T *V, double *s_part, double *s_warp, double *s_dot,
+                                    double *s_scal) {
+  typedef SmallOps<T> O;
   const int k = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int P = (n + 255) / 256;
-  double2 *V = sm_vec, *VP = sm_vec + n, *Wv = sm_vec + 2 * n;
-  double err = 1.0;  // thread 0
-  // the partial of 256 rows as k_dot_partial / k_lanczos_axpy_norm form it
+  T *VP = V + n, *Wv = V + 2 * n;
+  double err = 1.0;  // the first warp
+  // the partial of 256 rows as k_dot_partial / k_lanczos_axpy_norm form it: a tree per warp, the
+  // warps (those with rows) in order
   auto rows_part = [&](double sv, int vb) {
-    for (int o = 16; o; o >>= 1) sv += __shfl_xor_sync(0xffffffffu, sv, o);
-    if (lane == 0) s_warp[wid] = sv;
+    const int nw = min(8, (n - vb * 256 + 31) / 32);
+    if (wid < nw) {
+      for (int o = 16; o; o >>= 1) sv += __shfl_xor_sync(0xffffffffu, sv, o);
+      if (lane == 0) s_warp[wid] = sv;
+    }
     __syncthreads();
     if (tid == 0) {
-      double t = 0.0;
-      for (int w = 0; w < 8; w++) t += s_warp[w];
+      double t = s_warp[0];
+      for (int w = 1; w < nw; w++) t += s_warp[w];
       s_part[vb] = t;
     }
     __syncthreads();
   };
-  // the sum of the P partials as fin_sum forms it: warp 0's shuffle tree (lane 0)
+  // the sum of the P partials as fin_sum forms it, on the first warp
   auto fin = [&]() -> double {
-    double t = 0.0;
-    if (wid == 0) {
-      double s0 = 0.0;
-      if (lane < P) s0 += s_part[lane];
-      double sv = (s0 + 0.0) + (0.0 + 0.0);
-      for (int o = 16; o; o >>= 1) sv += __shfl_xor_sync(0xffffffffu, sv, o);
-      t = 0.0 + sv;
-    }
-    return t;  // thread 0
+    if (P == 1) return s_part[0];
+    double sv = lane < P ? s_part[lane] : 0.0;
+    for (int o = 16; o; o >>= 1) sv += __shfl_xor_sync(0xffffffffu, sv, o);
+    return sv;
   };
-  // the norm's scalars into s_scal[1..3] (b, scale, thr2) and the history at column col
+  // the norm's scalars into s_scal[1..3] (b, scale, thr2) and the history at column c
   auto norm_scalars = [&](bool first, int c) {
-    const double t = fin();
-    if (tid == 0) {
+    if (wid == 0) {
       double bb, sc, th2;
-      qg_lanczos_norm_scalars(t, first, eps, gamma, bb, sc, th2, err);
-      b_hist[(int64_t)k * ntri + c] = bb;
-      s_scal[1] = bb;
-      s_scal[2] = sc;
-      s_scal[3] = th2;
+      qg_lanczos_norm_scalars(fin(), first, eps, gamma, bb, sc, th2, err);
+      if (lane == 0) {
+        b_hist[(int64_t)k * ntri + c] = bb;
+        s_scal[1] = bb;
+        s_scal[2] = sc;
+        s_scal[3] = th2;
+      }
     }
     __syncthreads();
   };
   // dst = truncate(src * scale), and the Krylov vector of step c
-  auto normalise = [&](const double2 *src, double2 *dst, int c) {
+  auto normalise = [&](const T *src, T *dst, int c) {
     const double sc = s_scal[2], th2 = s_scal[3];
     for (int r = tid; r < n; r += 256) {
-      double2 v = src[r];
-      v.x *= sc;
-      v.y *= sc;
-      if (!(qg_norm2(v) > th2)) v = make_double2(0.0, 0.0);
+      T v = O::scaled(src[r], sc);
+      if (!qg_above(O::norm2(v), th2)) v = O::zero();
       dst[r] = v;
-      if (KRY) krylov[((int64_t)c * n + r) * nvec + k] = v;
+      if (KRY) krylov[((int64_t)c * n + r) * nvec + k] = O::to(v, part);
     }
     __syncthreads();
   };
   // Wv = H V - beta prev (prev null: zero), a = Re <V|H V> into s_scal[0] and the history
-  auto apply = [&](const double2 *prev, double beta, int c) {
+  auto apply = [&](const T *prev, double beta, int c) {
     for (int vb = 0; vb < P; vb++) {
       const int r = vb * 256 + tid;
       double dv = 0.0;
       if (r < n) {
-        double2 acc = make_double2(0.0, 0.0);
+        T acc = O::zero();
         const int e1 = rowptr[r + 1];
-        for (int e = rowptr[r]; e < e1; e++) {
-          const double2 v = val[e], xv = V[col[e]];
-          const unsigned char kd = kind[e];
-          if (kd < 2)
-            acc = qg_diag_mul(v, xv, kd == 1);
-          else if (kd == 3)
-            qg_cmac(acc, v.x, v.y, true, xv);
-          else
-            qg_cmac(acc, v.x, 0.0, false, xv);
-        }
-        dv = qg_redot(V[r], acc);
-        Wv[r] = qg_axpy2(acc, beta, prev ? prev[r] : make_double2(0.0, 0.0));
+#pragma unroll 4
+        for (int e = rowptr[r]; e < e1; e++) O::term(acc, val[e], kind[e], V[col[e]]);
+        dv = O::redot(V[r], acc);
+        Wv[r] = O::axpy(acc, beta, prev ? prev[r] : O::zero());
       }
       s_dot[tid] = dv;
       __syncthreads();
-      if (tid < 8) {
-        double t = 0.0;
-        for (int q = 0; q < 32; q++) t += s_dot[tid * 32 + q];
-        s_seg[tid] = t;
+      if (wid == 0) {
+        const int nr = min(8, (n - vb * 256 + 31) / 32);
+        double t = s_dot[lane];
+        for (int i = 1; i < nr; i++) t += s_dot[lane + 32 * i];
+        for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0) s_part[vb] = t;
       }
-      __syncthreads();
-      if (tid == 0) {
-        double t = 0.0;
-        for (int g = 0; g < 8; g++) t += s_seg[g];
-        s_part[vb] = t;
-      }
-      __syncthreads();
+      if (vb + 1 < P) __syncthreads();
     }
-    const double a = fin();
-    if (tid == 0) {
-      a_hist[(int64_t)k * (ntri + 1) + c] = a;
-      s_scal[0] = a;
+    if (wid == 0) {
+      __syncwarp();
+      const double a = fin();
+      if (lane == 0) {
+        a_hist[(int64_t)k * (ntri + 1) + c] = a;
+        s_scal[0] = a;
+      }
     }
     __syncthreads();
   };
@@ -670,11 +705,11 @@ __global__ void __launch_bounds__(256)
   for (int vb = 0; vb < P; vb++) {
     const int r = vb * 256 + tid;
     double sv = 0.0;
-    if (r < n) sv += qg_norm2(v0[(int64_t)r * nvec + k]);
+    if (r < n) sv += O::norm2(O::from(v0[(int64_t)r * nvec + k], part));
     rows_part(sv, vb);
   }
   norm_scalars(true, 0);
-  for (int r = tid; r < n; r += 256) Wv[r] = v0[(int64_t)r * nvec + k];
+  for (int r = tid; r < n; r += 256) Wv[r] = O::from(v0[(int64_t)r * nvec + k], part);
   __syncthreads();
   normalise(Wv, V, 0);
   apply(nullptr, 0.0, 1);
@@ -685,19 +720,42 @@ __global__ void __launch_bounds__(256)
       const int r = vb * 256 + tid;
       double sv = 0.0;
       if (r < n) {
-        const double2 o = qg_axpy2(Wv[r], a, V[r]);
+        const T o = O::axpy(Wv[r], a, V[r]);
         Wv[r] = o;
-        sv += qg_norm2(o);
+        sv += O::norm2(o);
       }
       rows_part(sv, vb);
     }
     norm_scalars(false, i);
     normalise(Wv, VP, i);  // VP held v_(i-2): now v_i
-    double2 *t = V;
+    T *t = V;
     V = VP;
     VP = t;
     apply(VP, s_scal[1], i + 1);
   }
+}
+
+template <bool KRY>
+__global__ void __launch_bounds__(256)
+    k_lanczos_small(int n, int nvec, const int *__restrict__ rowptr, const int *__restrict__ col,
+                    const double2 *__restrict__ val, const unsigned char *__restrict__ kind,
+                    const double2 *__restrict__ v0, int ntri, double eps, double gamma, double *__restrict__ a_hist,
+                    double *__restrict__ b_hist, double2 *__restrict__ krylov, int real_op) {
+  extern __shared__ double2 sm_vec[];
+  __shared__ double s_part[32], s_warp[8], s_dot[256], s_scal[4];
+  int parts = 0;  // bit 0: a real part that is not zero, bit 1: an imaginary one
+  if (real_op)
+    for (int r = threadIdx.x; r < n; r += 256) {
+      const double2 v = v0[(int64_t)r * nvec + blockIdx.x];
+      parts |= (qg_is_nonzero(v.x) ? 1 : 0) | (qg_is_nonzero(v.y) ? 2 : 0);
+    }
+  parts = real_op ? (__syncthreads_or(parts & 1) ? 1 : 0) | (__syncthreads_or(parts & 2) ? 2 : 0) : 3;
+  if (parts == 3)
+    lanczos_small_chain<double2, KRY>(n, nvec, rowptr, col, val, kind, v0, 0, ntri, eps, gamma, a_hist, b_hist, krylov,
+                                      sm_vec, s_part, s_warp, s_dot, s_scal);
+  else
+    lanczos_small_chain<double, KRY>(n, nvec, rowptr, col, val, kind, v0, parts == 2, ntri, eps, gamma, a_hist, b_hist,
+                                     krylov, reinterpret_cast<double *>(sm_vec), s_part, s_warp, s_dot, s_scal);
 }
 
 // The persistent path for nvec chains on a small basis; *done = false when it does not apply
@@ -727,14 +785,15 @@ static qg_status lanczos_small(qg_context ctx, qg_operator op, qg_basis b, const
   qg_status st = e == cudaSuccess ? QG_OK : qg_cuda_fail(ctx, e, "qg_lanczos_tridiag");
   if (st == QG_OK) {
     const size_t smem = (size_t)3 * n * sizeof(double2);
+    const int real = qg_operator_values_real(op) ? 1 : 0;
     if (krylov_dev)
       k_lanczos_small<true><<<(unsigned)nvec, 256, smem, s>>>(n, nvec, csr.rowptr, csr.col, csr.val, csr.kind,
                                                               (const double2 *)v0_dev, ntri, eps, gamma, ah, bh,
-                                                              (double2 *)krylov_dev);
+                                                              (double2 *)krylov_dev, real);
     else
       k_lanczos_small<false><<<(unsigned)nvec, 256, smem, s>>>(n, nvec, csr.rowptr, csr.col, csr.val, csr.kind,
                                                                (const double2 *)v0_dev, ntri, eps, gamma, ah, bh,
-                                                               nullptr);
+                                                               nullptr, real);
     ctx->launches++;
     st = qg_check_launch(ctx, "small-basis Lanczos");
   }

@@ -45,7 +45,7 @@ __global__ void k_dot_partial(int64_t n, int nvec, const double2 *__restrict__ x
         s.x += a.x * b.x + a.y * b.y;
         s.y += a.x * b.y - a.y * b.x;
       } else {
-        s.x += qg_norm2(a);
+        s.x = fma(a.x, a.x, fma(a.y, a.y, s.x));
       }
     }
     for (int o = 16; o; o >>= 1) {
@@ -88,7 +88,7 @@ __global__ void k_dot_partial_flat(int64_t len, int nvec, const double2 *__restr
       s.x += a.x * b.x + a.y * b.y;
       s.y += a.x * b.y - a.y * b.x;
     } else {
-      s.x += qg_norm2(a);
+      s.x = fma(a.x, a.x, fma(a.y, a.y, s.x));
     }
   }
   sh[tid] = s;
@@ -140,8 +140,8 @@ __global__ void k_norm_partial_split(int64_t n, int nvec, const double2 *__restr
     double2 s = make_double2(0.0, 0.0);
     for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
       double2 a = x[r * nvec + k];
-      s.x += __dmul_rn(a.x, a.x);  // each product rounded alone, as in one chain
-      s.y += __dmul_rn(a.y, a.y);
+      s.x = fma(a.x, a.x, s.x);  // as in one chain, whose other part adds nothing
+      s.y = fma(a.y, a.y, s.y);
     }
     for (int o = 16; o; o >>= 1) {
       s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
@@ -167,8 +167,8 @@ __global__ void k_norm_partial_split_flat(int64_t len, int nvec, const double2 *
   double2 s = make_double2(0.0, 0.0);
   for (int64_t i = blockIdx.x * (int64_t)T + tid; i < len; i += (int64_t)gridDim.x * T) {
     double2 a = x[i];
-    s.x += __dmul_rn(a.x, a.x);
-    s.y += __dmul_rn(a.y, a.y);
+    s.x = fma(a.x, a.x, s.x);
+    s.y = fma(a.y, a.y, s.y);
   }
   sh[tid] = s;
   __syncthreads();
@@ -287,7 +287,7 @@ __global__ void k_lanczos_axpy_norm(int64_t n, int nvec, const double2 *__restri
       double2 wv = w[r * nvec + k], pv = vp[r * nvec + k];
       double2 o = qg_axpy2(wv, ak, pv);
       v[r * nvec + k] = o;
-      s += qg_norm2(o);
+      s = fma(o.x, o.x, fma(o.y, o.y, s));
     }
     for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane == 0) sh[wid].x = s;
@@ -314,7 +314,7 @@ __global__ void k_lanczos_axpy_norm_flat(int64_t len, int nvec, const double2 *_
     double2 wv = w[i], pv = vp[i];
     double2 o = qg_axpy2(wv, ak, pv);
     v[i] = o;
-    s += qg_norm2(o);
+    s = fma(o.x, o.x, fma(o.y, o.y, s));
   }
   sh[tid].x = s;
   __syncthreads();
@@ -340,8 +340,8 @@ __global__ void k_lanczos_axpy_norm_split(int64_t n, int nvec, const double2 *__
       double2 wv = w[r * nvec + k], pv = vp[r * nvec + k];
       double2 o = make_double2(fma(-aa, pv.x, wv.x), fma(-ab, pv.y, wv.y));
       v[r * nvec + k] = o;
-      sa += __dmul_rn(o.x, o.x);
-      sb += __dmul_rn(o.y, o.y);
+      sa = fma(o.x, o.x, sa);
+      sb = fma(o.y, o.y, sb);
     }
     for (int o = 16; o; o >>= 1) {
       sa += __shfl_xor_sync(0xffffffffu, sa, o);
@@ -371,8 +371,8 @@ __global__ void k_lanczos_axpy_norm_split_flat(int64_t len, int nvec, const doub
     double2 wv = w[i], pv = vp[i];
     double2 o = make_double2(fma(-aa, pv.x, wv.x), fma(-ab, pv.y, wv.y));
     v[i] = o;
-    sa += __dmul_rn(o.x, o.x);
-    sb += __dmul_rn(o.y, o.y);
+    sa = fma(o.x, o.x, sa);
+    sb = fma(o.y, o.y, sb);
   }
   sh[tid] = make_double2(sa, sb);
   __syncthreads();
@@ -388,11 +388,17 @@ __global__ void k_lanczos_axpy_norm_split_flat(int64_t len, int nvec, const doub
 // partials with four independent accumulators (so a thread's loads overlap instead of waiting
 // on one another), a shuffle tree, then the warps' sums in order.  The total on thread 0.
 // c: 0 sums the .x parts, 1 the .y parts (the second chain of a split vector)
-__device__ double fin_sum(const double2 *__restrict__ part, int nblk, int nvec, int k, double *sh, int c = 0) {
+// FIN_SPLIT or more partials per share: the sum of a chain spread over gridDim.y blocks (15,231 partials
+// in one block are 3.9 us of FP64 additions alone)
+#define FIN_SPLIT 1024
+#define FIN_SHARES 16
+static int fin_shares(int nblk) { return std::max(1, std::min(FIN_SHARES, nblk / FIN_SPLIT)); }
+
+__device__ double fin_sum(const double2 *__restrict__ part, int b0, int nblk, int nvec, int k, double *sh, int c) {
   const int T = blockDim.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const double *pd = reinterpret_cast<const double *>(part) + c;
   double s0 = 0, s1 = 0, s2 = 0, s3 = 0;
-  int b = threadIdx.x;
+  int b = b0 + threadIdx.x;
   for (; b + 3 * T < nblk; b += 4 * T) {
     s0 += pd[2 * ((int64_t)b * nvec + k)];
     s1 += pd[2 * ((int64_t)(b + T) * nvec + k)];
@@ -410,6 +416,29 @@ __device__ double fin_sum(const double2 *__restrict__ part, int nblk, int nvec, 
   return s;  // every lane of the first warp
 }
 
+// the chain's sum on the first warp of the block that returns true: of the only block, or of the
+// last of its shares to finish (their sums in tmp, added by a fixed tree)
+__device__ bool fin_chain(const double2 *__restrict__ part, int nblk, int nvec, int k, int split, double *sh,
+                          double *tmp, unsigned int *tickets, double &t) {
+  const int S = gridDim.y, len = (nblk + S - 1) / S, b0 = blockIdx.y * len, b1 = min(nblk, b0 + len);
+  t = split ? fin_sum(part, b0, b1, nvec, k >> 1, sh, k & 1) : fin_sum(part, b0, b1, nvec, k, sh, 0);
+  if (threadIdx.x >= 32) return false;
+  if (S == 1) return true;
+  const int lane = threadIdx.x;
+  int last = 0;
+  if (lane == 0) {
+    tmp[k * FIN_SHARES + blockIdx.y] = t;
+    __threadfence();
+    last = atomicAdd(tickets + k, 1u) == (unsigned)S - 1;
+    if (last) tickets[k] = 0u;
+    __threadfence();
+  }
+  if (!__shfl_sync(0xffffffffu, last, 0)) return false;
+  t = lane < S ? __ldcg(tmp + k * FIN_SHARES + lane) : 0.0;
+  for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  return true;
+}
+
 #define QG_FIN_THREADS 512
 
 // a[k] <- Re(sum of dot partials), one block per chain; also stores a into the history at
@@ -417,11 +446,13 @@ __device__ double fin_sum(const double2 *__restrict__ part, int nblk, int nvec, 
 // (k_lanczos_axpy_norm*), after every block here has read it, so a captured step can be
 // replayed.  split: chain k is part k & 1 of vector k >> 1.
 __global__ void __launch_bounds__(QG_FIN_THREADS) k_fin_a(const double2 *part, int nblk, int nvec, double *a_now,
-                                                          double *a_hist, int stride, const int *step, int split) {
+                                                          double *a_hist, int stride, const int *step, int split,
+                                                          double *tmp, unsigned int *tickets) {
   __shared__ double sh[32];
   const int k = blockIdx.x;
   const int col = *step + 1;
-  double t = split ? fin_sum(part, nblk, nvec, k >> 1, sh, k & 1) : fin_sum(part, nblk, nvec, k, sh);
+  double t;
+  if (!fin_chain(part, nblk, nvec, k, split, sh, tmp, tickets, t)) return;
   if (threadIdx.x == 0) {
     a_now[k] = t;
     a_hist[k * stride + col] = t;
@@ -434,12 +465,12 @@ __global__ void __launch_bounds__(QG_FIN_THREADS) k_fin_a(const double2 *part, i
 __global__ void __launch_bounds__(QG_FIN_THREADS) k_fin_b(const double2 *part, int nblk, int nvec, double *b_now,
                                                           double *b_hist, int stride, const int *step, double *scale,
                                                           double *thr2, double *err, double eps, double gamma,
-                                                          int first, int split) {
+                                                          int first, int split, double *tmp, unsigned int *tickets) {
   __shared__ double sh[32];
   const int k = blockIdx.x;
   const int col = *step;
-  double t = split ? fin_sum(part, nblk, nvec, k >> 1, sh, k & 1) : fin_sum(part, nblk, nvec, k, sh);
-  if (threadIdx.x >= 32) return;
+  double t;
+  if (!fin_chain(part, nblk, nvec, k, split, sh, tmp, tickets, t)) return;
   double b, sc, th2, e = first ? 1.0 : err[k];
   qg_lanczos_norm_scalars(t, first != 0, eps, gamma, b, sc, th2, e);
   if (threadIdx.x == 0) {
@@ -493,7 +524,7 @@ __global__ void k_norm_partial_real(int64_t n, const double *__restrict__ x, dou
   int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   double s = 0.0;
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x)
-    s += __dmul_rn(x[r], x[r]);
+    s = fma(x[r], x[r], s);
   for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if (lane == 0) sh[wid] = s;
   __syncthreads();
@@ -515,7 +546,7 @@ __global__ void k_lanczos_axpy_norm_real(int64_t n, const double *__restrict__ w
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
     const double o = fma(-ak, vp[r], w[r]);
     v[r] = o;
-    s += __dmul_rn(o, o);
+    s = fma(o, o, s);
   }
   for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if (lane == 0) sh[wid] = s;
@@ -849,8 +880,10 @@ static qg_status lanczos_general(qg_context ctx, qg_operator op, qg_basis b, con
   ALLOC(zero, vb);
   ALLOC(npart, (size_t)P * nvec * 16);
   ALLOC(dpart, (size_t)Papply * nvec * 16);
-  // the scalars (one per chain), then one slot for the device step counter (zeroed with them)
-  size_t nscal = 6 * (size_t)nchain + (size_t)nchain * (ntri + 1) + (size_t)nchain * ntri + 1;
+  // the scalars (one per chain), the shares of k_fin_a / k_fin_b and their tickets, then one slot
+  // for the device step counter (zeroed with them)
+  const size_t nhist = 6 * (size_t)nchain + (size_t)nchain * (ntri + 1) + (size_t)nchain * ntri;
+  size_t nscal = nhist + (size_t)nchain * FIN_SHARES + nchain + 1;
   ALLOC(scal, nscal * 8);
 #undef ALLOC
   if (e != cudaSuccess) {
@@ -862,6 +895,8 @@ static qg_status lanczos_general(qg_context ctx, qg_operator op, qg_basis b, con
   double *a_now = scal, *b_now = scal + nchain, *scale = scal + 2 * nchain, *thr2 = scal + 3 * nchain,
          *err = scal + 4 * nchain, *zb = scal + 5 * nchain;
   double *a_hist = scal + 6 * nchain, *b_hist = a_hist + (size_t)nchain * (ntri + 1);
+  double *fin_tmp = scal + nhist;
+  unsigned int *fin_tickets = reinterpret_cast<unsigned int *>(fin_tmp + (size_t)nchain * FIN_SHARES);
   int *step_ctr = reinterpret_cast<int *>(scal + nscal - 1);
   qg_status st = QG_OK;
   k_zero<<<(unsigned)((nscal + 255) / 256), 256, 0, s>>>(scal, (int64_t)nscal);
@@ -904,8 +939,9 @@ static qg_status lanczos_general(qg_context ctx, qg_operator op, qg_basis b, con
   } else {
     launch_dot_partial(P, n, nvec, (const double2 *)v0_dev, nullptr, npart, s);
   }
-  k_fin_b<<<nchain, QG_FIN_THREADS, 0, s>>>(npart, P, nvec, b_now, b_hist, ntri, step_ctr, scale, thr2, err, eps,
-                                           gamma, 1, split);
+  k_fin_b<<<dim3(nchain, fin_shares(P)), QG_FIN_THREADS, 0, s>>>(npart, P, nvec, b_now, b_hist, ntri, step_ctr,
+                                                                   scale, thr2, err, eps,
+                                           gamma, 1, split, fin_tmp, fin_tickets);
   ctx->launches += 2;
   st = qg_check_launch(ctx, "lanczos start norm");
   if (st == QG_OK && nvec == 1) st = qg_apply_prepare(ctx, op, b, ntri);
@@ -922,7 +958,8 @@ static qg_status lanczos_general(qg_context ctx, qg_operator op, qg_basis b, con
   if (st == QG_OK && krylov_dev)
     e = cudaMemcpyAsync(krylov_dev, vc, len * 16, cudaMemcpyDeviceToDevice, s);
   if (st == QG_OK) {
-    k_fin_a<<<nchain, QG_FIN_THREADS, 0, s>>>(dpart, Papply, nvec, a_now, a_hist, ntri + 1, step_ctr, split);
+    k_fin_a<<<dim3(nchain, fin_shares(Papply)), QG_FIN_THREADS, 0, s>>>(dpart, Papply, nvec, a_now, a_hist, ntri + 1,
+                                                                        step_ctr, split, fin_tmp, fin_tickets);
     ctx->launches++;
   }
   // one step: every scalar stays on the device
@@ -942,8 +979,9 @@ static qg_status lanczos_general(qg_context ctx, qg_operator op, qg_basis b, con
       k_lanczos_axpy_norm_flat<<<P, T, T * sizeof(double2), s>>>(len, nvec, w, vp, a_now, vraw, npart, step_ctr);
     else
       k_lanczos_axpy_norm<<<P, RBLK, (RBLK / 32) * sizeof(double2), s>>>(n, nvec, w, vp, a_now, vraw, npart, step_ctr);
-    k_fin_b<<<nchain, QG_FIN_THREADS, 0, s>>>(npart, P, nvec, b_now, b_hist, ntri, step_ctr, scale, thr2, err, eps,
-                                             gamma, 0, split);
+    k_fin_b<<<dim3(nchain, fin_shares(P)), QG_FIN_THREADS, 0, s>>>(npart, P, nvec, b_now, b_hist, ntri, step_ctr,
+                                                                   scale, thr2, err, eps,
+                                             gamma, 0, split, fin_tmp, fin_tickets);
     ctx->launches += 2;
     qg_status sst = normalise(vraw);
     if (sst != QG_OK) return sst;
@@ -955,7 +993,8 @@ static qg_status lanczos_general(qg_context ctx, qg_operator op, qg_basis b, con
       cudaError_t ce = cudaMemcpyAsync(krylov_dev + 2 * (size_t)i * len, vc, len * 16, cudaMemcpyDeviceToDevice, s);
       if (ce != cudaSuccess) return qg_cuda_fail(ctx, ce, "krylov copy");
     }
-    k_fin_a<<<nchain, QG_FIN_THREADS, 0, s>>>(dpart, Papply, nvec, a_now, a_hist, ntri + 1, step_ctr, split);
+    k_fin_a<<<dim3(nchain, fin_shares(Papply)), QG_FIN_THREADS, 0, s>>>(dpart, Papply, nvec, a_now, a_hist, ntri + 1,
+                                                                        step_ctr, split, fin_tmp, fin_tickets);
     ctx->launches++;
     return sst;
   };

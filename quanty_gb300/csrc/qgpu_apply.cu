@@ -779,11 +779,19 @@ __device__ __forceinline__ void acc_real_term(double2 &acc, double v, const doub
     qg_cmac(acc, v, 0.0, false, __ldg(x + idx));
 }
 
+// Resident blocks asked of the list kernel by vectors per pass.  Its gathers wait on L2, and more warps
+// hide that better than registers beyond the sums do (a few bytes of spill at most).  us per apply with
+// 6 and with 8 blocks at one vector: 47.5 M determinants 3600 and 3316, real Lanczos step on 3.9 M
+// 314 and 285 (7 blocks as 8, 5 blocks 3941 and 355).  24 vectors on 1.7 M, registers unbounded and as
+// here: 2 per pass 5085 and 4444, 4 per pass 4538 and 4023, 8 per pass 4066 and 3970; one more block
+// each: 4502, 4406, 4043.
+constexpr int list_min_blocks(int nv) { return nv == 1 ? 8 : nv == 2 ? 6 : nv <= 4 ? 5 : 3; }
+
 // ORD: y is host memory (see the store at the end).  SPLIT (with FUSE and REAL): each complex
 // vector carries two real Lanczos chains, its real and imaginary parts.  RV (with FUSE, REAL
 // and NV = 1): x, y and prev hold one real number per row.
 template <int W, int NV, bool FUSE, bool REAL, bool ORD = false, bool SPLIT = false, bool RV = false>
-__global__ void __launch_bounds__(256, NV == 1 ? QG_APPLY_MIN_BLOCKS : 1)
+__global__ void __launch_bounds__(256, list_min_blocks(NV))
     k_apply_list(const Key<W> *__restrict__ rows, int64_t n_rows, const int64_t *__restrict__ cptr,
                  const uint2 *__restrict__ conn, const double2 *__restrict__ coef, const double2 *__restrict__ diag,
                  const double2 *__restrict__ x, int xs, double2 *__restrict__ y, int ys, int vec0, ApplyFuse fz,

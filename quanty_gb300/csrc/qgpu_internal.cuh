@@ -415,6 +415,8 @@ qg_status qg_apply_settle(qg_context ctx, qg_operator op, qg_basis b, const doub
 qg_status qg_eigh_device(qg_context ctx, int k, double2 *A, double *w_dev, double2 *V_dev, int nv);
 // the same for k > 1 by Householder reduction, bisection and inverse iteration (qgpu_hermitian.cu)
 qg_status qg_eigh_tridiag(qg_context ctx, int k, double2 *A, double *w_dev, double2 *V_dev, int nv);
+// all eigenpairs of a real symmetric tridiagonal matrix (host in and out; z k x k row-major, columns)
+qg_status qg_tri_eigh(qg_context ctx, int k, const double *d_host, const double *e_host, double *w_host, double *z_host);
 qg_status qg_eigh_host_io(qg_context ctx, int k, const double *a_host, double *w_host, double *v_host, int nv);
 int qg_partial_blocks(qg_context ctx, int64_t n);
 // *real = none of the n values of v (device) has an imaginary part (qgpu_eigen.cu)

@@ -364,22 +364,6 @@ static void tridiag_extremes(int nt, const double *a, const double *b, double *l
   }
 }
 
-static qg_status tridiag_eigen(qg_context ctx, int nt, const double *a, const double *b, std::vector<double> &ev,
-                               std::vector<cd> &Z) {
-  // diag a[1..nt], off-diagonal b[1..nt-1] (TriDiagonalMatrixToEigensystem's matrix)
-  std::vector<cd> M((size_t)nt * nt, cd(0, 0));
-  for (int i = 0; i < nt; i++) {
-    M[(size_t)i * nt + i] = a[i + 1];
-    if (i + 1 < nt) {
-      M[(size_t)i * nt + i + 1] = b[i + 1];
-      M[(size_t)(i + 1) * nt + i] = b[i + 1];
-    }
-  }
-  ev.assign(nt, 0.0);
-  Z.assign((size_t)nt * nt, cd(0, 0));
-  return qg_eigh_host_io(ctx, nt, (const double *)M.data(), ev.data(), (double *)Z.data(), nt);
-}
-
 extern "C" qg_status qg_resonant_spectra(qg_context ctx, qg_operator H1, qg_operator H2, qg_operator T1,
                                          const qg_operator *T2, int32_t nt2, qg_basis psi_basis, const double *psi_dev,
                                          qg_rixs_settings *o, double *g_host) {
@@ -424,9 +408,9 @@ extern "C" qg_status qg_resonant_spectra(qg_context ctx, qg_operator H1, qg_oper
     if ((e = qg_malloc(ctx, &K, (size_t)o->ntri1 * std::max<int64_t>(n1, 1) * 16)) != cudaSuccess) break;
     if ((st = lanczos_krylov(ctx, H1, b1, x1, o->ntri1, o->epsilon, a1.data(), b1v.data(), (double2 *)K)) != QG_OK)
       break;
-    std::vector<double> ev;
-    std::vector<cd> Z;
-    if ((st = tridiag_eigen(ctx, o->ntri1, a1.data(), b1v.data(), ev, Z)) != QG_OK) break;
+    // diagonal a[1..nt], off-diagonal b[1..nt-1] (TriDiagonalMatrixToEigensystem's matrix)
+    std::vector<double> ev(o->ntri1), Z((size_t)o->ntri1 * o->ntri1);
+    if ((st = qg_tri_eigh(ctx, o->ntri1, a1.data() + 1, b1v.data() + 1, ev.data(), Z.data())) != QG_OK) break;
     int nt = o->ntri1;
     // intermediate-state energy range defaults (Core/ResonantSpectra.cpp:80-112)
     if (o->emin1 > 0.001 * DBL_MAX && o->emax1 < -0.001 * DBL_MAX) {

@@ -2100,11 +2100,12 @@ static bool op_values_real(qg_operator op);
 template <bool FUSE, bool SPLIT, bool RV>
 __global__ void __launch_bounds__(256)
     k_apply_sell(int64_t n_rows, const int *__restrict__ len_r, const int *__restrict__ ptr,
-                 const uint32_t *__restrict__ col, const double *__restrict__ val, const double2 *__restrict__ x, int xs,
-                 double2 *__restrict__ y, int ys, ApplyFuse fz) {
+                 const uint32_t *__restrict__ col, const double *__restrict__ val, const double2 *x, int xs, double2 *y,
+                 int ys, ApplyFuse fz) {
   constexpr int U = 8;
   const int64_t r = blockIdx.x * (int64_t)256 + threadIdx.x;
   const bool live = r < n_rows;
+  qg_chain_wait();
   const int len = live ? __ldg(len_r + r) : 0;
   const int64_t base = live ? (int64_t)__ldg(ptr + (r >> 5)) * 32 + (r & 31) : 0;
   const double *xr = reinterpret_cast<const double *>(x);
@@ -2124,9 +2125,9 @@ __global__ void __launch_bounds__(256)
     for (int u = 0; u < U; u++)
       if (k0 + u < len) {
         if (RV)
-          xv[u].x = __ldg(xr + j[u]);
+          xv[u].x = xr[j[u]];
         else
-          xv[u] = __ldg(x + (int64_t)j[u] * xs);
+          xv[u] = x[(int64_t)j[u] * xs];
       }
 #pragma unroll
     for (int u = 0; u < U; u++)
@@ -2167,17 +2168,16 @@ __global__ void __launch_bounds__(256)
 static void launch_sell(qg_context ctx, const OpBasisCache *c, qg_basis b, const double2 *x, int xs, double2 *y, int ys,
                         const ApplyFuse *fz) {
   const unsigned g = (unsigned)qg_apply_grid(b);
-  const ApplyFuse f = fz ? *fz : ApplyFuse();
-  cudaStream_t s = ctx->stream;
-  if (!fz)
-    k_apply_sell<false, false, false><<<g, 256, 0, s>>>(b->n, c->s_len, c->s_ptr, c->s_col, c->s_val, x, xs, y, ys, f);
-  else if (f.real_vector)
-    k_apply_sell<true, false, true><<<g, 256, 0, s>>>(b->n, c->s_len, c->s_ptr, c->s_col, c->s_val, x, xs, y, ys, f);
-  else if (f.split)
-    k_apply_sell<true, true, false><<<g, 256, 0, s>>>(b->n, c->s_len, c->s_ptr, c->s_col, c->s_val, x, xs, y, ys, f);
-  else
-    k_apply_sell<true, false, false><<<g, 256, 0, s>>>(b->n, c->s_len, c->s_ptr, c->s_col, c->s_val, x, xs, y, ys, f);
-  ctx->launches++;
+  if (!fz) {
+    k_apply_sell<false, false, false>
+        <<<g, 256, 0, ctx->stream>>>(b->n, c->s_len, c->s_ptr, c->s_col, c->s_val, x, xs, y, ys, ApplyFuse());
+    ctx->launches++;
+    return;
+  }
+  auto kernel = fz->real_vector ? k_apply_sell<true, false, true>
+                : fz->split     ? k_apply_sell<true, true, false>
+                                : k_apply_sell<true, false, false>;
+  qg_chain_launch(ctx, kernel, g, 256, 0, b->n, c->s_len, c->s_ptr, c->s_col, c->s_val, x, xs, y, ys, *fz);
 }
 
 // entries of the longest row of every slice of 32 rows

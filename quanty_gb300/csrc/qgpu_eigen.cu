@@ -299,10 +299,14 @@ qg_status qg_all_real(qg_context ctx, const double2 *v, int64_t n, bool *real) {
 //   v_(j+1) = w / b_(j+1)                                               (k_one_scale)
 // The three-term part removes what is not small, so the one full projection after it leaves
 // w orthogonal to eps, as the second of two full ones does: V is read twice per step, not four
-// times.  Bound by those two reads from L2 (FP64 above a few hundred thousand rows).
+// times.  Bound by those two reads from L2 (FP64 above a few hundred thousand rows) and by the
+// latency of four dependent kernels of 5 to 15 us, so each is launched while the one before it drains.
 // Ground state of a 29,635-determinant impurity to a variance of 1e-12, 1305 steps in 9
-// restarts: 123 ms, against 578 ms with block products of one column (complex storage, 16 bytes per
-// entry strided by the Krylov dimension), host round trips and allocations in every step.
+// restarts: 63 ms, with plain launches 75 ms, with block products of one column (complex
+// storage, 16 bytes per entry strided by the Krylov dimension), host round trips and allocations in
+// every step 578 ms.  Not faster: a block's warps sharing out the vectors of the update, over 32 or
+// 64 rows (to a variance of 1e-10 43.2 to 53 ms, a row per thread 42.5 and 50.8), and letting the next
+// kernel's blocks up before the last block of the one before has ended (52).
 // scalars of the chain, in device memory
 struct OneScal {
   double alpha;  // a_j of the current step
@@ -339,11 +343,11 @@ __global__ void __launch_bounds__(256) k_one_alpha(const double2 *__restrict__ p
 // launch less; every block sums them alike), 0: from k_one_alpha
 template <bool REAL>
 __global__ void __launch_bounds__(256)
-    k_one_project(const typename OneT<REAL>::T *__restrict__ V, int64_t n, int j, const typename OneT<REAL>::T *__restrict__ w,
-                  typename OneT<REAL>::T *__restrict__ wo, typename OneT<REAL>::T *__restrict__ part,
-                  typename OneT<REAL>::T *__restrict__ c, typename OneT<REAL>::T *__restrict__ ct, OneScal *sc,
-                  const double2 *__restrict__ dpart, int np) {
+    k_one_project(const typename OneT<REAL>::T *V, int64_t n, int j, const typename OneT<REAL>::T *w,
+                  typename OneT<REAL>::T *wo, typename OneT<REAL>::T *part, typename OneT<REAL>::T *c,
+                  typename OneT<REAL>::T *ct, OneScal *sc, const double2 *dpart, int np) {
   typedef typename OneT<REAL>::T T;
+  qg_chain_wait();
   const double alpha = np ? one_alpha(dpart, np) : sc->alpha, beta = sc->beta;
   const T *vj = V + (int64_t)j * n;
   one_multidot<T>(
@@ -364,14 +368,15 @@ __global__ void __launch_bounds__(256)
 // leaves beta = |w|, its reciprocal and, when the vector vanished, the step in `dead`.
 template <bool REAL>
 __global__ void __launch_bounds__(128)
-    k_one_update(const typename OneT<REAL>::T *__restrict__ V, int64_t n, int k, const typename OneT<REAL>::T *__restrict__ c,
-                 typename OneT<REAL>::T *__restrict__ w, double *__restrict__ part, int step, OneScal *sc) {
+    k_one_update(const typename OneT<REAL>::T *V, int64_t n, int k, const typename OneT<REAL>::T *c,
+                 typename OneT<REAL>::T *w, double *part, int step, OneScal *sc) {
   typedef typename OneT<REAL>::T T;
   extern __shared__ __align__(16) char smem_raw[];
   T *cs = reinterpret_cast<T *>(smem_raw);
   __shared__ double sh[4];
   __shared__ int s_last;
   const int tid = threadIdx.x;
+  qg_chain_wait();
   for (int i = tid; i < k; i += 128) cs[i] = c[i];
   __syncthreads();
   double s = 0.0;
@@ -391,9 +396,10 @@ __global__ void __launch_bounds__(128)
 }
 
 template <bool REAL>
-__global__ void k_one_scale(int64_t n, const typename OneT<REAL>::T *__restrict__ w, const OneScal *__restrict__ sc,
-                            typename OneT<REAL>::T *__restrict__ v, double *__restrict__ tsub) {
+__global__ void k_one_scale(int64_t n, const typename OneT<REAL>::T *w, const OneScal *sc, typename OneT<REAL>::T *v,
+                            double *tsub) {
   const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  qg_chain_wait();
   if (r == 0 && tsub) *tsub = sc->beta;
   if (r < n) v[r] = one_scaled(w[r], sc->scale);
 }
@@ -512,13 +518,11 @@ static qg_status groundstate_one(qg_context ctx, qg_operator op, qg_basis b, dou
         k_one_alpha<<<1, 256, 0, s>>>(dpart, Pa, sc);
         ctx->launches++;
       }
-      k_one_project<REAL><<<one_multidot_grid(ctx, n, j + 1), 256, one_multidot_smem<T>(j + 1), s>>>(
-          V, n, j, w, wo, part, c, ct + (size_t)j * K, sc, dpart, Pa > ONE_ALPHA ? 0 : Pa);
-      ctx->launches++;
+      qg_chain_launch(ctx, k_one_project<REAL>, one_multidot_grid(ctx, n, j + 1), 256, one_multidot_smem<T>(j + 1), V, n,
+                      j, w, wo, part, c, ct + (size_t)j * K, sc, dpart, Pa > ONE_ALPHA ? 0 : Pa);
       if (j + 1 < Kcur) {
-        k_one_update<REAL><<<gu, 128, (size_t)(j + 1) * sizeof(T), s>>>(V, n, j + 1, c, wo, npart, j, sc);
-        k_one_scale<REAL><<<g1, 256, 0, s>>>(n, wo, sc, V + (size_t)(j + 1) * n, sub + j);
-        ctx->launches += 2;
+        qg_chain_launch(ctx, k_one_update<REAL>, gu, 128, (size_t)(j + 1) * sizeof(T), V, n, j + 1, c, wo, npart, j, sc);
+        qg_chain_launch(ctx, k_one_scale<REAL>, g1, 256, 0, n, wo, sc, V + (size_t)(j + 1) * n, sub + j);
       }
     }
     if (st == QG_OK) st = qg_check_launch(ctx, "qg_block_groundstate");

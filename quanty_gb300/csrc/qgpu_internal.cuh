@@ -415,6 +415,30 @@ qg_status qg_apply_settle(qg_context ctx, qg_operator op, qg_basis b, const doub
 qg_status qg_eigh_device(qg_context ctx, int k, double2 *A, double *w_dev, double2 *V_dev, int nv);
 // the same for k > 1 by Householder reduction, bisection and inverse iteration (qgpu_hermitian.cu)
 qg_status qg_eigh_tridiag(qg_context ctx, int k, double2 *A, double *w_dev, double2 *V_dev, int nv);
+// A launch in a chain of short kernels (a programmatic dependent launch): the blocks come up while the
+// kernel before them on the stream drains, and qg_chain_wait(), the kernel's first access to memory
+// before it, holds them until that kernel has completed with its writes visible.  What kernels of the
+// chain write is read through plain pointers: read-only loads may not see a write of the kernel's lifetime.
+// Saves about 1.6 us per kernel: the ground state's chain of four on 29,635 rows 50.8 -> 42.5 ms.
+__device__ __forceinline__ void qg_chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename... P, typename... A>
+static inline cudaError_t qg_chain_launch(qg_context ctx, void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem,
+                                          A... args) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = ctx->stream;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  ctx->launches++;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // all eigenpairs of a real symmetric tridiagonal matrix (host in and out; z k x k row-major, columns)
 qg_status qg_tri_eigh(qg_context ctx, int k, const double *d_host, const double *e_host, double *w_host, double *z_host);
 qg_status qg_eigh_host_io(qg_context ctx, int k, const double *a_host, double *w_host, double *v_host, int nv);

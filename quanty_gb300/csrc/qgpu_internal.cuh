@@ -439,8 +439,10 @@ static inline cudaError_t qg_chain_launch(qg_context ctx, void (*kernel)(P...), 
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
-// all eigenpairs of a real symmetric tridiagonal matrix (host in and out; z k x k row-major, columns)
-qg_status qg_tri_eigh(qg_context ctx, int k, const double *d_host, const double *e_host, double *w_host, double *z_host);
+// all eigenvalues and the lowest nv eigenvectors of a real symmetric tridiagonal matrix (host in and out; z k x
+// nv row-major, columns)
+qg_status qg_tri_eigh(qg_context ctx, int k, const double *d_host, const double *e_host, int nv, double *w_host,
+                      double *z_host);
 qg_status qg_eigh_host_io(qg_context ctx, int k, const double *a_host, double *w_host, double *v_host, int nv);
 int qg_partial_blocks(qg_context ctx, int64_t n);
 // *real = none of the n values of v (device) has an imaginary part (qgpu_eigen.cu)

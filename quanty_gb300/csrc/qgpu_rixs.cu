@@ -410,7 +410,7 @@ extern "C" qg_status qg_resonant_spectra(qg_context ctx, qg_operator H1, qg_oper
       break;
     // diagonal a[1..nt], off-diagonal b[1..nt-1] (TriDiagonalMatrixToEigensystem's matrix)
     std::vector<double> ev(o->ntri1), Z((size_t)o->ntri1 * o->ntri1);
-    if ((st = qg_tri_eigh(ctx, o->ntri1, a1.data() + 1, b1v.data() + 1, ev.data(), Z.data())) != QG_OK) break;
+    if ((st = qg_tri_eigh(ctx, o->ntri1, a1.data() + 1, b1v.data() + 1, o->ntri1, ev.data(), Z.data())) != QG_OK) break;
     int nt = o->ntri1;
     // intermediate-state energy range defaults (Core/ResonantSpectra.cpp:80-112)
     if (o->emin1 > 0.001 * DBL_MAX && o->emax1 < -0.001 * DBL_MAX) {

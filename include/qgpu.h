@@ -296,6 +296,12 @@ qg_status qg_cf_spectra(qg_context ctx, int32_t nspec, int32_t ntri, const doubl
                         const double *b_host, const double *e0_host, double emin, double de,
                         int32_t ne, double gamma, double *g_host);
 
+/* Lowest and highest eigenvalue of every chain's tridiagonal matrix (the pole range of a spectrum,
+ * LuaInterface/ssp.cpp:2651-2663): a and b as in qg_cf_spectra; early != 0: a chain ends before its
+ * first b = 0.  lo_hi (host) receives 2 * nspec values, all chains in one kernel. */
+qg_status qg_tri_extremes(qg_context ctx, int32_t nspec, int32_t ntri, const double *a_host,
+                          const double *b_host, int32_t early, double *lo_hi_host);
+
 /* Lowest nvec eigenpairs of a Hermitian op on a fixed basis by restarted block (band)
  * Lanczos with full reorthogonalisation (BlockLanczosGroundStateConserveBasis,
  * Core/BlockLanczos.cpp:5707, its Krylov solver :5350).  x_dev holds nvec start vectors

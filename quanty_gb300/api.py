@@ -1147,20 +1147,38 @@ def _lanczos_spectra(A, B, e0, o, gamma, ntri, eng):
     """Spectra of the Lanczos branch from the coefficients: pole range from the extreme
     eigenvalues of every tridiagonal matrix, the default Emin/Emax/Gamma from it
     (ssp.cpp:2651-2684), all spectra at all frequencies in one kernel."""
+    if isinstance(eng, Engine):
+        W = _chain_extremes(A, B, ntri, eng)
+    else:
+        W = np.empty((A.shape[0], 2))
+        for s in range(A.shape[0]):
+            m = ntri
+            for k in range(1, ntri):  # a chain that ended early (b = 0) is shorter
+                if B[s, k] == 0.0:
+                    m = k
+                    break
+            W[s] = _tri_extremes(A[s, 1:m + 1], B[s, 1:m])
     lo, hi = np.inf, -np.inf
     for s in range(A.shape[0]):
-        m = ntri
-        for k in range(1, ntri):  # a chain that ended early (b = 0) is shorter
-            if B[s, k] == 0.0:
-                m = k
-                break
-        w0, w1 = _tri_extremes(A[s, 1:m + 1], B[s, 1:m])
-        lo, hi = min(lo, w0 - e0[s]), max(hi, w1 - e0[s])
+        lo, hi = min(lo, W[s, 0] - e0[s]), max(hi, W[s, 1] - e0[s])
     emin, emax, NE = o["Emin"], o["Emax"], int(o["NE"])
     emin, emax, gamma = _default_window(lo, hi, emin, emax, gamma, NE)
     G = TriDiagonalMatrixToSpectrum(e0, A, B, emin, emax, NE, gamma, eng)
     tri = [(np.r_[0.0, A[s, 1:] - e0[s]], B[s].copy()) for s in range(A.shape[0])]
     return Spectra(G, emin, emax, NE, gamma, lo, hi), tri
+
+
+def _chain_extremes(A, B, ntri, eng):
+    """_tri_extremes of every chain at once on the device; rows of A and B as in qg_cf_spectra."""
+    a = np.ascontiguousarray(A[:, :ntri + 1], dtype=np.float64)
+    b = np.ascontiguousarray(B[:, :ntri], dtype=np.float64)
+    live = np.cumprod(b[:, 1:] != 0.0, axis=1, dtype=bool)  # the steps before a chain's end
+    if not (np.isfinite(a[:, 1]).all() and np.isfinite(np.where(live, a[:, 2:], 0.0)).all()
+            and np.isfinite(np.where(live, b[:, 1:], 0.0)).all()):
+        raise ValueError("array must not contain infs or NaNs")
+    w = np.empty((len(a), 2))
+    eng.check(eng.L.qg_tri_extremes(eng.ctx, len(a), ntri, _ptr(a), _ptr(b), 1, _ptr(w)))
+    return w
 
 
 def _tri_extremes(a, b):

@@ -326,44 +326,6 @@ extern "C" qg_status qg_lanczos_krylov(qg_context ctx, qg_operator op, qg_basis 
 
 // ------------------------------------------------------------------ RIXS
 
-// Lowest and highest eigenvalue of the symmetric tridiagonal matrix diag a[1..nt], off-diagonal
-// b[1..nt-1] by bisection on Sturm counts inside the Gershgorin interval: only the final-state
-// pole range is needed of the second-stage chains, not their eigenvectors.
-static int sturm_below(int nt, const double *a, const double *b, double x) {
-  int cnt = 0;
-  double d = 1.0;
-  for (int i = 0; i < nt; i++) {
-    const double off = i ? b[i] * b[i] : 0.0;
-    d = (a[i + 1] - x) - (i ? off / d : 0.0);
-    if (d == 0.0) d = -1e-300;  // a zero pivot counts as negative (the limit from below)
-    cnt += d < 0.0;
-  }
-  return cnt;
-}
-
-static void tridiag_extremes(int nt, const double *a, const double *b, double *lo, double *hi) {
-  double g0 = DBL_MAX, g1 = -DBL_MAX;
-  for (int i = 0; i < nt; i++) {
-    const double r = (i ? std::fabs(b[i]) : 0.0) + (i + 1 < nt ? std::fabs(b[i + 1]) : 0.0);
-    g0 = std::min(g0, a[i + 1] - r);
-    g1 = std::max(g1, a[i + 1] + r);
-  }
-  for (int which = 0; which < 2; which++) {
-    // the eigenvalue with (which ? nt - 1 : 0) eigenvalues below it
-    const int target = which ? nt - 1 : 0;
-    double l = g0, h = g1;
-    for (int it = 0; it < 200 && h - l > 4 * DBL_EPSILON * std::max(std::fabs(l), std::fabs(h)); it++) {
-      const double m = 0.5 * (l + h);
-      if (m <= l || m >= h) break;
-      if (sturm_below(nt, a, b, m) > target)
-        h = m;
-      else
-        l = m;
-    }
-    (which ? *hi : *lo) = 0.5 * (l + h);
-  }
-}
-
 extern "C" qg_status qg_resonant_spectra(qg_context ctx, qg_operator H1, qg_operator H2, qg_operator T1,
                                          const qg_operator *T2, int32_t nt2, qg_basis psi_basis, const double *psi_dev,
                                          qg_rixs_settings *o, double *g_host) {
@@ -473,11 +435,11 @@ extern "C" qg_status qg_resonant_spectra(qg_context ctx, qg_operator H1, qg_oper
     if (st != QG_OK) break;
     // final-state energy range from the poles (Core/ResonantSpectra.cpp:221-262)
     double lo = DBL_MAX, hi = -DBL_MAX;
+    std::vector<double> ends(2 * (size_t)ncol);
+    if ((st = qg_tri_extremes(ctx, ncol, o->ntri2, a2.data(), b2v.data(), 0, ends.data())) != QG_OK) break;
     for (int c = 0; c < ncol; c++) {
-      double e0, e1;
-      tridiag_extremes(o->ntri2, &a2[(size_t)c * (o->ntri2 + 1)], &b2v[(size_t)c * o->ntri2], &e0, &e1);
-      lo = std::min(lo, e0 - o->energy2);
-      hi = std::max(hi, e1 - o->energy2);
+      lo = std::min(lo, ends[2 * c] - o->energy2);
+      hi = std::max(hi, ends[2 * c + 1] - o->energy2);
     }
     if (o->emin2 > 0.001 * DBL_MAX || o->emax2 < -0.001 * DBL_MAX) {
       if (o->emin2 > 0.001 * DBL_MAX && o->emax2 < -0.001 * DBL_MAX) {

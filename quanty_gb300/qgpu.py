@@ -78,6 +78,7 @@ def load(path=LIB_PATH):
         "qg_axpy": (C.c_int, [P, I64, I32, P, P, P]),
         "qg_lanczos_tridiag": (C.c_int, [P, P, P, P, I32, I32, D, D, P, P, P]),
         "qg_cf_spectra": (C.c_int, [P, I32, I32, P, P, P, D, D, I32, D, P]),
+        "qg_tri_extremes": (C.c_int, [P, I32, I32, P, P, I32, P]),
         "qg_block_lanczos": (C.c_int, [P, P, P, P, I32, I32, D, D, P, P, P, P]),
         "qg_krylov_combine": (C.c_int, [P, P, I64, I32, P, I32, P]),
         "qg_block_adjoint_product": (C.c_int, [P, P, I32, I32, P, I32, I32, I64, P]),

@@ -302,12 +302,13 @@ qg_status qg_all_real(qg_context ctx, const double2 *v, int64_t n, bool *real) {
 // w orthogonal to eps, as the second of two full ones does: V is read twice per step, not four
 // times.  Bound by those two reads from L2 (FP64 above a few hundred thousand rows) and by the
 // latency of four dependent kernels of 5 to 15 us, so each is launched while the one before it drains.
-// Ground state of a 29,635-determinant impurity to a variance of 1e-12, 1305 steps in 9
-// restarts: 63 ms, with plain launches 75 ms, with block products of one column (complex
-// storage, 16 bytes per entry strided by the Krylov dimension), host round trips and allocations in
-// every step 578 ms.  Not faster: a block's warps sharing out the vectors of the update, over 32 or
+// Ground state of a 29,635-determinant impurity to a variance of 1e-12, 1305 steps in 9 restarts, with
+// closure and spectrum: 58 ms (75 with plain launches and every projected matrix reduced in full);
+// with block products of one column (complex storage, 16 bytes per entry strided by the Krylov
+// dimension), host round trips and allocations in every step 578 ms.  Not faster: a block's warps sharing out the vectors of the update, over 32 or
 // 64 rows (to a variance of 1e-10 43.2 to 53 ms, a row per thread 42.5 and 50.8), and letting the next
 // kernel's blocks up before the last block of the one before has ended (52).
+
 // scalars of the chain, in device memory
 struct OneScal {
   double alpha;  // a_j of the current step
@@ -461,7 +462,8 @@ __global__ void __launch_bounds__(128)
   x[r] = one_minus_sum(one_zero(T()), V, n, k, cs, r);
 }
 
-#define ONE_STRAY 4.0  // 0.25 to 1.1 where the space has not run out (1,245 and 29,635 determinants, 101 to 167 vectors)
+#define ONE_STRAY 4.0  // measured 0.25 to 1.1 where the space has not run out (1,245 and 29,635
+                       // determinants, 101 to 167 vectors)
 #define ONE_MAX_K 2500  // the coefficients of a step fit one block's default shared memory
 
 // One wanted state on a basis with connection lists: the restarts of qg_block_groundstate with

@@ -1174,6 +1174,78 @@ __global__ void k_diag(const Key<W> *__restrict__ rows, int64_t n, const GroupDe
   diag[r] = acc;
 }
 
+// k_diag with a warp per row, for bases of few rows: the lanes test 32 groups at a time and, where a
+// group holds one term (densities and their products), form its value; the sum runs over them in
+// k_diag's order, so the bits are the same.  A thread per row is a chain through the whole table, 66 to
+// 94 us for 16 to 66 orbitals however few the rows are; a warp per row costs a full FP64
+// instruction for every term of a row.  26 orbitals, 1,245 rows 66 -> 21 us; 56 orbitals, 780 rows
+// 94 -> 28, 15,045 rows 88 -> 236; 46 orbitals, 10,445 rows 82 -> 157: the line lies below where they meet,
+// about 5,000 rows.
+#define QG_DIAG_WARP_ROWS 16  // rows per SM up to which a warp takes a row
+template <int W>
+__global__ void __launch_bounds__(128)
+    k_diag_warp(const Key<W> *__restrict__ rows, int64_t n, const GroupDev<W> *__restrict__ groups, int ngroups,
+                const TermDev<W> *__restrict__ terms, double2 *diag) {
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int64_t r = (blockIdx.x * (int64_t)128 + threadIdx.x) >> 5;
+  if (r >= n) return;
+  const Key<W> d = rows[r];
+  double2 acc = make_double2(0.0, 0.0);
+  double vr = 0.0, vi = 0.0;
+  auto applies = [&](int t) {  // term t on the row: its signed value in vr, vi
+    bool app = true;
+    int par = 0;
+#pragma unroll
+    for (int i = 0; i < W; i++) {
+      app &= (d.w[i] & terms[t].need0[i]) == 0;
+      par += __popcll(d.w[i] & terms[t].sgn[i]);
+    }
+    vr = qg_flip_sign(terms[t].vre, par);
+    vi = qg_flip_sign(terms[t].vim, par);
+    return app;
+  };
+  auto add = [&](int src) {
+    acc.x += __shfl_sync(full, vr, src);
+    const double y = __shfl_sync(full, vi, src);
+    if (qg_is_nonzero(y)) acc.y += y;
+  };
+  for (int g0 = 0; g0 < ngroups; g0 += 32) {
+    const int g = g0 + lane;
+    bool ok = g < ngroups;
+    int b = 0, e = 0;
+    if (ok) {
+#pragma unroll
+      for (int i = 0; i < W; i++) ok &= (d.w[i] & groups[g].need1[i]) == groups[g].need1[i];
+      b = groups[g].begin;
+      e = groups[g].end;
+    }
+    const bool one = e - b == 1;
+    if (ok && one) ok = applies(b);
+    const double gr = vr, gi = vi;
+    unsigned m = __ballot_sync(full, ok && e > b);
+    while (m) {
+      const int q = __ffs(m) - 1;
+      m &= m - 1;
+      const int bb = __shfl_sync(full, b, q), ee = __shfl_sync(full, e, q);
+      if (ee - bb == 1) {
+        add(q);
+        continue;
+      }
+      for (int t0 = bb; t0 < ee; t0 += 32) {
+        unsigned mt = __ballot_sync(full, t0 + lane < ee && applies(t0 + lane));
+        while (mt) {
+          add(__ffs(mt) - 1);
+          mt &= mt - 1;
+        }
+      }
+      vr = gr;
+      vi = gi;
+    }
+  }
+  if (lane == 0) diag[r] = acc;
+}
+
 template <int W>
 __global__ void k_local_cfg(const Key<W> *keys, int64_t n, int lo, uint32_t lmask, uint32_t *cfg, uint32_t *flag) {
   int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -1631,16 +1703,21 @@ static qg_status refresh_values(qg_basis b, qg_operator op, OpBasisCache &c) {
   return qg_check_launch(ctx, "value refresh");
 }
 
+template <int W>
+static void diag_of(qg_context ctx, qg_operator op, qg_basis b, double *d_diag) {
+  const bool few = b->n <= (int64_t)QG_DIAG_WARP_ROWS * ctx->num_sms;
+  auto kernel = few ? k_diag_warp<W> : k_diag<W>;
+  kernel<<<few ? (unsigned)((b->n + 3) / 4) : (unsigned)grid_for(b->n, 256), few ? 128 : 256, 0, ctx->stream>>>(
+      (const Key<W> *)b->d_keys, b->n, (const GroupDev<W> *)op->diag.d_groups, op->diag.ngroups,
+      (const TermDev<W> *)op->diag.d_terms, (double2 *)d_diag);
+}
+
 // the diagonal of op on every row of b (all flip == 0 terms), into d_diag
 static void launch_diag(qg_context ctx, qg_operator op, qg_basis b, double *d_diag) {
   if (op->W == 1)
-    k_diag<1><<<grid_for(b->n, 256), 256, 0, ctx->stream>>>((const Key<1> *)b->d_keys, b->n,
-                                                            (const GroupDev<1> *)op->diag.d_groups, op->diag.ngroups,
-                                                            (const TermDev<1> *)op->diag.d_terms, (double2 *)d_diag);
+    diag_of<1>(ctx, op, b, d_diag);
   else
-    k_diag<2><<<grid_for(b->n, 256), 256, 0, ctx->stream>>>((const Key<2> *)b->d_keys, b->n,
-                                                            (const GroupDev<2> *)op->diag.d_groups, op->diag.ngroups,
-                                                            (const TermDev<2> *)op->diag.d_terms, (double2 *)d_diag);
+    diag_of<2>(ctx, op, b, d_diag);
   ctx->launches++;
 }
 

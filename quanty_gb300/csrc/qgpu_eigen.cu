@@ -299,8 +299,12 @@ qg_status qg_all_real(qg_context ctx, const double2 *v, int64_t n, bool *real) {
 //   w -= V c;  b_(j+1) = |w|                                            (k_one_update)
 //   v_(j+1) = w / b_(j+1)                                               (k_one_scale)
 // The three-term part removes what is not small, so the one full projection after it leaves
-// w orthogonal to eps, as the second of two full ones does: V is read twice per step, not four
-// times.  Bound by those two reads from L2 (FP64 above a few hundred thousand rows) and by the
+// w orthogonal to eps, as the second of two full ones does, as long as it does not take more than
+// it leaves (|c| <= |w|): V is read twice per step, not four times.  Where it does take more, w was
+// rounding along the stored vectors (the space is invariant to rounding), what is left is not
+// orthogonal to them, and each further such step would multiply the loss: the space ends there.
+// The steps after it are zero, and the Ritz vector, normalised before its residual is taken, is formed of
+// the vectors before it.  Bound by those two reads from L2 (FP64 above a few hundred thousand rows) and by the
 // latency of four dependent kernels of 5 to 15 us, so each is launched while the one before it drains.
 // Ground state of a 29,635-determinant impurity to a variance of 1e-12, 1305 steps in 9 restarts, with
 // closure and spectrum: 58 ms (75 with plain launches and every projected matrix reduced in full);
@@ -316,7 +320,7 @@ struct OneScal {
   double scale;  // 1 / beta, 0 for a vanished vector
   double norm2;  // the squared norm of the last update
   unsigned long long stray;  // bits of the largest part of the projected matrix beside its tridiagonal one
-  int dead;      // first step whose next vector vanished (the space is invariant), else a large number
+  int dead;      // first step whose next vector is lost (the space is invariant), else a large number
   unsigned int tickets[1 + ONE_SHARES];
 };
 
@@ -370,8 +374,11 @@ __global__ void __launch_bounds__(256)
       });
 }
 
+#define ONE_TINY 1e-280  // a squared norm below has lost digits
+
 // w -= sum_i c_i v_i over i < k (out = w), and the squared norm of the result: the last block
-// leaves beta = |w|, its reciprocal and, when the vector vanished, the step in `dead`.
+// leaves beta = |w|, its reciprocal and, when the vector vanished or the projection took more than it
+// left, zero for both and the step in `dead`.
 template <bool REAL>
 __global__ void __launch_bounds__(128)
     k_one_update(const typename OneT<REAL>::T *V, int64_t n, int k, const typename OneT<REAL>::T *c,
@@ -381,10 +388,20 @@ __global__ void __launch_bounds__(128)
   T *cs = reinterpret_cast<T *>(smem_raw);
   __shared__ double sh[4];
   __shared__ int s_last;
+  __shared__ unsigned s_top;
   const int tid = threadIdx.x;
   qg_chain_wait();
   for (int i = tid; i < k; i += 128) cs[i] = c[i];
   __syncthreads();
+  if (k && tid >= 96) {  // the largest upper word of c's parts: |c|^2 <= t by it unless t is rounding
+    unsigned top = 0;
+    for (int i = tid - 96; i < k; i += 32) {
+      const double2 z = one_complex(cs[i]);
+      top = max(top, (unsigned)max(__double2hiint(z.x) & 0x7fffffff, __double2hiint(z.y) & 0x7fffffff));
+    }
+    top = __reduce_max_sync(0xffffffffu, top);
+    if (tid == 96) s_top = top;
+  }
   double s = 0.0;
   for (int64_t r = (int64_t)blockIdx.x * 128 + tid; r < n; r += (int64_t)gridDim.x * 128) {
     const T x = one_minus_sum(w[r], V, n, k, cs, r);
@@ -393,11 +410,17 @@ __global__ void __launch_bounds__(128)
   }
   const double t = one_total128(s, part, sh, &s_last, &sc->tickets[0]);
   if (s_last && tid == 0) {
-    const double b = sqrt(t);
+    const double b = sqrt(t), cm = __hiloint2double((int)s_top, -1);  // no part of c is above cm
+    bool lost = !(t > (k ? ONE_TINY : 0.0));
+    if (k && !lost && !(cm * cm * (2.0 * k) <= t)) {
+      double c2 = 0.0;
+      for (int i = 0; i < k; i++) c2 += one_abs2(cs[i]);
+      lost = !(c2 <= t);
+    }
     sc->norm2 = t;
-    sc->beta = b;
-    sc->scale = b > 0.0 ? 1.0 / b : 0.0;
-    if (!(b > 0.0) && step < sc->dead) sc->dead = step;
+    sc->beta = lost ? 0.0 : b;
+    sc->scale = lost ? 0.0 : 1.0 / b;
+    if (lost && step < sc->dead) sc->dead = step;
   }
 }
 
@@ -583,7 +606,7 @@ static qg_status groundstate_one(qg_context ctx, qg_operator op, qg_basis b, dou
       st = qg_cuda_fail(ctx, e, "qg_block_groundstate");
       break;
     }
-    const int k = std::min(Kcur, h.dead + 1);  // the vectors before the one that vanished
+    const int k = std::min(Kcur, h.dead + 1);  // the vectors before the one that was lost
     if (k <= 0) {
       ctx->last_error = "qg_block_groundstate: start vectors are zero";
       st = QG_ERR_ARG;
@@ -591,7 +614,9 @@ static qg_status groundstate_one(qg_context ctx, qg_operator op, qg_basis b, dou
     }
     if ((st = lowest(k, h.stray)) != QG_OK) break;
     k_one_combine<REAL><<<gc, 128, (size_t)k * sizeof(T), s>>>(V, n, k, Y, x);
-    ctx->launches++;
+    k_one_update<REAL><<<gu, 128, 0, s>>>(V, n, 0, c, x, npart, 1 << 30, sc);
+    k_one_scale<REAL><<<g1, 256, 0, s>>>(n, x, sc, x, nullptr);
+    ctx->launches += 3;
     // the variance |H x - theta x|^2, from the residual itself
     fz.prev = (const double2 *)x;
     fz.beta = wd;

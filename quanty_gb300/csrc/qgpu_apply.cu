@@ -1469,68 +1469,82 @@ uint32_t to_local(const uint64_t *m, int lo, int W) {
 
 }  // namespace
 
-// the operator's local terms on the device, grouped by flip, with its current values
-static qg_status local_terms(qg_context ctx, qg_operator op) {
-  if (op->n_lflip >= 0 && op->lterm_version == op->version) return QG_OK;
+// the operator's local terms with its current values, grouped by flip: the flips, then the terms (device).
+// Each build of a basis' moves copies them to a block of its own, used in the order of its context's stream.
+struct LocalTerms {
+  void *d = nullptr;
+  int nflip = 0;
+  const LocalFlip *flips() const { return (const LocalFlip *)d; }
+  const LocalTerm *terms() const { return (const LocalTerm *)((const char *)d + term_offset(nflip)); }
+  static size_t term_offset(size_t nflip) { return (nflip * sizeof(LocalFlip) + 15) / 16 * 16; }
+};
+
+// the same on the host, kept by the operator for its value version (contexts in several threads may
+// share it)
+static std::shared_ptr<const LocalTable> local_table(qg_operator op) {
+  std::lock_guard<std::mutex> l(op->local_m);
+  if (op->local_tab && op->local_tab->version == op->version) return op->local_tab;
   const int lo = op->nf - op->H, W = op->W;
-  std::map<uint32_t, std::vector<LocalTerm>> by;
-  for (auto &t : op->local_off)
-    by[to_local(t.fl, lo, W)].push_back(
-        {to_local(t.n1, lo, W), to_local(t.n0, lo, W), to_local(t.sg, lo, W), 0u, t.re, t.im});
+  // the terms of a flip stay in the operator's order
+  std::vector<std::pair<uint32_t, int>> by(op->local_off.size());
+  for (size_t i = 0; i < by.size(); i++) by[i] = {to_local(op->local_off[i].fl, lo, W), (int)i};
+  std::sort(by.begin(), by.end());
   std::vector<LocalFlip> flips;
   std::vector<LocalTerm> terms;
-  for (auto &kv : by) {
-    LocalFlip f{kv.first, (int)terms.size(), 0};
-    terms.insert(terms.end(), kv.second.begin(), kv.second.end());
-    f.end = (int)terms.size();
-    flips.push_back(f);
+  for (auto &f : by) {
+    const HostTerm &t = op->local_off[f.second];
+    if (flips.empty() || flips.back().fl != f.first) flips.push_back({f.first, (int)terms.size(), 0});
+    terms.push_back({to_local(t.n1, lo, W), to_local(t.n0, lo, W), to_local(t.sg, lo, W), 0u, t.re, t.im});
+    flips.back().end = (int)terms.size();
   }
-  cudaError_t e = cudaSuccess;
-  if (op->n_lflip < 0) {
-    e = qg_malloc_bytes(op->ctx, &op->d_lflip, std::max<size_t>(flips.size(), 1) * sizeof(LocalFlip));
-    if (e == cudaSuccess) e = qg_malloc_bytes(op->ctx, &op->d_lterm, std::max<size_t>(terms.size(), 1) * sizeof(LocalTerm));
+  auto tab = std::make_shared<LocalTable>();
+  tab->version = op->version;
+  tab->nflip = (int)flips.size();
+  const size_t off = LocalTerms::term_offset(flips.size());
+  tab->blob.resize(off + terms.size() * sizeof(LocalTerm));
+  if (!flips.empty()) {
+    memcpy(tab->blob.data(), flips.data(), flips.size() * sizeof(LocalFlip));
+    memcpy(tab->blob.data() + off, terms.data(), terms.size() * sizeof(LocalTerm));
   }
-  if (e == cudaSuccess && !flips.empty()) {
-    e = cudaMemcpyAsync(op->d_lflip, flips.data(), flips.size() * sizeof(LocalFlip), cudaMemcpyHostToDevice, ctx->stream);
-    if (e == cudaSuccess) e = qg_upload(ctx, op->d_lterm, terms.data(), terms.size() * sizeof(LocalTerm));
-  }
-  if (e != cudaSuccess) {
-    if (op->n_lflip < 0) {
-      qg_free(op->d_lflip);
-      qg_free(op->d_lterm);
-      op->d_lflip = op->d_lterm = nullptr;
-    }
-    return qg_cuda_fail(ctx, e, "local terms");
-  }
-  op->n_lflip = (int)flips.size();
-  op->lterm_version = op->version;
-  return QG_OK;
+  return op->local_tab = tab;
+}
+
+static qg_status local_terms(qg_context ctx, qg_operator op, LocalTerms *out) {
+  const std::shared_ptr<const LocalTable> tab = local_table(op);
+  out->nflip = tab->nflip;
+  cudaError_t e = qg_malloc_bytes(ctx, &out->d, std::max<size_t>(tab->blob.size(), 16));
+  if (e == cudaSuccess && !tab->blob.empty())
+    e = cudaMemcpyAsync(out->d, tab->blob.data(), tab->blob.size(), cudaMemcpyHostToDevice, ctx->stream);
+  if (e == cudaSuccess) return QG_OK;
+  qg_free(out->d);
+  out->d = nullptr;
+  return qg_cuda_fail(ctx, e, "local terms");
 }
 
 template <int W>
-static void launch_local_entries_w(qg_context ctx, qg_operator op, qg_basis b, const OpBasisCache &c, bool fill,
-                                   uint32_t *cnt, unsigned int *flags) {
-  const size_t smem = (size_t)std::max(1, (op->n_lflip + 31) / 32) * 4;
-  const LocalFlip *f = (const LocalFlip *)op->d_lflip;
-  const LocalTerm *t = (const LocalTerm *)op->d_lterm;
+static void launch_local_entries_w(qg_context ctx, qg_operator op, const LocalTerms &lt, qg_basis b, const OpBasisCache &c,
+                                   bool fill, uint32_t *cnt, unsigned int *flags) {
+  const size_t smem = (size_t)std::max(1, (lt.nflip + 31) / 32) * 4;
+  const LocalFlip *f = lt.flips();
+  const LocalTerm *t = lt.terms();
   const int lo = b->nf - op->H, kz = op->keep_zero ? 1 : 0;
   if (fill)
-    k_local_entries<W, true><<<c.nblocks, 128, smem, ctx->stream>>>(c.d_bcfg, f, op->n_lflip, t, c.d_cfg, c.d_bstart,
+    k_local_entries<W, true><<<c.nblocks, 128, smem, ctx->stream>>>(c.d_bcfg, f, lt.nflip, t, c.d_cfg, c.d_bstart,
                                                                     c.d_class, kz, lo, b->nres, b->d_rmask, cnt,
                                                                     c.d_eoff, c.d_ent, c.d_ent_target, flags);
   else
-    k_local_entries<W, false><<<c.nblocks, 128, smem, ctx->stream>>>(c.d_bcfg, f, op->n_lflip, t, c.d_cfg, c.d_bstart,
+    k_local_entries<W, false><<<c.nblocks, 128, smem, ctx->stream>>>(c.d_bcfg, f, lt.nflip, t, c.d_cfg, c.d_bstart,
                                                                      c.d_class, kz, lo, b->nres, b->d_rmask, cnt,
                                                                      nullptr, nullptr, nullptr, flags);
   ctx->launches++;
 }
 
-static void launch_local_entries(qg_context ctx, qg_operator op, qg_basis b, const OpBasisCache &c, bool fill,
-                                 uint32_t *cnt, unsigned int *flags) {
+static void launch_local_entries(qg_context ctx, qg_operator op, const LocalTerms &lt, qg_basis b, const OpBasisCache &c,
+                                 bool fill, uint32_t *cnt, unsigned int *flags) {
   if (b->W == 1)
-    launch_local_entries_w<1>(ctx, op, b, c, fill, cnt, flags);
+    launch_local_entries_w<1>(ctx, op, lt, b, c, fill, cnt, flags);
   else
-    launch_local_entries_w<2>(ctx, op, b, c, fill, cnt, flags);
+    launch_local_entries_w<2>(ctx, op, lt, b, c, fill, cnt, flags);
 }
 
 static qg_status build_local(qg_basis bs, qg_operator op, OpBasisCache &c) {
@@ -1624,7 +1638,8 @@ static qg_status build_local(qg_basis bs, qg_operator op, OpBasisCache &c) {
   }
   if (e != cudaSuccess) return qg_cuda_fail(ctx, e, "local blocks");
   // the moves: counted, then written
-  QG_TRY(local_terms(ctx, op));
+  LocalTerms lt;
+  QG_TRY(local_terms(ctx, op, &lt));
   uint32_t *cnt = nullptr;
   void *scan = nullptr;
   size_t sb = 0;
@@ -1635,7 +1650,7 @@ static qg_status build_local(qg_basis bs, qg_operator op, OpBasisCache &c) {
   if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(nullptr, sb, cnt, c.d_eoff, (int)nb + 1, s);
   if (e == cudaSuccess) e = qg_malloc_bytes(ctx, &scan, std::max<size_t>(sb, 16));
   if (e == cudaSuccess) {
-    launch_local_entries(ctx, op, bs, c, false, cnt, cnt + nb + 1);
+    launch_local_entries(ctx, op, lt, bs, c, false, cnt, cnt + nb + 1);
     e = cub::DeviceScan::ExclusiveSum(scan, sb, cnt, c.d_eoff, (int)nb + 1, s);
     ctx->launches += 2;
   }
@@ -1645,7 +1660,7 @@ static qg_status build_local(qg_basis bs, qg_operator op, OpBasisCache &c) {
   if (e == cudaSuccess) e = qg_malloc(ctx, &c.d_ent, std::max<size_t>(c.nent, 1) * sizeof(LocalEntry));
   if (e == cudaSuccess) e = qg_malloc(ctx, &c.d_ent_target, std::max<size_t>(c.nent, 1) * 4);
   if (e == cudaSuccess) {
-    launch_local_entries(ctx, op, bs, c, true, cnt, cnt + nb + 1);
+    launch_local_entries(ctx, op, lt, bs, c, true, cnt, cnt + nb + 1);
     if (c.wreq_exact) {
       e = cudaMemcpyAsync(head + 1, cnt + nb + 1, 4, cudaMemcpyDeviceToHost, s);
       if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -1653,6 +1668,7 @@ static qg_status build_local(qg_basis bs, qg_operator op, OpBasisCache &c) {
   }
   qg_free(cnt);
   qg_free(scan);
+  qg_free(lt.d);
   if (e != cudaSuccess) return qg_cuda_fail(ctx, e, "local entries");
   if (head[1]) c.wreq_exact = false;
   return qg_check_launch(ctx, "local entries");
@@ -1661,11 +1677,14 @@ static qg_status build_local(qg_basis bs, qg_operator op, OpBasisCache &c) {
 // new values of a sum operator: the entries again, in place (their structure does not change)
 static qg_status refresh_local(qg_basis bs, qg_operator op, OpBasisCache &c) {
   if (c.nent == 0) return QG_OK;
-  QG_TRY(local_terms(bs->ctx, op));
+  LocalTerms lt;
+  QG_TRY(local_terms(bs->ctx, op, &lt));
   unsigned int *flags = nullptr;
-  QG_CUDA(bs->ctx, qg_malloc(bs->ctx, &flags, sizeof(unsigned int)));
-  launch_local_entries(bs->ctx, op, bs, c, true, nullptr, flags);
+  const cudaError_t e = qg_malloc(bs->ctx, &flags, sizeof(unsigned int));
+  if (e == cudaSuccess) launch_local_entries(bs->ctx, op, lt, bs, c, true, nullptr, flags);
   qg_free(flags);
+  qg_free(lt.d);
+  if (e != cudaSuccess) return qg_cuda_fail(bs->ctx, e, "local entries");
   return qg_check_launch(bs->ctx, "local entries");
 }
 

@@ -18,6 +18,7 @@
 #include <stdint.h>
 
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -129,6 +130,13 @@ struct HostTerm {
   int src = -1, sgn = 1;  // forward term it came from, sign its value carries
 };
 
+// local_off grouped by flip, as the device reads it (qgpu_apply.cu), and the value version it holds
+struct LocalTable {
+  uint64_t version = 0;
+  int nflip = 0;
+  std::vector<unsigned char> blob;
+};
+
 struct qg_operator_s {
   qg_context ctx = nullptr;
   int nf = 0, W = 1;
@@ -145,11 +153,8 @@ struct qg_operator_s {
   // configuration of a basis; the rest (pull_nl, host copy nl_host in table order) is scanned
   int H = 0;
   std::vector<HostTerm> local_off;
-  // local_off on the device (qgpu_apply.cu), grouped by flip: LocalFlip[n_lflip], LocalTerm[], and
-  // the value version they hold
-  void *d_lflip = nullptr, *d_lterm = nullptr;
-  int n_lflip = -1;
-  uint64_t lterm_version = 0;
+  std::mutex local_m;  // guards local_tab
+  std::shared_ptr<const LocalTable> local_tab;
   HostTable pull_nl;
   std::vector<HostTerm> nl_host;
   // forward terms in creation order (masks and values)

@@ -431,8 +431,6 @@ extern "C" qg_status qg_operator_create(qg_context ctx, int32_t nf, int32_t nter
 extern "C" qg_status qg_operator_destroy(qg_operator op) {
   if (!op) return QG_OK;
   qg_free_now(op->pull.d_blob);  // waits for the device: another context may still be using the operator
-  qg_free(op->d_lflip);
-  qg_free(op->d_lterm);
   qg_free(op->pull_off.d_blob);
   qg_free(op->diag.d_blob);
   qg_free(op->pull_nl.d_blob);

@@ -1719,6 +1719,7 @@ static qg_status refresh_values(qg_basis b, qg_operator op, OpBasisCache &c) {
     }
   }
   c.op_version = op->version;
+  c.complete = false;
   return qg_check_launch(ctx, "value refresh");
 }
 
@@ -1740,15 +1741,21 @@ static void launch_diag(qg_context ctx, qg_operator op, qg_basis b, double *d_di
   ctx->launches++;
 }
 
-OpBasisCache *qg_basis_cache(qg_basis b, qg_operator op, qg_status *st) {
+// The cache is filled on the stream of the basis' context: another context waits for it once.
+static qg_status cache_complete(qg_context user, qg_basis b, OpBasisCache &c) {
+  if (c.complete || user == b->ctx) return QG_OK;
+  QG_CUDA(user, cudaStreamSynchronize(b->ctx->stream));
+  c.complete = true;
+  return QG_OK;
+}
+
+OpBasisCache *qg_basis_cache(qg_context user, qg_basis b, qg_operator op, qg_status *st) {
   *st = QG_OK;
   for (auto &c : b->caches)
     if (c.op_uid == op->uid) {
-      if (c.op_version != op->version) {
-        *st = refresh_values(b, op, c);
-        if (*st != QG_OK) return nullptr;
-      }
-      return &c;
+      if (c.op_version != op->version) *st = refresh_values(b, op, c);
+      if (*st == QG_OK) *st = cache_complete(user, b, c);
+      return *st == QG_OK ? &c : nullptr;
     }
   qg_context ctx = b->ctx;
   if (b->caches.size() >= 4) {  // small cache: drop the oldest
@@ -1798,6 +1805,7 @@ OpBasisCache *qg_basis_cache(qg_basis b, qg_operator op, qg_status *st) {
   }
   b->caches.push_back(c);
   *st = qg_check_launch(ctx, "operator-basis cache");
+  if (*st == QG_OK) *st = cache_complete(user, b, b->caches.back());
   return &b->caches.back();
 }
 
@@ -1956,7 +1964,7 @@ bool qg_apply_uses_lists(qg_operator op, qg_basis b) {
   qg_context ctx = b->ctx;
   if (!ctx->conn_lists || op->nf != b->nf || b->n <= 0) return false;
   qg_status st = QG_OK;
-  OpBasisCache *c = qg_basis_cache(b, op, &st);
+  OpBasisCache *c = qg_basis_cache(ctx, b, op, &st);
   if (st != QG_OK || !c) return false;
   if (ensure_conn(ctx, op, b, c) != QG_OK) return false;
   return c->conn_state == 1;
@@ -2118,7 +2126,7 @@ qg_status qg_small_csr(qg_context ctx, qg_operator op, qg_basis b, int64_t max_n
   *out = SmallCsr();
   if (!qg_apply_uses_lists(op, b) || b->n > (1 << 30)) return QG_OK;
   qg_status st = QG_OK;
-  OpBasisCache *c = qg_basis_cache(b, op, &st);
+  OpBasisCache *c = qg_basis_cache(ctx, b, op, &st);
   if (st != QG_OK) return st;
   const HostTable *tab;
   LocalView lv;
@@ -2338,6 +2346,7 @@ static qg_status build_sell(qg_context ctx, qg_operator op, qg_basis b, OpBasisC
                                                          (double2 *)c->s_val, nullptr);
     ctx->launches++;
     e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // another context may use the rows next
   }
   if (e == cudaSuccess) {
     c->sell_state = 1;
@@ -2374,7 +2383,7 @@ static qg_status use_sell(qg_context ctx, qg_operator op, qg_basis b, OpBasisCac
 qg_status qg_apply_prepare(qg_context ctx, qg_operator op, qg_basis b, int applies) {
   if (!qg_apply_uses_lists(op, b)) return QG_OK;
   qg_status st = QG_OK;
-  OpBasisCache *c = qg_basis_cache(b, op, &st);
+  OpBasisCache *c = qg_basis_cache(ctx, b, op, &st);
   if (st != QG_OK) return st;
   bool use = false;
   return use_sell(ctx, op, b, c, applies, &use);
@@ -2476,7 +2485,7 @@ qg_status qg_apply_strided(qg_context ctx, qg_operator op, qg_basis dst, qg_basi
   int chunk = 8;
   if (dst == src && nvec >= 2) {
     qg_status st = QG_OK;
-    OpBasisCache *c = qg_basis_cache(dst, op, &st);
+    OpBasisCache *c = qg_basis_cache(ctx, dst, op, &st);
     if (st != QG_OK) return st;
     OpBasisCache::Chunk *p = chunk_of(c, nvec);
     if (ctx->autotune && !(p && p->settled)) {
@@ -2496,7 +2505,7 @@ qg_status qg_apply_strided(qg_context ctx, qg_operator op, qg_basis dst, qg_basi
 qg_status qg_apply_settle(qg_context ctx, qg_operator op, qg_basis b, const double *x, double *y, int nvec) {
   if (nvec < 2 || !ctx->autotune || !qg_apply_uses_lists(op, b)) return QG_OK;
   qg_status st = QG_OK;
-  OpBasisCache *c = qg_basis_cache(b, op, &st);
+  OpBasisCache *c = qg_basis_cache(ctx, b, op, &st);
   if (st != QG_OK) return st;
   const OpBasisCache::Chunk *p = chunk_of(c, nvec);
   return p && !p->settled ? autotune(ctx, op, b, c, x, nvec, y, nvec, nvec, true) : QG_OK;
@@ -2514,7 +2523,7 @@ static qg_status apply_chunked(qg_context ctx, qg_operator op, qg_basis dst, qg_
   LocalView lv{};
   lv.on = 0;
   if (dst == src) {
-    OpBasisCache *c = qg_basis_cache(dst, op, &st);
+    OpBasisCache *c = qg_basis_cache(ctx, dst, op, &st);
     if (st != QG_OK) return st;
     diag = (const double2 *)c->d_diag;
     if (op->H > 0) {
@@ -2747,7 +2756,7 @@ extern "C" qg_status qg_apply_set_chunk(qg_context ctx, qg_operator op, qg_basis
   if (!(chunk == 1 || chunk == 2 || chunk == 3 || chunk == 4 || chunk == 8 || chunk == -32 || chunk == -64))
     return QG_ERR_ARG;
   qg_status st = QG_OK;
-  OpBasisCache *c = qg_basis_cache(b, op, &st);
+  OpBasisCache *c = qg_basis_cache(ctx, b, op, &st);
   if (st != QG_OK) return st;
   if (OpBasisCache::Chunk *p = chunk_of(c, nvec)) {
     p->chunk = chunk;
@@ -2785,7 +2794,7 @@ extern "C" qg_status qg_apply_fp64_ops(qg_context ctx, qg_operator op, qg_basis 
     return QG_ERR_ARG;
   }
   qg_status st = QG_OK;
-  OpBasisCache *c = qg_basis_cache(b, op, &st);
+  OpBasisCache *c = qg_basis_cache(ctx, b, op, &st);
   if (st != QG_OK) return st;
   const HostTable *tab;
   LocalView lv;

@@ -181,6 +181,7 @@ struct LocalEntry {
 struct OpBasisCache {
   uint64_t op_uid = 0;
   uint64_t op_version = 0;        // the operator's value version the cached values belong to
+  bool complete = false;          // a context other than the basis' own has waited for its build
   double *d_diag = nullptr;       // complex per row: all diagonal terms
   uint64_t *d_wreq = nullptr;     // per term of op->pull_nl: window bits its source needs
   bool wreq_exact = false;        // every term's window change fits the bit encoding
@@ -375,7 +376,7 @@ qg_status qg_basis_build_hash(qg_basis b);
 qg_status qg_basis_set_windows(qg_basis b, int nres, const uint64_t *mask_host, const int32_t *min_host,
                                const int32_t *max_host);
 // per-(operator, basis) cache (diagonal, window bits, local blocks); nullptr on failure
-OpBasisCache *qg_basis_cache(qg_basis b, qg_operator op, qg_status *st);
+OpBasisCache *qg_basis_cache(qg_context user, qg_basis b, qg_operator op, qg_status *st);
 void qg_cache_free(OpBasisCache &c);
 
 // Epilogue options for the fused Lanczos step (see qgpu_krylov.cu):

@@ -77,3 +77,28 @@ def test_operator_of_another_context(api, engines):
     a.torch.cuda.synchronize()
     for w, (ya, yb) in zip(want, got):
         assert np.array_equal(w, ya.cpu().numpy()) and np.array_equal(w, yb.cpu().numpy())
+
+
+def test_fresh_caches(api, engines):
+    """Context B applies right behind A's call that built the moves, and right behind the one that built
+    the explicit rows."""
+    a, b = engines
+    ops, R, det = _operators(api, 3)
+    start = api.dets_to_bytes([det], ops[0].nf)
+    basis = api.closure(ops[0], start, ops[0].nf, R, -1, a)
+    xs = _vectors(a, basis.n, 2)
+    want = _reference(api, a, ops, basis, xs)
+    fresh = api.closure(ops[0], start, ops[0].nf, R, -1, a)
+    ys = [[e.empty(fresh.n) for _ in range(6)] for e in (a, b)]
+    a.torch.cuda.synchronize()
+    for i, H in enumerate(ops):
+        for k in range(6):  # the rows are there from the fourth apply on; B alone applies on the odd rounds
+            x = xs[k % 2]
+            if (i + k) % 2 == 0:
+                _apply(api, a, H.handle(a), fresh, x, ys[0][k])
+            _apply(api, b, H.handle(a), fresh, x, ys[1][k])
+        a.torch.cuda.synchronize()
+        for k in range(6):
+            w = want[2 * i + k % 2]
+            assert np.array_equal(w, ys[1][k].cpu().numpy())
+            assert (i + k) % 2 or np.array_equal(w, ys[0][k].cpu().numpy())

@@ -150,7 +150,8 @@ cudaError_t qg_free(void *p) {
 }
 
 cudaError_t qg_free_now(void *p) {
-  if (p) {
+  if (!p) return cudaSuccess;
+  {
     std::lock_guard<std::mutex> l(g_live_m);
     g_live.erase(p);
   }

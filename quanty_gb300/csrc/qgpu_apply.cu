@@ -1759,7 +1759,9 @@ OpBasisCache *qg_basis_cache(qg_context user, qg_basis b, qg_operator op, qg_sta
     }
   qg_context ctx = b->ctx;
   if (b->caches.size() >= 4) {  // small cache: drop the oldest
-    cudaStreamSynchronize(ctx->stream);
+    // waits for the device: another context may still be applying with it
+    qg_free_now(b->caches.front().d_diag);
+    b->caches.front().d_diag = nullptr;
     qg_cache_free(b->caches.front());
     b->caches.erase(b->caches.begin());
   }

@@ -172,7 +172,7 @@ static qg_status build_hash_t(qg_basis b) {
   qg_context ctx = b->ctx;
   int64_t hcap = hcap_for(b->n);
   if (b->d_slots && b->hcap != hcap) {
-    qg_free(b->d_slots);
+    qg_free_now(b->d_slots);  // waits for the device, as in qg_basis_destroy
     qg_free(b->d_slot_row);
     b->d_slots = nullptr;
     b->d_slot_row = nullptr;
@@ -356,7 +356,7 @@ extern "C" qg_status qg_basis_destroy(qg_basis b) {
 qg_status qg_basis_set_windows(qg_basis b, int nres, const uint64_t *mask_host, const int32_t *min_host,
                                const int32_t *max_host) {
   qg_context ctx = b->ctx;
-  qg_free(b->d_rmask);
+  qg_free_now(b->d_rmask);  // waits for the device, as in qg_basis_destroy
   qg_free(b->d_rmin);
   qg_free(b->d_rmax);
   b->d_rmask = nullptr;

@@ -347,8 +347,8 @@ qg_status qg_check_launch(qg_context ctx, const char *what);
 // waits for the whole device) in every call: an H*psi with growth from 38,635 determinants made
 // 31 of them, 4.05 ms with and 2.79 ms without; T*psi from 45, 0.94 and 0.51 ms.
 // Everything a context allocates is used in the order of its stream, which is what makes the
-// reuse safe; what other contexts may use too (bases, operators) is destroyed after a wait for
-// the device.  Bounded (QG_POOL_BYTES per context; larger blocks are not kept), given back by
+// reuse safe; what other contexts may use too (bases, operators, the caches of a basis) goes back
+// after a wait for the device, the qg_free_now of its first block.  Bounded (QG_POOL_BYTES per context; larger blocks are not kept), given back by
 // qg_finalize and whenever an allocation fails.  While the stream is being captured the pool
 // stands aside.
 cudaError_t qg_malloc_bytes(qg_context ctx, void **p, size_t bytes);
@@ -357,7 +357,8 @@ inline cudaError_t qg_malloc(qg_context ctx, T **p, size_t bytes) {
   return qg_malloc_bytes(ctx, reinterpret_cast<void **>(p), bytes);
 }
 cudaError_t qg_free(void *p);
-// to the device at once, after a wait for everything running on it (cudaFree)
+// to the device at once, after a wait for everything running on it (cudaFree: a kernel in flight may
+// be using any block)
 cudaError_t qg_free_now(void *p);
 // free device memory, counting what the pools hold as free
 cudaError_t qg_mem_info(size_t *free_bytes, size_t *total_bytes);

@@ -102,3 +102,26 @@ def test_fresh_caches(api, engines):
             w = want[2 * i + k % 2]
             assert np.array_equal(w, ys[1][k].cpu().numpy())
             assert (i + k) % 2 or np.array_equal(w, ys[0][k].cpu().numpy())
+
+
+def test_evicted_caches(api, engines):
+    """A basis keeps four operators: context A goes round seven of them, so that caches are dropped and
+    their blocks used again, while context B has applies queued on them."""
+    a, b = engines
+    ops, R, det = _operators(api, 7)
+    basis = api.closure(ops[0], api.dets_to_bytes([det], ops[0].nf), ops[0].nf, R, -1, a)
+    xs = _vectors(a, basis.n, 1)
+    want = _reference(api, a, ops, basis, xs)
+    ys = [b.empty(basis.n) for _ in range(14)]
+    ya = a.empty(basis.n)
+    val = np.zeros(2)
+    a.torch.cuda.synchronize()
+    for k in range(14):
+        h = ops[k % 7].handle(a)
+        for _ in range(8):
+            _apply(api, b, h, basis, xs[0], ys[k])
+        # another operator: a new cache, an eviction from the fifth on; and blocks taken and written
+        _apply(api, a, ops[(k + 1) % 7].handle(a), basis, xs[0], ya)
+        a.check(a.L.qg_expectation(a.ctx, ops[(k + 1) % 7].handle(a), basis.h, api._ptr(xs[0]), 1, api._ptr(val)))
+    a.torch.cuda.synchronize()
+    assert all(np.array_equal(want[k % 7], ys[k].cpu().numpy()) for k in range(14))

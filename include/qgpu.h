@@ -65,6 +65,11 @@ const char *qg_last_error(qg_context ctx);
 /* Number of kernels this library launched on the context since qg_init (for accounting). */
 int64_t qg_launch_count(qg_context ctx);
 qg_status qg_synchronize(qg_context ctx);
+/* Contexts keep the blocks of finished calls for the next ones.  qg_device_memory: free and total
+ * bytes of a device, these idle blocks counted as free; qg_trim gives them back (for an allocator
+ * beside the library that has run out). */
+qg_status qg_device_memory(int device, int64_t *free_bytes, int64_t *total_bytes);
+qg_status qg_trim(int device);
 
 /* ------------------------------------------------------------------ operators */
 

@@ -69,8 +69,7 @@ class Engine:
         return int(self.L.qg_launch_count(self.ctx))
 
     def empty(self, n, nvec=1):
-        with self.torch.cuda.stream(self.stream):
-            return self.torch.zeros((max(n, 1), nvec), dtype=self.torch.complex128, device="cuda:%d" % self.device)
+        return _allocate(self, lambda dev: self.torch.zeros((max(n, 1), nvec), dtype=self.torch.complex128, device=dev))
 
     def on_stream(self):
         """Context manager: torch work ordered with this engine's kernels."""
@@ -92,6 +91,19 @@ class Engine:
             self.close()
         except Exception:
             pass
+
+
+def _allocate(eng, make):
+    """make(device), a torch allocation, on the engine's stream; where torch is out of memory, once
+    more without the blocks that the library's contexts keep between calls."""
+    dev = "cuda:%d" % eng.device
+    with eng.on_stream():
+        try:
+            return make(dev)
+        except eng.torch.cuda.OutOfMemoryError:
+            pass
+        eng.check(eng.L.qg_trim(eng.device))
+        return make(dev)
 
 
 def engine():
@@ -478,8 +490,7 @@ def _upload(eng, basis, perm, values, nvec=1):
     v = np.zeros((max(n, 1), nvec), dtype=np.complex128)
     vals = np.asarray(values).reshape(len(perm), nvec)
     np.add.at(v, perm, vals)
-    with eng.on_stream():
-        return torch.from_numpy(v).to("cuda:%d" % eng.device)
+    return _allocate(eng, lambda dev: torch.from_numpy(v).to(dev))
 
 
 # ----------------------------------------------------------------------------- H * psi
@@ -866,8 +877,7 @@ def _spectra_tensor(H, Tpsi, E0, o, R, method, eng):
         G = (ListOfPolesToSpectrum(0.0, poles, Wt.real.copy(), emin, emax, NE, gamma, eng)
              + 1j * ListOfPolesToSpectrum(0.0, poles, Wt.imag.copy(), emin, emax, NE, gamma, eng))
         return Spectra(G, emin, emax, NE, gamma, lo, hi), {"poles": poles, "weights": Wt}
-    with eng.on_stream():
-        x = eng.torch.from_numpy(X).to("cuda:%d" % eng.device).contiguous()
+    x = _allocate(eng, lambda dev: eng.torch.from_numpy(X).to(dev).contiguous())
     sv = float(o.get("SingularValue", DEFAULTS["SingularValue"]))
     A, B, sizes = block_lanczos(H, ub, x, ntri, eps, sv, eng)
     val, _ = hermitian_eigh(block_tridiagonal_dense(A, B), 0, eng)
@@ -1016,8 +1026,7 @@ def _krylov_vectors(H, basis, x, ntri, eps, eng):
     """The reference's Krylov-basis Lanczos on the device (qg_lanczos_krylov: full
     reorthogonalisation, orthogonality test, truncation): its non-empty vectors as
     wavefunctions (zero amplitudes left out, as the reference's truncated vectors), a and b."""
-    with eng.on_stream():
-        K = eng.torch.zeros((ntri, basis.n), dtype=eng.torch.complex128, device="cuda:%d" % eng.device)
+    K = _allocate(eng, lambda dev: eng.torch.zeros((ntri, basis.n), dtype=eng.torch.complex128, device=dev))
     a = np.zeros(ntri + 1)
     b = np.zeros(ntri)
     eng.check(eng.L.qg_lanczos_krylov(eng.ctx, H.handle(eng), basis.h, _ptr(x), ntri, eps, _ptr(a), _ptr(b), _ptr(K)))
@@ -1050,8 +1059,7 @@ def _batched_lanczos_device(H, Ts, psis, o, R, eng, pairs=None):
     for j, p in enumerate(psis):
         np.add.at(X[:, j], perm[off:off + p.N], np.asarray(p.val, dtype=np.complex128))
         off += p.N
-    with eng.on_stream():
-        Xd = torch.from_numpy(X).to("cuda:%d" % eng.device)
+    Xd = _allocate(eng, lambda dev: torch.from_numpy(X).to(dev))
     if o.get("E0") is None:
         out = np.zeros(2 * npsi)
         eng.check(eng.L.qg_expectation(eng.ctx, H.handle(eng), b0.h, _ptr(Xd), npsi, _ptr(out)))
@@ -1316,13 +1324,12 @@ def EigensystemOnBasis(H, basis, Npsi, options=None, eng=None, seed=12345, max_r
         x0 += 1j * rng.standard_normal((n, Npsi))
     # a real H starts from real vectors and keeps them real, as the reference's real-vector
     # solver does: the eigenstates come out real, and so do the Lanczos chains built on them
-    with eng.on_stream():
-        x = eng.torch.from_numpy(x0).to("cuda:%d" % eng.device).contiguous()
+    x = _allocate(eng, lambda dev: eng.torch.from_numpy(x0).to(dev).contiguous())
     en = np.zeros(Npsi)
     it = C.c_int32()
     # Krylov space up to Npsi + NKrylovMax vectors (grown per restart from Npsi + 100), within
     # half of the free device memory
-    free = eng.torch.cuda.mem_get_info(eng.device)[0]
+    free = qgpu.free_memory(eng.device)
     K = int(min(Npsi + int(o["NKrylovMax"]), n, max(2 * Npsi, free // (2 * 16 * max(n, 1)))))
     tol = float(o["Zero"])
     st = eng.L.qg_block_groundstate(eng.ctx, H.handle(eng), basis.h, Npsi, _ptr(x), _ptr(en), tol, K,
@@ -1491,8 +1498,8 @@ def _apply_between(O, dst, src, X, eng, device=False):
 
 
 def _to_dev(eng, A):
-    with eng.on_stream():
-        return eng.torch.from_numpy(np.ascontiguousarray(A, dtype=np.complex128)).to("cuda:%d" % eng.device)
+    A = np.ascontiguousarray(A, dtype=np.complex128)
+    return _allocate(eng, lambda dev: eng.torch.from_numpy(A).to(dev))
 
 
 def _adjoint_product(eng, A, B):
@@ -1643,7 +1650,6 @@ def _rixs_krylov_tensor(H1, H2, T1s, T2s, psis, o, eng):
     l + (NE1+1)(j2 + NT2(i1 + NT1(n2 + NT2(m1 + NT1(r + Npsi s)))))
     holds the element between v_(r, m1, n2) (left) and v_(s, i1, j2) (right)."""
     torch = eng.torch
-    dev = "cuda:%d" % eng.device
     npsi, nt1, nt2 = len(psis), len(T1s), len(T2s)
     M1, nf = npsi * nt1, H1.nf
     eps, ntri1, ntri2 = float(o["Epsilon"]), int(o["NTri1"]), int(o["NTri2"])
@@ -1668,9 +1674,8 @@ def _rixs_krylov_tensor(H1, H2, T1s, T2s, psis, o, eng):
             v = np.where(t.val.real ** 2 + t.val.imag ** 2 > eps * eps, t.val, 0.0)
             np.add.at(X1[:, j], b1.find(t.det), v)
     nk = ntri1 * M1
-    with eng.on_stream():
-        x1 = torch.from_numpy(X1).to(dev)
-        K1 = torch.zeros((nk, n1), dtype=torch.complex128, device=dev)
+    x1 = _allocate(eng, lambda dev: torch.from_numpy(X1).to(dev))
+    K1 = _allocate(eng, lambda dev: torch.zeros((nk, n1), dtype=torch.complex128, device=dev))
     A1, B1, sizes1 = block_lanczos(H1, b1, x1, ntri1, eps, sv, eng, krylov=K1)
     A1, B1 = block_chop(A1, eps), block_chop(B1, eps)
     T1m = block_tridiagonal_dense(A1, B1)

@@ -55,6 +55,7 @@ qg_status qg_check_device_error(qg_context ctx, const char *what) {
 struct QgPool {
   std::mutex m;
   bool open = true;
+  int device = 0;
   size_t held = 0;
   std::list<std::pair<void *, size_t>> idle;  // oldest first
 
@@ -74,12 +75,29 @@ std::mutex g_live_m;
 std::unordered_map<void *, std::pair<std::shared_ptr<QgPool>, size_t>> g_live;
 std::vector<std::weak_ptr<QgPool>> g_pools;
 
-std::vector<std::shared_ptr<QgPool>> all_pools() {
+std::vector<std::shared_ptr<QgPool>> pools_of(int device) {
   std::lock_guard<std::mutex> l(g_live_m);
   std::vector<std::shared_ptr<QgPool>> out;
   for (auto &w : g_pools)
-    if (auto p = w.lock()) out.push_back(p);
+    if (auto p = w.lock())
+      if (p->device == device) out.push_back(p);
   return out;
+}
+
+void drain_pools(int device) {
+  for (auto &q : pools_of(device)) {
+    std::lock_guard<std::mutex> l(q->m);
+    q->shrink(0);
+  }
+}
+
+// cudaMalloc, tried again without what the pools of the device hold
+cudaError_t malloc_or_drain(qg_context ctx, void **p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  drain_pools(ctx->device);
+  return cudaMalloc(p, bytes);
 }
 }  // namespace
 
@@ -108,15 +126,7 @@ cudaError_t qg_malloc_bytes(qg_context ctx, void **p, size_t bytes) {
     }
   }
   if (!*p) {
-    cudaError_t e = cudaMalloc(p, need);
-    if (e == cudaErrorMemoryAllocation) {  // what the pools hold may be what is missing
-      cudaGetLastError();
-      for (auto &q : all_pools()) {
-        std::lock_guard<std::mutex> l(q->m);
-        q->shrink(0);
-      }
-      e = cudaMalloc(p, need);
-    }
+    const cudaError_t e = malloc_or_drain(ctx, p, need);
     if (e != cudaSuccess) {
       *p = nullptr;
       return e;
@@ -158,14 +168,55 @@ cudaError_t qg_free_now(void *p) {
   return cudaFree(p);
 }
 
-cudaError_t qg_mem_info(size_t *free_bytes, size_t *total_bytes) {
+// of the current device, which is `device`
+static cudaError_t memory_of(int device, size_t *free_bytes, size_t *total_bytes) {
   cudaError_t e = cudaMemGetInfo(free_bytes, total_bytes);
   if (e != cudaSuccess) return e;
-  for (auto &q : all_pools()) {
+  for (auto &q : pools_of(device)) {
     std::lock_guard<std::mutex> l(q->m);
     *free_bytes += q->held;
   }
   return cudaSuccess;
+}
+
+cudaError_t qg_mem_info(qg_context ctx, size_t *free_bytes, size_t *total_bytes) {
+  return memory_of(ctx->device, free_bytes, total_bytes);
+}
+
+// the device for the time of a call
+struct OnDevice {
+  int before = -1;
+  cudaError_t e;
+  explicit OnDevice(int device) {
+    e = cudaGetDevice(&before);
+    if (e == cudaSuccess && before != device) e = cudaSetDevice(device);
+  }
+  ~OnDevice() {
+    if (before >= 0) cudaSetDevice(before);
+  }
+};
+
+extern "C" qg_status qg_device_memory(int device, int64_t *free_bytes, int64_t *total_bytes) {
+  if (!free_bytes || !total_bytes) return QG_ERR_ARG;
+  OnDevice on(device);
+  size_t fr = 0, tot = 0;
+  if (on.e != cudaSuccess || memory_of(device, &fr, &tot) != cudaSuccess) {
+    cudaGetLastError();
+    return QG_ERR_CUDA;
+  }
+  *free_bytes = (int64_t)fr;
+  *total_bytes = (int64_t)tot;
+  return QG_OK;
+}
+
+extern "C" qg_status qg_trim(int device) {
+  OnDevice on(device);
+  if (on.e != cudaSuccess) {
+    cudaGetLastError();
+    return QG_ERR_CUDA;
+  }
+  drain_pools(device);
+  return QG_OK;
 }
 
 cudaError_t qg_upload(qg_context ctx, void *dst, const void *src, size_t bytes) {
@@ -180,7 +231,7 @@ qg_status qg_ensure_scratch(qg_context ctx, size_t bytes) {
   ctx->d_scratch = nullptr;
   ctx->scratch_bytes = 0;
   size_t b = bytes < 65536 ? 65536 : bytes;
-  QG_CUDA(ctx, cudaMalloc(&ctx->d_scratch, b));
+  QG_CUDA(ctx, malloc_or_drain(ctx, (void **)&ctx->d_scratch, b));
   ctx->scratch_bytes = b;
   return QG_OK;
 }
@@ -219,6 +270,7 @@ extern "C" qg_status qg_init(int device, qg_context *out) {
     return QG_ERR_CUDA;
   }
   ctx->pool = std::make_shared<QgPool>();
+  ctx->pool->device = device;
   {
     std::lock_guard<std::mutex> l(g_live_m);
     g_pools.erase(std::remove_if(g_pools.begin(), g_pools.end(), [](const std::weak_ptr<QgPool> &w) { return w.expired(); }),

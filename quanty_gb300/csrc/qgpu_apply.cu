@@ -1877,7 +1877,7 @@ static qg_status build_conn(qg_context ctx, qg_operator op, qg_basis b, OpBasisC
   same_basis_view(op, b, &c, &tab, &lv, &wreq);
   cudaStream_t s = ctx->stream;
   size_t fr = 0, tot = 0;
-  if (qg_mem_info(&fr, &tot) != cudaSuccess) {
+  if (qg_mem_info(ctx, &fr, &tot) != cudaSuccess) {
     cudaGetLastError();
     return QG_OK;
   }
@@ -1910,7 +1910,7 @@ static qg_status build_conn(qg_context ctx, qg_operator op, qg_basis b, OpBasisC
   }
   QG_TRY(qg_check_device_error(ctx, "connection counts"));
   size_t conn_bytes = (size_t)std::max<int64_t>(total, 1) * sizeof(uint2);
-  if (qg_mem_info(&fr, &tot) != cudaSuccess || 4 * conn_bytes > fr) {
+  if (qg_mem_info(ctx, &fr, &tot) != cudaSuccess || 4 * conn_bytes > fr) {
     cudaGetLastError();
     qg_free(cptr);
     return QG_OK;

@@ -349,7 +349,7 @@ qg_status qg_check_launch(qg_context ctx, const char *what);
 // Everything a context allocates is used in the order of its stream, which is what makes the
 // reuse safe; what other contexts may use too (bases, operators, the caches of a basis) goes back
 // after a wait for the device, the qg_free_now of its first block.  Bounded (QG_POOL_BYTES per context; larger blocks are not kept), given back by
-// qg_finalize and whenever an allocation fails.  While the stream is being captured the pool
+// qg_finalize, by qg_trim and whenever an allocation of the library fails.  While the stream is being captured the pool
 // stands aside.
 cudaError_t qg_malloc_bytes(qg_context ctx, void **p, size_t bytes);
 template <typename T>
@@ -360,8 +360,8 @@ cudaError_t qg_free(void *p);
 // to the device at once, after a wait for everything running on it (cudaFree: a kernel in flight may
 // be using any block)
 cudaError_t qg_free_now(void *p);
-// free device memory, counting what the pools hold as free
-cudaError_t qg_mem_info(size_t *free_bytes, size_t *total_bytes);
+// free memory of the context's device (the current one), counting what its contexts' pools hold as free
+cudaError_t qg_mem_info(qg_context ctx, size_t *free_bytes, size_t *total_bytes);
 // host to device in the order of the context's stream, complete on return
 cudaError_t qg_upload(qg_context ctx, void *dst, const void *src, size_t bytes);
 qg_status qg_check_device_error(qg_context ctx, const char *what);

@@ -36,6 +36,8 @@ def load(path=LIB_PATH):
     sig = {
         "qg_init": (C.c_int, [C.c_int, PP]),
         "qg_finalize": (C.c_int, [P]),
+        "qg_device_memory": (C.c_int, [C.c_int, C.POINTER(I64), C.POINTER(I64)]),
+        "qg_trim": (C.c_int, [C.c_int]),
         "qg_set_stream": (C.c_int, [P, P]),
         "qg_get_stream": (P, [P]),
         "qg_last_error": (C.c_char_p, [P]),
@@ -112,3 +114,12 @@ class RixsSettings(C.Structure):
                 ("emin1", C.c_double), ("emax1", C.c_double), ("ne1", C.c_int32), ("gamma1", C.c_double),
                 ("emin2", C.c_double), ("emax2", C.c_double), ("ne2", C.c_int32), ("gamma2", C.c_double),
                 ("energy1", C.c_double), ("energy2", C.c_double), ("res1", C.c_void_p), ("res2", C.c_void_p)]
+
+
+def free_memory(device=0):
+    """Free bytes of a device, what the contexts keep between calls counted as free."""
+    free, total = C.c_int64(), C.c_int64()
+    st = load().qg_device_memory(device, C.byref(free), C.byref(total))
+    if st != 0:
+        raise QGError(st, "qg_device_memory")
+    return free.value

@@ -22,7 +22,7 @@ from concurrent.futures import Future
 
 import numpy as np
 
-from . import api
+from . import api, qgpu
 
 
 def _footprint(n_det, nvec, ntri=0, krylov=False):
@@ -117,8 +117,7 @@ class Server:
         self.merge, self.max_merge = bool(merge), int(max_merge)
         self.paused = bool(paused)  # workers admit nothing until resume()
         if hbm_budget is None:
-            free, total = torch.cuda.mem_get_info(device)
-            hbm_budget = int(0.8 * free)
+            hbm_budget = int(0.8 * qgpu.free_memory(device))
         self.budget = int(hbm_budget)
         self.in_use = 0
         self.queue = deque()

@@ -374,7 +374,7 @@ __global__ void __launch_bounds__(256)
       });
 }
 
-#define ONE_TINY 1e-280  // a squared norm below has lost digits
+#define ONE_TINY 0x05d00000  // upper word of 2^-930: a squared norm below has lost digits
 
 // w -= sum_i c_i v_i over i < k (out = w), and the squared norm of the result: the last block
 // leaves beta = |w|, its reciprocal and, when the vector vanished or the projection took more than it
@@ -388,20 +388,19 @@ __global__ void __launch_bounds__(128)
   T *cs = reinterpret_cast<T *>(smem_raw);
   __shared__ double sh[4];
   __shared__ int s_last;
-  __shared__ unsigned s_top;
+  __shared__ int s_top[4];
   const int tid = threadIdx.x;
   qg_chain_wait();
-  for (int i = tid; i < k; i += 128) cs[i] = c[i];
-  __syncthreads();
-  if (k && tid >= 96) {  // the largest upper word of c's parts: |c|^2 <= t by it unless t is rounding
-    unsigned top = 0;
-    for (int i = tid - 96; i < k; i += 32) {
-      const double2 z = one_complex(cs[i]);
-      top = max(top, (unsigned)max(__double2hiint(z.x) & 0x7fffffff, __double2hiint(z.y) & 0x7fffffff));
-    }
-    top = __reduce_max_sync(0xffffffffu, top);
-    if (tid == 96) s_top = top;
+  int top = 0;  // the largest upper word of c's parts
+  for (int i = tid; i < k; i += 128) {
+    const T ci = c[i];
+    const double2 z = one_complex(ci);
+    cs[i] = ci;
+    top = max(top, max(__double2hiint(z.x) & 0x7fffffff, __double2hiint(z.y) & 0x7fffffff));
   }
+  top = __reduce_max_sync(0xffffffffu, top);
+  if ((tid & 31) == 0) s_top[tid >> 5] = top;
+  __syncthreads();
   double s = 0.0;
   for (int64_t r = (int64_t)blockIdx.x * 128 + tid; r < n; r += (int64_t)gridDim.x * 128) {
     const T x = one_minus_sum(w[r], V, n, k, cs, r);
@@ -410,16 +409,23 @@ __global__ void __launch_bounds__(128)
   }
   const double t = one_total128(s, part, sh, &s_last, &sc->tickets[0]);
   if (s_last && tid == 0) {
-    const double b = sqrt(t), cm = __hiloint2double((int)s_top, -1);  // no part of c is above cm
-    bool lost = !(t > (k ? ONE_TINY : 0.0));
-    if (k && !lost && !(cm * cm * (2.0 * k) <= t)) {
-      double c2 = 0.0;
-      for (int i = 0; i < k; i++) c2 += one_abs2(cs[i]);
-      lost = !(c2 <= t);
+    const double b = sqrt(t), inv = 1.0 / b;
+    // |c|^2 <= t by the exponents (integers, beside the FP64 chain of the root), summed only where they do not
+    // settle it: no part of c reaches 2^(et + 1), so the sum of the 2 k squares stays below 2^(2 et + 2 + bits)
+    const int th = __double2hiint(t);
+    bool lost = !(t > 0.0);
+    if (k) {
+      const int et = (max(max(s_top[0], s_top[1]), max(s_top[2], s_top[3])) >> 20) - 1023;
+      lost = th < ONE_TINY || th >= 0x7ff00000;
+      if (!lost && 2 * et + 2 + (32 - __clz(2 * k - 1)) > (th >> 20) - 1023) {
+        double c2 = 0.0;
+        for (int i = 0; i < k; i++) c2 += one_abs2(cs[i]);
+        lost = !(c2 <= t);
+      }
     }
     sc->norm2 = t;
     sc->beta = lost ? 0.0 : b;
-    sc->scale = lost ? 0.0 : 1.0 / b;
+    sc->scale = lost ? 0.0 : inv;
     if (lost && step < sc->dead) sc->dead = step;
   }
 }

@@ -2298,7 +2298,7 @@ __global__ void k_slice_width(const int *__restrict__ len, int64_t n, int *__res
 #define QG_SELL_APPLIES 4    // the apply that builds them when nothing was said before
 
 // Build the explicit rows of (op, b); sell_state -1 where the lists stay in use: large bases, complex
-// values, and sum operators, whose values change.
+// values, sum operators, whose values change, and rows of more than a quarter of the free memory.
 static qg_status build_sell(qg_context ctx, qg_operator op, qg_basis b, OpBasisCache *c) {
   c->sell_state = -1;
   const int64_t n = b->n;
@@ -2333,6 +2333,9 @@ static qg_status build_sell(qg_context ctx, qg_operator op, qg_basis b, OpBasisC
   qg_free(width);
   qg_free(tmp);
   const size_t cells = std::max<size_t>((size_t)total * 32, 1);
+  size_t fr = 0, tot = 0;  // as the lists, the rows take at most a quarter of the free memory
+  if (e == cudaSuccess) e = qg_mem_info(ctx, &fr, &tot);
+  if (e == cudaSuccess && 4 * cells * (sizeof(uint32_t) + sizeof(double)) > fr) e = cudaErrorMemoryAllocation;
   if (e == cudaSuccess) e = qg_malloc(ctx, &c->s_col, cells * sizeof(uint32_t));
   if (e == cudaSuccess) e = qg_malloc(ctx, &c->s_val, cells * sizeof(double));
   if (e == cudaSuccess) {

@@ -779,19 +779,37 @@ __device__ __forceinline__ void acc_real_term(double2 &acc, double v, const doub
     qg_cmac(acc, v, 0.0, false, __ldg(x + idx));
 }
 
-// Resident blocks asked of the list kernel by vectors per pass.  Its gathers wait on L2, and more warps
-// hide that better than registers beyond the sums do (a few bytes of spill at most).  us per apply with
-// 6 and with 8 blocks at one vector: 47.5 M determinants 3600 and 3316, real Lanczos step on 3.9 M
-// 314 and 285 (7 blocks as 8, 5 blocks 3941 and 355).  24 vectors on 1.7 M, registers unbounded and as
-// here: 2 per pass 5085 and 4444, 4 per pass 4538 and 4023, 8 per pass 4066 and 3970; one more block
-// each: 4502, 4406, 4043.
-constexpr int list_min_blocks(int nv) { return nv == 1 ? 8 : nv == 2 ? 6 : nv <= 4 ? 5 : 3; }
+// Resident blocks per SM asked of the list kernel, by vectors per pass.  TIGHT: its gathers wait on L2, and where
+// a launch is many times what the chip holds, more warps hide that better than registers beyond the sums do (a few
+// bytes of spill at most).  Otherwise the registers that the sums and gathers want: where the blocks find room at
+// once there is little to hide, and the fuller thread is the faster.
+constexpr int list_blocks(int nv, bool tight) {
+  return !tight ? (nv == 1 ? 6 : 1) : nv == 1 ? 8 : nv == 2 ? 6 : nv <= 4 ? 5 : 3;
+}
+
+// The form for a launch of `blocks` blocks with nv vectors per pass.  us, six and eight blocks per SM:
+//   one vector, plain  real 94,995 rows 22.7, 24.8; 164,965 24.8, 26.7; 290,280 42.6, 41.1; 417,840 52.0, 54.2; 753,645
+//                      83.4, 85.0; 1.7 M 170, 171; 2.8 M 199, 194; 10.3 M 896, 849; 47.5 M 3600, 3316; complex 531,835
+//                      102.7, 105.0; 1.1 M 196, 198
+//   a real Lanczos step 94,995 rows 31.8, 33.9; 290,280 46.0, 40.1; 417,840 50.8, 52.9; 753,645 78.9, 75.7; 2.8 M 187, 174
+// so eight where they save a wave, which plain vectors (twice the bytes) show up to one wave of eight and then again
+// from some 64 blocks per SM.  Several vectors, own registers (2 to 3 blocks per SM) and tight:
+//   2: 29,635 rows 20.7, 22.6; 127,895 42.1, 41.2; 1.7 M 345, 324        4: 29,635 28.9, 30.9; 164,965 76.7, 85.6; 1.7 M 679, 638
+//   8: 29,635 45.4, 49.4; 94,995 144, 125; 164,965 152.7, 166.9; 945,835 623, 600
+// so tight beyond two blocks per SM, until a basis' second call has timed both (autotune).
+static bool list_tight(qg_context ctx, int nv, int64_t blocks, bool real_vector) {
+  const int64_t sms = ctx->num_sms;
+  if (nv > 1) return blocks > 2 * sms;
+  if (blocks <= 6 * sms) return false;
+  if (blocks <= 8 * sms || blocks > 64 * sms) return true;
+  return real_vector && (blocks + 8 * sms - 1) / (8 * sms) < (blocks + 6 * sms - 1) / (6 * sms);
+}
 
 // ORD: y is host memory (see the store at the end).  SPLIT (with FUSE and REAL): each complex
 // vector carries two real Lanczos chains, its real and imaginary parts.  RV (with FUSE, REAL
 // and NV = 1): x, y and prev hold one real number per row.
-template <int W, int NV, bool FUSE, bool REAL, bool ORD = false, bool SPLIT = false, bool RV = false>
-__global__ void __launch_bounds__(256, list_min_blocks(NV))
+template <int W, int NV, bool FUSE, bool TIGHT, bool REAL, bool ORD = false, bool SPLIT = false, bool RV = false>
+__global__ void __launch_bounds__(256, list_blocks(NV, TIGHT))
     k_apply_list(const Key<W> *__restrict__ rows, int64_t n_rows, const int64_t *__restrict__ cptr,
                  const uint2 *__restrict__ conn, const double2 *__restrict__ coef, const double2 *__restrict__ diag,
                  const double2 *__restrict__ x, int xs, double2 *__restrict__ y, int ys, int vec0, ApplyFuse fz,
@@ -1972,33 +1990,40 @@ bool qg_apply_uses_lists(qg_operator op, qg_basis b) {
   return c->conn_state == 1;
 }
 
-template <int W, int NV, bool FUSE>
-static void launch_apply_list_t(qg_context ctx, const OpBasisCache *c, const double2 *diag, qg_basis dst,
+template <int W, int NV, bool FUSE, bool TIGHT>
+static void launch_apply_list_f(qg_context ctx, const OpBasisCache *c, const double2 *diag, qg_basis dst,
                                 const double2 *x, int xs, double2 *y, int ys, int vec0, int npass,
                                 const ApplyFuse &fz, const LocalView &lv, bool real) {
   dim3 grid((unsigned)qg_apply_grid(dst), (unsigned)npass);
   const Key<W> *keys = (const Key<W> *)dst->d_keys;
-  if (NV == 1 && !FUSE && ctx->y_host) {  // one vector into host memory: rows stored in order
-    if (real)
-      k_apply_list<W, 1, false, true, true><<<grid, 256, 0, ctx->stream>>>(keys, dst->n, c->d_cptr, c->d_conn,
-                                                                        c->d_coef, diag, x, xs, y, ys, vec0, fz, lv);
-    else
-      k_apply_list<W, 1, false, false, true><<<grid, 256, 0, ctx->stream>>>(keys, dst->n, c->d_cptr, c->d_conn,
-                                                                         c->d_coef, diag, x, xs, y, ys, vec0, fz, lv);
-  } else if (NV == 1 && FUSE && fz.real_vector) {  // real operators only (the caller checks)
-    k_apply_list<W, 1, true, true, false, false, true><<<grid, 256, 0, ctx->stream>>>(
-        keys, dst->n, c->d_cptr, c->d_conn, c->d_coef, diag, x, xs, y, ys, vec0, fz, lv);
-  } else if (FUSE && fz.split) {  // real operators only (the caller checks)
-    k_apply_list<W, NV, true, true, false, true><<<grid, 256, 0, ctx->stream>>>(
-        keys, dst->n, c->d_cptr, c->d_conn, c->d_coef, diag, x, xs, y, ys, vec0, fz, lv);
-  } else if (real) {
-    k_apply_list<W, NV, FUSE, true><<<grid, 256, 0, ctx->stream>>>(keys, dst->n, c->d_cptr, c->d_conn, c->d_coef,
-                                                                   diag, x, xs, y, ys, vec0, fz, lv);
-  } else {
-    k_apply_list<W, NV, FUSE, false><<<grid, 256, 0, ctx->stream>>>(keys, dst->n, c->d_cptr, c->d_conn, c->d_coef,
-                                                                    diag, x, xs, y, ys, vec0, fz, lv);
+  auto run = [&](auto kernel) {
+    kernel<<<grid, 256, 0, ctx->stream>>>(keys, dst->n, c->d_cptr, c->d_conn, c->d_coef, diag, x, xs, y, ys, vec0, fz, lv);
+    ctx->launches++;
+  };
+  if constexpr (NV == 1 && !FUSE) {
+    if (ctx->y_host)  // one vector into host memory: rows stored in order
+      return real ? run(k_apply_list<W, 1, false, TIGHT, true, true>) : run(k_apply_list<W, 1, false, TIGHT, false, true>);
   }
-  ctx->launches++;
+  if constexpr (FUSE) {  // real operators only (the caller checks)
+    if (NV == 1 && fz.real_vector) return run(k_apply_list<W, 1, true, TIGHT, true, false, false, true>);
+    if (fz.split) return run(k_apply_list<W, NV, true, TIGHT, true, false, true>);
+  }
+  return real ? run(k_apply_list<W, NV, FUSE, TIGHT, true>) : run(k_apply_list<W, NV, FUSE, TIGHT, false>);
+}
+
+// form: LIST_FREE, LIST_TIGHT, or LIST_RULE for the rule above (one vector per pass always goes by it)
+enum { LIST_RULE = -1, LIST_FREE = 0, LIST_TIGHT = 1 };
+
+template <int W, int NV, bool FUSE>
+static void launch_apply_list_t(qg_context ctx, const OpBasisCache *c, const double2 *diag, qg_basis dst,
+                                const double2 *x, int xs, double2 *y, int ys, int vec0, int npass,
+                                const ApplyFuse &fz, const LocalView &lv, bool real, int form) {
+  const int64_t blocks = (int64_t)qg_apply_grid(dst) * npass;
+  const bool tight = NV == 1 || form == LIST_RULE ? list_tight(ctx, NV, blocks, FUSE && fz.real_vector) : form == LIST_TIGHT;
+  if (tight)
+    launch_apply_list_f<W, NV, FUSE, true>(ctx, c, diag, dst, x, xs, y, ys, vec0, npass, fz, lv, real);
+  else
+    launch_apply_list_f<W, NV, FUSE, false>(ctx, c, diag, dst, x, xs, y, ys, vec0, npass, fz, lv, real);
 }
 
 // Passes of 8, 4, 3, 2 or 1 vectors (at most `chunk` per pass); all passes of one width run as
@@ -2008,7 +2033,7 @@ static void launch_apply_list_t(qg_context ctx, const OpBasisCache *c, const dou
 template <int W, bool FUSE>
 static void launch_apply_list(qg_context ctx, const OpBasisCache *c, const double2 *diag, qg_basis dst,
                               const double2 *x, int xs, double2 *y, int ys, int nvec, const ApplyFuse &fz,
-                              const LocalView &lv, int chunk, bool real) {
+                              const LocalView &lv, int chunk, bool real, int form) {
   if (chunk <= 0) chunk = 8;
   int v = 0;
   while (v < nvec) {
@@ -2016,15 +2041,15 @@ static void launch_apply_list(qg_context ctx, const OpBasisCache *c, const doubl
     int per = left >= 8 ? 8 : left >= 4 ? 4 : left == 3 ? 3 : left >= 2 ? 2 : 1;
     int np = std::min((nvec - v) / per, 65535);
     if (per == 8)
-      launch_apply_list_t<W, 8, FUSE>(ctx, c, diag, dst, x, xs, y, ys, v, np, fz, lv, real);
+      launch_apply_list_t<W, 8, FUSE>(ctx, c, diag, dst, x, xs, y, ys, v, np, fz, lv, real, form);
     else if (per == 4)
-      launch_apply_list_t<W, 4, FUSE>(ctx, c, diag, dst, x, xs, y, ys, v, np, fz, lv, real);
+      launch_apply_list_t<W, 4, FUSE>(ctx, c, diag, dst, x, xs, y, ys, v, np, fz, lv, real, form);
     else if (per == 3)
-      launch_apply_list_t<W, 3, FUSE>(ctx, c, diag, dst, x, xs, y, ys, v, np, fz, lv, real);
+      launch_apply_list_t<W, 3, FUSE>(ctx, c, diag, dst, x, xs, y, ys, v, np, fz, lv, real, form);
     else if (per == 2)
-      launch_apply_list_t<W, 2, FUSE>(ctx, c, diag, dst, x, xs, y, ys, v, np, fz, lv, real);
+      launch_apply_list_t<W, 2, FUSE>(ctx, c, diag, dst, x, xs, y, ys, v, np, fz, lv, real, form);
     else
-      launch_apply_list_t<W, 1, FUSE>(ctx, c, diag, dst, x, xs, y, ys, v, np, fz, lv, real);
+      launch_apply_list_t<W, 1, FUSE>(ctx, c, diag, dst, x, xs, y, ys, v, np, fz, lv, real, form);
     v += per * np;
   }
 }
@@ -2413,7 +2438,7 @@ static OpBasisCache::Chunk *chunk_of(OpBasisCache *c, int nvec) {
 }
 
 static qg_status apply_chunked(qg_context ctx, qg_operator op, qg_basis dst, qg_basis src, const double *x, int xs,
-                               double *y, int ys, int nvec, const ApplyFuse *fz, bool x_packed, int chunk);
+                               double *y, int ys, int nvec, const ApplyFuse *fz, bool x_packed, int chunk, int form);
 
 // Vectors per pass over connection lists, for the first call on a basis.  All passes of one width
 // are one launch, the passes in the grid's second dimension, so narrow passes fill the chip on
@@ -2436,7 +2461,7 @@ static int list_chunk(int64_t n, int nvec) {
 
 // Times one plain apply per candidate number of vectors per pass and keeps the fastest for that
 // vector count: over lists 8, 4, 3, 2 or 1, on the second call (a basis that is used once never
-// pays for it: ten of the 54 ms of a RIXS call were timing); on the hash path also a warp per row with
+// pays for it: ten of the 54 ms of a RIXS call were timing), then the other form of that width; on the hash path also a warp per row with
 // 32 or 64, on the first.  Not while the stream is captured.  The candidates compute bitwise
 // the same result (each vector's sum runs in the same order), so the choice changes only the speed.
 static qg_status autotune(qg_context ctx, qg_operator op, qg_basis b, OpBasisCache *c, const double *x, int xs,
@@ -2452,42 +2477,47 @@ static qg_status autotune(qg_context ctx, qg_operator op, qg_basis b, OpBasisCac
     cudaGetLastError();
     return QG_OK;  // untimed: the choice in force stays
   }
-  int best = 8;
+  int best = 8, form = LIST_RULE;
   float best_ms = 0;
-  const int cand[7] = {8, 4, 3, 2, 1, -32, -64};
   qg_status st = QG_OK;
+  auto timed = [&](int ch, int fm, bool warm) -> float {  // < 0: not timed
+    if (warm && st == QG_OK) st = apply_chunked(ctx, op, b, b, x, xs, y, ys, nvec, nullptr, false, ch, fm);
+    cudaEventRecord(e0, ctx->stream);
+    if (st == QG_OK) st = apply_chunked(ctx, op, b, b, x, xs, y, ys, nvec, nullptr, false, ch, fm);
+    cudaEventRecord(e1, ctx->stream);
+    float ms = 0;
+    return st == QG_OK && cudaEventSynchronize(e1) == cudaSuccess && cudaEventElapsedTime(&ms, e0, e1) == cudaSuccess ? ms : -1.0f;
+  };
+  const int cand[7] = {8, 4, 3, 2, 1, -32, -64};
   for (int i = 0; i < 7 && st == QG_OK; i++) {
     int ch = cand[i];
     if (ch > nvec && ch != 8) continue;
     if (ch < 0 && (lists || nvec < 16 || (ch == -64 && nvec <= 32))) continue;
-    if (i == 0) st = apply_chunked(ctx, op, b, b, x, xs, y, ys, nvec, nullptr, false, ch);  // warm
-    cudaEventRecord(e0, ctx->stream);
-    if (st == QG_OK) st = apply_chunked(ctx, op, b, b, x, xs, y, ys, nvec, nullptr, false, ch);
-    cudaEventRecord(e1, ctx->stream);
-    float ms = 0;
-    if (st == QG_OK && cudaEventSynchronize(e1) == cudaSuccess && cudaEventElapsedTime(&ms, e0, e1) == cudaSuccess) {
-      if (i == 0 || ms < best_ms) {
-        best = ch;
-        best_ms = ms;
-      }
+    const float ms = timed(ch, LIST_RULE, i == 0);
+    if (ms >= 0.0f && (best_ms == 0 || ms < best_ms)) {
+      best_ms = ms;
+      best = ch;
     }
+  }
+  if (st == QG_OK && lists && best > 1 && best_ms > 0) {  // the other form of that width
+    const int other = list_tight(ctx, best, (int64_t)qg_apply_grid(b) * std::max(1, nvec / best), false) ? LIST_FREE : LIST_TIGHT;
+    const float ms = timed(best, other, true);
+    if (ms > 0.0f && ms < best_ms) form = other;
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   cudaGetLastError();
   if (st != QG_OK) return st;
-  if (OpBasisCache::Chunk *p = chunk_of(c, nvec)) {
-    p->chunk = best;
-    p->settled = 1;
-  } else {
-    c->chunk.push_back({nvec, best, 1});
-  }
+  if (OpBasisCache::Chunk *p = chunk_of(c, nvec))
+    *p = {nvec, best, 1, form};
+  else
+    c->chunk.push_back({nvec, best, 1, form});
   return QG_OK;
 }
 
 qg_status qg_apply_strided(qg_context ctx, qg_operator op, qg_basis dst, qg_basis src, const double *x, int xs,
                            double *y, int ys, int nvec, const ApplyFuse *fz, bool x_packed) {
-  int chunk = 8;
+  int chunk = 8, form = LIST_RULE;
   if (dst == src && nvec >= 2) {
     qg_status st = QG_OK;
     OpBasisCache *c = qg_basis_cache(ctx, dst, op, &st);
@@ -2497,14 +2527,17 @@ qg_status qg_apply_strided(qg_context ctx, qg_operator op, qg_basis dst, qg_basi
       if (!p) QG_TRY(ensure_conn(ctx, op, dst, c));
       const bool lists = c->conn_state == 1;
       if (!p && lists)
-        c->chunk.push_back({nvec, list_chunk(dst->n, nvec), 0});
+        c->chunk.push_back({nvec, list_chunk(dst->n, nvec), 0, LIST_RULE});
       else if (!lists || !fz)  // a step of a recursion is no second call (qg_apply_settle)
         QG_TRY(autotune(ctx, op, dst, c, x, xs, y, ys, nvec, lists));
       p = chunk_of(c, nvec);
     }
-    chunk = p ? p->chunk : 8;
+    if (p) {
+      chunk = p->chunk;
+      form = p->form;
+    }
   }
-  return apply_chunked(ctx, op, dst, src, x, xs, y, ys, nvec, fz, x_packed, chunk);
+  return apply_chunked(ctx, op, dst, src, x, xs, y, ys, nvec, fz, x_packed, chunk, form);
 }
 
 qg_status qg_apply_settle(qg_context ctx, qg_operator op, qg_basis b, const double *x, double *y, int nvec) {
@@ -2517,7 +2550,7 @@ qg_status qg_apply_settle(qg_context ctx, qg_operator op, qg_basis b, const doub
 }
 
 static qg_status apply_chunked(qg_context ctx, qg_operator op, qg_basis dst, qg_basis src, const double *x, int xs,
-                               double *y, int ys, int nvec, const ApplyFuse *fz, bool x_packed, int chunk) {
+                               double *y, int ys, int nvec, const ApplyFuse *fz, bool x_packed, int chunk, int form) {
   ApplyFuse none;
   const double2 *x2 = (const double2 *)x;
   double2 *y2 = (double2 *)y;
@@ -2560,14 +2593,14 @@ static qg_status apply_chunked(qg_context ctx, qg_operator op, qg_basis dst, qg_
         const bool real = op_values_real(op);
         if (op->W == 1) {
           if (fz)
-            launch_apply_list<1, true>(ctx, c, diag, dst, x2, xs, y2, ys, nvec, f, lv, chunk, real);
+            launch_apply_list<1, true>(ctx, c, diag, dst, x2, xs, y2, ys, nvec, f, lv, chunk, real, form);
           else
-            launch_apply_list<1, false>(ctx, c, diag, dst, x2, xs, y2, ys, nvec, f, lv, chunk, real);
+            launch_apply_list<1, false>(ctx, c, diag, dst, x2, xs, y2, ys, nvec, f, lv, chunk, real, form);
         } else {
           if (fz)
-            launch_apply_list<2, true>(ctx, c, diag, dst, x2, xs, y2, ys, nvec, f, lv, chunk, real);
+            launch_apply_list<2, true>(ctx, c, diag, dst, x2, xs, y2, ys, nvec, f, lv, chunk, real, form);
           else
-            launch_apply_list<2, false>(ctx, c, diag, dst, x2, xs, y2, ys, nvec, f, lv, chunk, real);
+            launch_apply_list<2, false>(ctx, c, diag, dst, x2, xs, y2, ys, nvec, f, lv, chunk, real, form);
         }
         return qg_check_launch(ctx, "qg_apply");
       }
@@ -2764,10 +2797,9 @@ extern "C" qg_status qg_apply_set_chunk(qg_context ctx, qg_operator op, qg_basis
   OpBasisCache *c = qg_basis_cache(ctx, b, op, &st);
   if (st != QG_OK) return st;
   if (OpBasisCache::Chunk *p = chunk_of(c, nvec)) {
-    p->chunk = chunk;
-    p->settled = 1;
+    *p = {nvec, chunk, 1, LIST_RULE};
   } else {
-    c->chunk.push_back({nvec, chunk, 1});
+    c->chunk.push_back({nvec, chunk, 1, LIST_RULE});
   }
   return QG_OK;
 }

@@ -215,9 +215,10 @@ struct OpBasisCache {
   uint32_t *s_col = nullptr;
   double *s_val = nullptr;
   // vectors per pass of the apply kernel, per number of vectors (nvec, chunk, settled: pinned or
-  // timed; otherwise from the rule, until the second call)
+  // timed; otherwise from the rule, until the second call), and the form of the list kernel
+  // (LIST_*, qgpu_apply.cu)
   struct Chunk {
-    int nvec, chunk, settled;
+    int nvec, chunk, settled, form;
   };
   std::vector<Chunk> chunk;
 };

@@ -1452,6 +1452,7 @@ void qg_cache_free(OpBasisCache &c) {
   qg_free(c.s_ptr);
   qg_free(c.s_col);
   qg_free(c.s_val);
+  if (c.built) cudaEventDestroy(c.built);
   c = OpBasisCache();
 }
 
@@ -1710,6 +1711,20 @@ static void launch_diag(qg_context ctx, qg_operator op, qg_basis b, double *d_di
 template <int W>
 __global__ void k_term_coef(const TermDev<W> *__restrict__ terms, int nterms, double2 *coef);
 
+// ctx has queued what fills the cache: marked, so that another context can wait for it
+static void cache_filled(qg_context ctx, OpBasisCache &c) {
+  c.builder = ctx;
+  c.complete = false;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  const bool capturing = cudaStreamIsCapturing(ctx->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
+  if (!capturing && (c.built || cudaEventCreateWithFlags(&c.built, cudaEventDisableTiming) == cudaSuccess) &&
+      cudaEventRecord(c.built, ctx->stream) == cudaSuccess)
+    return;
+  cudaGetLastError();
+  if (!capturing) cudaStreamSynchronize(ctx->stream);
+  c.complete = true;  // a captured build runs with its graph
+}
+
 // A sum operator was rescaled since this cache was built: recompute what depends on values
 // (the diagonal, the local entries' values, the list coefficients); the structure -- blocks,
 // entries, window bits, connection lists -- stays.
@@ -1737,7 +1752,7 @@ static qg_status refresh_values(qg_basis b, qg_operator op, OpBasisCache &c) {
     }
   }
   c.op_version = op->version;
-  c.complete = false;
+  cache_filled(ctx, c);
   return qg_check_launch(ctx, "value refresh");
 }
 
@@ -1759,10 +1774,10 @@ static void launch_diag(qg_context ctx, qg_operator op, qg_basis b, double *d_di
   ctx->launches++;
 }
 
-// The cache is filled on the stream of the basis' context: another context waits for it once.
-static qg_status cache_complete(qg_context user, qg_basis b, OpBasisCache &c) {
-  if (c.complete || user == b->ctx) return QG_OK;
-  QG_CUDA(user, cudaStreamSynchronize(b->ctx->stream));
+// Another context than the one that filled the cache waits, once, for what that one queued.
+static qg_status cache_complete(qg_context user, OpBasisCache &c) {
+  if (c.complete || user == c.builder) return QG_OK;
+  QG_CUDA(user, cudaEventSynchronize(c.built));
   c.complete = true;
   return QG_OK;
 }
@@ -1772,7 +1787,7 @@ OpBasisCache *qg_basis_cache(qg_context user, qg_basis b, qg_operator op, qg_sta
   for (auto &c : b->caches)
     if (c.op_uid == op->uid) {
       if (c.op_version != op->version) *st = refresh_values(b, op, c);
-      if (*st == QG_OK) *st = cache_complete(user, b, c);
+      if (*st == QG_OK) *st = cache_complete(user, c);
       return *st == QG_OK ? &c : nullptr;
     }
   qg_context ctx = b->ctx;
@@ -1823,9 +1838,10 @@ OpBasisCache *qg_basis_cache(qg_context user, qg_basis b, qg_operator op, qg_sta
       c.d_wreq = nullptr;
     }
   }
+  cache_filled(ctx, c);
   b->caches.push_back(c);
   *st = qg_check_launch(ctx, "operator-basis cache");
-  if (*st == QG_OK) *st = cache_complete(user, b, b->caches.back());
+  if (*st == QG_OK) *st = cache_complete(user, b->caches.back());
   return &b->caches.back();
 }
 
@@ -2320,6 +2336,7 @@ __global__ void k_slice_width(const int *__restrict__ len, int64_t n, int *__res
 }
 
 #define QG_SELL_ROWS 80000   // most rows of a basis with explicit rows (see above)
+#define QG_SELL_UNSEEN ((size_t)64 << 20)
 #define QG_SELL_APPLIES 4    // the apply that builds them when nothing was said before
 
 // Build the explicit rows of (op, b); sell_state -1 where the lists stay in use: large bases, complex
@@ -2358,9 +2375,13 @@ static qg_status build_sell(qg_context ctx, qg_operator op, qg_basis b, OpBasisC
   qg_free(width);
   qg_free(tmp);
   const size_t cells = std::max<size_t>((size_t)total * 32, 1);
-  size_t fr = 0, tot = 0;  // as the lists, the rows take at most a quarter of the free memory
-  if (e == cudaSuccess) e = qg_mem_info(ctx, &fr, &tot);
-  if (e == cudaSuccess && 4 * cells * (sizeof(uint32_t) + sizeof(double)) > fr) e = cudaErrorMemoryAllocation;
+  // as the lists, the rows take at most a quarter of the free memory; small ones without the 20 us of a look at it
+  const size_t row_bytes = cells * (sizeof(uint32_t) + sizeof(double));
+  if (e == cudaSuccess && row_bytes > QG_SELL_UNSEEN) {
+    size_t fr = 0, tot = 0;
+    e = qg_mem_info(ctx, &fr, &tot);
+    if (e == cudaSuccess && 4 * row_bytes > fr) e = cudaErrorMemoryAllocation;
+  }
   if (e == cudaSuccess) e = qg_malloc(ctx, &c->s_col, cells * sizeof(uint32_t));
   if (e == cudaSuccess) e = qg_malloc(ctx, &c->s_val, cells * sizeof(double));
   if (e == cudaSuccess) {
@@ -2376,9 +2397,9 @@ static qg_status build_sell(qg_context ctx, qg_operator op, qg_basis b, OpBasisC
                                                          (double2 *)c->s_val, nullptr);
     ctx->launches++;
     e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // another context may use the rows next
   }
   if (e == cudaSuccess) {
+    cache_filled(ctx, *c);
     c->sell_state = 1;
     return QG_OK;
   }

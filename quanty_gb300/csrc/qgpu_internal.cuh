@@ -181,7 +181,10 @@ struct LocalEntry {
 struct OpBasisCache {
   uint64_t op_uid = 0;
   uint64_t op_version = 0;        // the operator's value version the cached values belong to
-  bool complete = false;          // a context other than the basis' own has waited for its build
+  // the context that filled it last, an event behind that, and whether another context has waited for it
+  qg_context builder = nullptr;
+  cudaEvent_t built = nullptr;
+  bool complete = false;
   double *d_diag = nullptr;       // complex per row: all diagonal terms
   uint64_t *d_wreq = nullptr;     // per term of op->pull_nl: window bits its source needs
   bool wreq_exact = false;        // every term's window change fits the bit encoding

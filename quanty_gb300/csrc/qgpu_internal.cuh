@@ -87,6 +87,7 @@ struct qg_context_s {
   int device = 0;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
+  bool load_only = false;  // launches of the list kernel only load it (autotune)
   std::string last_error;
   int64_t launches = 0;
   unsigned int *d_err = nullptr;      // device error word

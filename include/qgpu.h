@@ -186,9 +186,8 @@ qg_status qg_hermitian_eigh(qg_context ctx, int32_t k, const double *a_host, dou
  * handle one vector at a time).  Over connection lists the first apply of an operator with
  * nvec >= 2 vectors on a basis (as its own source and target) takes the number of vectors
  * handled per pass from a rule on the rows and the vectors, and the second times (outside
- * stream capture) 8, 4, 3, 2 and 1 and keeps the fastest for that (operator, basis, nvec);
- * without lists the first apply times them: a
- * thread per row carrying 8, 4, 3, 2 or 1 vectors per pass, or (nvec >= 16) a warp per row with
+ * stream capture) 8, 4, 3, 2 and 1, and the kernel's other form at the fastest of them, and keeps the
+ * fastest for that (operator, basis, nvec); without lists the first apply times them: a thread per row carrying 8, 4, 3, 2 or 1 vectors per pass, or (nvec >= 16) a warp per row with
  * its lanes over 32 or 64 vectors per pass (chunk -32, -64).  Every choice sums each vector's
  * connections in the same order, so the result is bitwise the same.  qg_set_autotune(ctx, 0)
  * turns the choice off (passes of 8 vectors); qg_apply_chunk reports the choice in force (0

@@ -2480,15 +2480,17 @@ static qg_status apply_chunked(qg_context ctx, qg_operator op, qg_basis dst, qg_
 // A warp per row (32 or 64 vectors per pass, no lists) was 2 to 110 times slower there.
 static int list_chunk(int64_t n, int nvec) {
   const int64_t work = n * nvec;
+  // the lines, in half powers of two, that minimise the mean over those timings
   if (work < ((int64_t)1 << 19)) return 1;  // launches and latency
-  if (work > (nvec < 8 ? (int64_t)5931641 : nvec % 8 ? (int64_t)1 << 22 : (int64_t)1 << 21)) return 8;
+  const int64_t wide = nvec < 8 ? (int64_t)5931641 /* 2^22.5 */ : nvec % 8 ? (int64_t)1 << 22 : (int64_t)1 << 21;
+  if (work > wide) return 8;
   return nvec % 2 ? 1 : 2;
 }
 
 // Times one plain apply per candidate number of vectors per pass and keeps the fastest for that
 // vector count: over lists 8, 4, 3, 2 or 1, on the second call (a basis that is used once never
-// pays for it: ten of the 54 ms of a RIXS call were timing), then the other form of that width; on the hash path also a warp per row with
-// 32 or 64, on the first.  Not while the stream is captured.  The candidates compute bitwise
+// pays for it: ten of the 54 ms of a RIXS call were timing), then the other form of that width; on the
+// hash path also a warp per row with 32 or 64, on the first.  Not while the stream is captured.  The candidates compute bitwise
 // the same result (each vector's sum runs in the same order), so the choice changes only the speed.
 static qg_status autotune(qg_context ctx, qg_operator op, qg_basis b, OpBasisCache *c, const double *x, int xs,
                           double *y, int ys, int nvec, bool lists) {

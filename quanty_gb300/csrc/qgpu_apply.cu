@@ -794,7 +794,8 @@ constexpr int list_blocks(int nv, bool tight) {
 //   a real Lanczos step 94,995 rows 31.8, 33.9; 290,280 46.0, 40.1; 417,840 50.8, 52.9; 753,645 78.9, 75.7; 2.8 M 187, 174
 // so eight where they save a wave, which plain vectors (twice the bytes) show up to one wave of eight and then again
 // from some 64 blocks per SM.  Several vectors, own registers (2 to 3 blocks per SM) and tight:
-//   2: 29,635 rows 20.7, 22.6; 127,895 42.1, 41.2; 1.7 M 345, 324        4: 29,635 28.9, 30.9; 164,965 76.7, 85.6; 1.7 M 679, 638
+//   2: 29,635 rows 20.7, 22.6; 127,895 42.1, 41.2; 1.7 M 345, 324
+//   4: 29,635 28.9, 30.9; 164,965 76.7, 85.6; 1.7 M 679, 638
 //   8: 29,635 45.4, 49.4; 94,995 144, 125; 164,965 152.7, 166.9; 945,835 623, 600
 // so tight beyond two blocks per SM, until a basis' second call has timed both (autotune).
 static bool list_tight(qg_context ctx, int nv, int64_t blocks, bool real_vector) {
@@ -2490,8 +2491,9 @@ static int list_chunk(int64_t n, int nvec) {
 // Times one plain apply per candidate number of vectors per pass and keeps the fastest for that
 // vector count: over lists 8, 4, 3, 2 or 1, on the second call (a basis that is used once never
 // pays for it: ten of the 54 ms of a RIXS call were timing), then the other form of that width; on the
-// hash path also a warp per row with 32 or 64, on the first.  Not while the stream is captured.  The candidates compute bitwise
-// the same result (each vector's sum runs in the same order), so the choice changes only the speed.
+// hash path also a warp per row with 32 or 64, on the first.  Not while the stream is captured.  The
+// candidates compute bitwise the same result (each vector's sum runs in the same order), so the choice
+// changes only the speed.
 static qg_status autotune(qg_context ctx, qg_operator op, qg_basis b, OpBasisCache *c, const double *x, int xs,
                           double *y, int ys, int nvec, bool lists) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -2519,7 +2521,8 @@ static qg_status autotune(qg_context ctx, qg_operator op, qg_basis b, OpBasisCac
     if (st == QG_OK) st = apply_chunked(ctx, op, b, b, x, xs, y, ys, nvec, nullptr, false, ch, fm);
     cudaEventRecord(e1, ctx->stream);
     float ms = 0;
-    return st == QG_OK && cudaEventSynchronize(e1) == cudaSuccess && cudaEventElapsedTime(&ms, e0, e1) == cudaSuccess ? ms : -1.0f;
+    if (st != QG_OK || cudaEventSynchronize(e1) != cudaSuccess) return -1.0f;
+    return cudaEventElapsedTime(&ms, e0, e1) == cudaSuccess ? ms : -1.0f;
   };
   const int cand[7] = {8, 4, 3, 2, 1, -32, -64};
   for (int i = 0; i < 7 && st == QG_OK; i++) {
@@ -2533,7 +2536,8 @@ static qg_status autotune(qg_context ctx, qg_operator op, qg_basis b, OpBasisCac
     }
   }
   if (st == QG_OK && lists && best > 1 && best_ms > 0) {  // the other form of that width
-    const int other = list_tight(ctx, best, (int64_t)qg_apply_grid(b) * std::max(1, nvec / best), false) ? LIST_FREE : LIST_TIGHT;
+    const int64_t blocks = (int64_t)qg_apply_grid(b) * std::max(1, nvec / best);
+    const int other = list_tight(ctx, best, blocks, false) ? LIST_FREE : LIST_TIGHT;
     const float ms = timed(best, other, false);
     if (ms > 0.0f && ms < best_ms) form = other;
   }

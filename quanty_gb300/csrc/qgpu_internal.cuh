@@ -353,9 +353,9 @@ qg_status qg_check_launch(qg_context ctx, const char *what);
 // 31 of them, 4.05 ms with and 2.79 ms without; T*psi from 45, 0.94 and 0.51 ms.
 // Everything a context allocates is used in the order of its stream, which is what makes the
 // reuse safe; what other contexts may use too (bases, operators, the caches of a basis) goes back
-// after a wait for the device, the qg_free_now of its first block.  Bounded (QG_POOL_BYTES per context; larger blocks are not kept), given back by
-// qg_finalize, by qg_trim and whenever an allocation of the library fails.  While the stream is being captured the pool
-// stands aside.
+// after a wait for the device, the qg_free_now of its first block.  Bounded (QG_POOL_BYTES per
+// context; larger blocks are not kept), given back by qg_finalize, by qg_trim and whenever an allocation
+// of the library fails.  While the stream is being captured the pool stands aside.
 cudaError_t qg_malloc_bytes(qg_context ctx, void **p, size_t bytes);
 template <typename T>
 inline cudaError_t qg_malloc(qg_context ctx, T **p, size_t bytes) {
